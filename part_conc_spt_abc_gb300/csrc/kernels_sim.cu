@@ -7,9 +7,11 @@
  * launch with one warp per video).  Work items are (proposal, range of
  * particles) pulled from a device counter, so proposals with uneven Poisson
  * particle counts pack densely onto all SMs.  Per particle the walk state
- * lives in registers; each track's (K, DE) goes to a histogram whose first
- * rows are privatised in shared memory (flushed with red.global.add after
- * each item) and whose remaining rows take global atomics.
+ * lives in registers.  k_simulate_walk, the default, records tracks by global
+ * atomics and screens out the particles that are never detected; k_simulate
+ * (a tile of histogram rows privatised in shared memory, several walkers per
+ * thread, replayed draws) walks an item per CTA, and k_simulate_split is the
+ * slab-split walk.
  *
  * Arithmetic contract: the walk, DE and binning use explicit round-to-nearest
  * intrinsics (__fmul_rn/__fadd_rn/__fdiv_rn) in the reference's evaluation
@@ -44,13 +46,12 @@ __device__ __forceinline__ float wrap_(float v, float m, float two_m)
 /* The three wraps of one step.  A step is much shorter than the box, so a
  * wrap is rare: one combined test skips the three selects on the common
  * path (same values as three wrap_ calls). */
-__device__ __forceinline__ void wrap3_(float& x, float& y, float& z, float hx, float hy, float hz, float tx,
-                                       float ty, float tz)
+__device__ __forceinline__ void wrap3_(float& x, float& y, float& z, float hx, float hy, float hz)
 {
     if (__builtin_expect(fabsf(x) > hx || fabsf(y) > hy || fabsf(z) > hz, 0)) {
-        x = wrap_(x, hx, tx);
-        y = wrap_(y, hy, ty);
-        z = wrap_(z, hz, tz);
+        x = wrap_(x, hx, 2.0f * hx);
+        y = wrap_(y, hy, 2.0f * hy);
+        z = wrap_(z, hz, 2.0f * hz);
     }
 }
 
@@ -160,13 +161,20 @@ __device__ __forceinline__ void record_(const ItemCtx& c, uint32_t* tile, uint32
     record_out_<AGG>(c.four_dt, c.dde, c.B, c.RB, c.tile_rows, c.hist, c.err, tile, k, de);
 }
 
+/* Where a walk's tracks go: the item's tile (and the histogram past it). */
+template <bool AGG>
+struct TileSink {
+    uint32_t* tile;
+    __device__ __forceinline__ void record(const ItemCtx& c, uint32_t k, float de) const { record_<AGG>(c, tile, k, de); }
+};
+
 /* One frame of the walk.  CHECK: the frame may lie past the particle's
  * last one (s >= F) and is then skipped; full groups of four frames call it
  * without the test.  SCALED: the normals already carry the step sd (fresh
  * Philox draws); replayed normals are unit normals, scaled here as the
  * reference scales them. */
-template <bool AGG, bool CHECK = true, bool SCALED = false>
-__device__ __forceinline__ void step_(const ItemCtx& c, uint32_t* tile, Walker& w, uint32_t s,
+template <class SINK, bool CHECK = true, bool SCALED = false>
+__device__ __forceinline__ void step_(const ItemCtx& c, const SINK& sink, Walker& w, uint32_t s,
                                       float n0, float n1, float n2)
 {
     if (CHECK && s >= w.F) return;
@@ -176,7 +184,7 @@ __device__ __forceinline__ void step_(const ItemCtx& c, uint32_t* tile, Walker& 
     w.x = __fadd_rn(w.x, dx);
     w.y = __fadd_rn(w.y, dy);
     w.z = __fadd_rn(w.z, dz);
-    wrap3_(w.x, w.y, w.z, c.hlx, c.hly, c.hlz, c.two_hlx, c.two_hly, c.two_hlz);
+    wrap3_(w.x, w.y, w.z, c.hlx, c.hly, c.hlz);
     /* kernel-simulate.inl:70-93: a detected step extends the track (DE from
      * its second frame on), an undetected one closes it (recorded if K >=
      * kmin).  (Updating the track state by selects instead keeps all lanes
@@ -187,7 +195,7 @@ __device__ __forceinline__ void step_(const ItemCtx& c, uint32_t* tile, Walker& 
         if (kp >= 2u) w.de = __fadd_rn(w.de, __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
         w.k = kp;
     } else {
-        if (w.k >= c.kmin) record_<AGG>(c, tile, w.k, w.de);
+        if (w.k >= c.kmin) sink.record(c, w.k, w.de);
         w.k = 0u;
         w.de = 0.0f;
     }
@@ -335,65 +343,25 @@ __device__ __forceinline__ void group_normals_(const SimArgs& a, const Walker& q
 
 /* Frames 1 .. F-1 of one walker, four per group: the full groups skip the
  * per-frame end test, the tail group keeps it. */
-template <bool REPLAY, bool AGG>
-__device__ __forceinline__ void walk_single_(const SimArgs& a, const ItemCtx& c, uint32_t* tile, Walker& q)
+template <bool REPLAY, class SINK>
+__device__ __forceinline__ void walk_single_(const SimArgs& a, const ItemCtx& c, const SINK& sink, Walker& q)
 {
     uint32_t s0 = 1;
     for (; s0 + 3u < q.F; s0 += 4u) {
         float nn[12];
         group_normals_<REPLAY>(a, q, s0, nn);
-        step_<AGG, false, !REPLAY>(c, tile, q, s0 + 0u, nn[0], nn[1], nn[2]);
-        step_<AGG, false, !REPLAY>(c, tile, q, s0 + 1u, nn[3], nn[4], nn[5]);
-        step_<AGG, false, !REPLAY>(c, tile, q, s0 + 2u, nn[6], nn[7], nn[8]);
-        step_<AGG, false, !REPLAY>(c, tile, q, s0 + 3u, nn[9], nn[10], nn[11]);
+        step_<SINK, false, !REPLAY>(c, sink, q, s0 + 0u, nn[0], nn[1], nn[2]);
+        step_<SINK, false, !REPLAY>(c, sink, q, s0 + 1u, nn[3], nn[4], nn[5]);
+        step_<SINK, false, !REPLAY>(c, sink, q, s0 + 2u, nn[6], nn[7], nn[8]);
+        step_<SINK, false, !REPLAY>(c, sink, q, s0 + 3u, nn[9], nn[10], nn[11]);
     }
     if (s0 < q.F) {
         float nn[12];
         group_normals_<REPLAY>(a, q, s0, nn);
-        step_<AGG, true, !REPLAY>(c, tile, q, s0 + 0u, nn[0], nn[1], nn[2]);
-        step_<AGG, true, !REPLAY>(c, tile, q, s0 + 1u, nn[3], nn[4], nn[5]);
-        step_<AGG, true, !REPLAY>(c, tile, q, s0 + 2u, nn[6], nn[7], nn[8]);
-        step_<AGG, true, !REPLAY>(c, tile, q, s0 + 3u, nn[9], nn[10], nn[11]);
-    }
-}
-
-/* Work without a shared-memory histogram tile (every record a global
- * atomic): nothing ties a CTA's warps to one work item, so each warp takes
- * its own 32-particle slice of an item from the queue (slice s is part
- * s % slices of item s / slices) and no CTA barrier is needed.  Same walkers,
- * same draws, same records as the CTA loop. */
-template <bool AGG>
-__device__ __noinline__ void simulate_warp_slices_(const SimArgs& a)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t slices = (a.chunk + 31u) / 32u;
-    const uint32_t n_slices = *a.n_items * slices;
-    for (;;) {
-        uint32_t sl = 0u;
-        if (lane == 0u) sl = atomicAdd(a.queue_head, 1u);
-        sl = __shfl_sync(0xFFFFFFFFu, sl, 0);
-        if (sl >= n_slices) break;
-        const uint32_t item = sl / slices, part = sl - item * slices;
-        const PropDev& prop = a.props[a.item_prop[item]];
-        const JobDev& job = a.jobs[prop.job];
-        const ItemCtx c = item_ctx_(a, job, prop);
-        const uint32_t i0 = (item - prop.item_begin) * a.chunk;
-        const uint32_t i1 = min(i0 + a.chunk, prop.total_particles);
-        const uint32_t n = i0 + part * 32u + lane;
-        if (n < i1) {
-            Walker q;
-            q.n = n;
-            q.F = 0;
-            q.k = 0;
-            q.de = 0.0f;
-            q.x = q.y = q.z = 0.0f;
-            q.sd = 0.0f;
-            q.haz = 0.0f;
-            init_walker_<false, true>(a, c, job, prop, a.counts + prop.counts_off + job.V, n, prop.slot,
-                                pcs_ctr_gen_trial(prop.gen, prop.trial), job.seed_lo, job.seed_hi, q);
-            walk_single_<false, AGG>(a, c, nullptr, q);
-            if (q.F > 0u && q.k >= c.kmin) record_<AGG>(c, nullptr, q.k, q.de);
-        }
+        step_<SINK, true, !REPLAY>(c, sink, q, s0 + 0u, nn[0], nn[1], nn[2]);
+        step_<SINK, true, !REPLAY>(c, sink, q, s0 + 1u, nn[3], nn[4], nn[5]);
+        step_<SINK, true, !REPLAY>(c, sink, q, s0 + 2u, nn[6], nn[7], nn[8]);
+        step_<SINK, true, !REPLAY>(c, sink, q, s0 + 3u, nn[9], nn[10], nn[11]);
     }
 }
 
@@ -411,10 +379,6 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
     __shared__ PropDev s_prop;
     __shared__ JobDev s_job;
 
-    if (!REPLAY && PPT == 1 && a.tile_words == 0u) {
-        simulate_warp_slices_<AGG>(a);
-        return;
-    }
     const uint32_t tid = threadIdx.x, bd = blockDim.x;
     for (uint32_t i = tid; i < a.tile_words; i += bd) s_tile[i] = 0u;
     const uint32_t n_items = *a.n_items;
@@ -427,6 +391,7 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
         if (item >= n_items) break;
         load_item_(a, item, s_prop, s_job);
         const ItemCtx c = item_ctx_(a, s_job, s_prop);
+        const TileSink<AGG> sink = {s_tile};
 
         const uint32_t V = s_job.V;
         const uint32_t* prefix = a.counts + s_prop.counts_off + V; /* [V+1] */
@@ -461,7 +426,7 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
             /* frames 1 .. F-1, four per group; one walker per thread: the
              * full groups skip the per-frame end test, the tail group keeps it */
             if (PPT == 1) {
-                walk_single_<REPLAY, AGG>(a, c, s_tile, w[0]);
+                walk_single_<REPLAY>(a, c, sink, w[0]);
             } else
             for (uint32_t s0 = 1; s0 < fmax; s0 += 4u) {
 #pragma unroll
@@ -470,10 +435,10 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
                     if (s0 >= q.F) continue;
                     float nn[12];
                     group_normals_<REPLAY>(a, q, s0, nn);
-                    step_<AGG, true, !REPLAY>(c, s_tile, q, s0 + 0u, nn[0], nn[1], nn[2]);
-                    step_<AGG, true, !REPLAY>(c, s_tile, q, s0 + 1u, nn[3], nn[4], nn[5]);
-                    step_<AGG, true, !REPLAY>(c, s_tile, q, s0 + 2u, nn[6], nn[7], nn[8]);
-                    step_<AGG, true, !REPLAY>(c, s_tile, q, s0 + 3u, nn[9], nn[10], nn[11]);
+                    step_<TileSink<AGG>, true, !REPLAY>(c, sink, q, s0 + 0u, nn[0], nn[1], nn[2]);
+                    step_<TileSink<AGG>, true, !REPLAY>(c, sink, q, s0 + 1u, nn[3], nn[4], nn[5]);
+                    step_<TileSink<AGG>, true, !REPLAY>(c, sink, q, s0 + 2u, nn[6], nn[7], nn[8]);
+                    step_<TileSink<AGG>, true, !REPLAY>(c, sink, q, s0 + 3u, nn[9], nn[10], nn[11]);
                 }
             }
 #pragma unroll
@@ -492,6 +457,426 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
             }
         }
     }
+}
+
+/* ----------------------------------------------------------------------- */
+/* The walk without a shared-memory histogram tile (k_simulate_walk).
+ *
+ * Every record is a global atomic, so nothing ties a CTA's warps to one work
+ * item: each warp takes 32-particle slices of the items from the device
+ * queue (slice s is part s % slices of item s / slices).
+ *
+ * Screening.  A particle is recorded only if some frame finds all three
+ * coordinates in the detection region, which is a tenth of the box's depth
+ * and a quarter of its area in the benchmark configurations: most particles
+ * of a video are never detected, and nothing of their walk reaches the
+ * histogram.  So a particle that starts far enough from the region along one
+ * coordinate is first walked along that coordinate alone, unwrapped: if it
+ * provably stays outside the region's images all along, it is done.  This
+ * costs the same Philox draws as the walk (a coordinate's normals lie in all
+ * three blocks of a group) but a third of the Box-Muller trigonometry, no
+ * wraps, no detection tests and no divergence.  A particle that comes too
+ * near is walked in full from its start, as are those that start too near:
+ * the histogram is the same, count for count.
+ *
+ * The screen walk's sums differ from the walk's own positions by rounding
+ * only.  With k = sd sqrt(2 ln 2) and the box half length h (6k <= h is
+ * required), per step: the trigonometric approximations and their arguments
+ * differ by less than 6e-5 (their documented error is far smaller), times
+ * the largest radius sqrt(33) k; the products' roundings, 7e-7 k; the
+ * position's additions and wraps, below 4 (h + 6k) 2^-24; the sum's own
+ * addition, below 2h 2^-24 while the particle is inside the interval.
+ * screen_margin_ bounds their total by 4e-4 k + 1e-6 h per frame, and the
+ * interval is narrowed by it on both sides.
+ *
+ * Screened and full walks go to full warps through a queue per CTA (entries
+ * (proposal, particle), guarded by a lock that is held for ~100 cycles once
+ * per 32-particle walk): a warp takes 32 candidates to screen if there are
+ * as many, else 32 full walks, else a new slice, whose particles it sorts
+ * into the queue.  What is left in the queue at the end is walked in full.
+ *
+ * Measured (forward model alone, before -> after): 1e10 particle-steps of
+ * configuration 3 in one proposal 28.1 -> 22.4 ms; configuration 1, prior
+ * pass and three generations (5.6e10 particle-steps) 158 -> 122 ms;
+ * configuration 0, a whole job's 66 short rounds 24.7 -> 20.9 ms.  The bound
+ * is the FMA-heavy pipe, where a Philox round's 32 x 32 -> 64 bit product
+ * takes four cycles: 52 products a group, 208 of the ~440 cycles per warp
+ * and group of a full walk and of the ~290 of a screen walk. */
+
+constexpr uint32_t kScreenQueue = 96;     /* entries of each queue: at most 62 stay between visits, 32 more during one */
+constexpr uint32_t kLockLimit = 1u << 22; /* tries before a wait for the queue's lock is given up */
+/* What is screened, and where.  A screen walk costs about 0.65 of a walk, so
+ * a particle is a candidate where it is likely to pass: its distance to the
+ * region is above kScreenSigmas standard deviations of its whole walk (0.7,
+ * 0.9, 1.1, 1.2 and 1.5 were timed; 1.1 and 1.2 are best, and flat).  Videos
+ * shorter than kScreenMinFrames are walked at once: sorting and starting
+ * their particles twice would weigh too much.  A launch of fewer than
+ * kScreenSlices slices per warp is over after a walk or two, which screening
+ * first would only lengthen; and the last slices, one for
+ * every kScreenTail-th warp, are walked at once so that no screened particle
+ * starts its full walk when the other warps are done (configuration 0's
+ * short rounds: 21.8 -> 20.9 ms of walks per job). */
+constexpr float kScreenSigmas = 1.1f;
+constexpr uint32_t kScreenMinFrames = 48;
+constexpr uint32_t kScreenSlices = 2;
+constexpr uint32_t kScreenTail = 2;
+
+struct ScreenQueue {
+    uint32_t lock, nc, nf;
+    uint2 c[kScreenQueue]; /* candidates to screen */
+    uint2 f[kScreenQueue]; /* full walks */
+};
+
+namespace {
+
+enum Visit { kVisitNone = 0, kVisitScreen = 1, kVisitFull = 2, kVisitAbort = 3, kVisitSort = 4 };
+
+/* One visit of a warp to its CTA's queue: lanes with push 1 or 2 add their
+ * entry to the candidates or the full walks; then the warp takes 32 of one
+ * kind (entry 0xFFFFFFFF: none for this lane).  `sorting`: more entries will
+ * come, so fewer than 32 stay; then they are taken, all for full walks.  After a visit at most 62 entries are left:
+ * 32 are taken whenever one queue holds that many. */
+__device__ __forceinline__ Visit queue_visit_(ScreenQueue& s, uint2& e, uint32_t push, bool sorting, uint32_t* err)
+{
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    uint32_t held = 0u;
+    if (lane == 0u) {
+        for (uint32_t it = 0; it < kLockLimit && !held; ++it) {
+            held = atomicCAS(&s.lock, 0u, 1u) == 0u ? 1u : 0u;
+            if (!held) __nanosleep(40);
+        }
+        if (!held) atomicOr(err, PCS_ERRBIT_TIMEOUT);
+    }
+    if (!__shfl_sync(0xFFFFFFFFu, held, 0)) return kVisitAbort;
+    __threadfence_block();
+    volatile ScreenQueue& q = s;
+    uint32_t nc = q.nc, nf = q.nf;
+    const unsigned mc = __ballot_sync(0xFFFFFFFFu, push == 1u), mf = __ballot_sync(0xFFFFFFFFu, push == 2u);
+    if (push == 1u) {
+        q.c[nc + __popc(mc & lt)].x = e.x;
+        q.c[nc + __popc(mc & lt)].y = e.y;
+    } else if (push == 2u) {
+        q.f[nf + __popc(mf & lt)].x = e.x;
+        q.f[nf + __popc(mf & lt)].y = e.y;
+    }
+    nc += __popc(mc);
+    nf += __popc(mf);
+    __threadfence_block();
+    __syncwarp();
+    Visit v = kVisitNone;
+    e.x = 0xFFFFFFFFu;
+    if (nc >= 32u) {
+        v = kVisitScreen;
+        nc -= 32u;
+        e.x = q.c[nc + lane].x;
+        e.y = q.c[nc + lane].y;
+    } else if (nf >= 32u || (!sorting && nf + nc > 0u)) {
+        v = kVisitFull;
+        const uint32_t tf = min(nf, 32u), tc = min(nc, 32u - tf);
+        nf -= tf;
+        if (lane < tf) {
+            e.x = q.f[nf + lane].x;
+            e.y = q.f[nf + lane].y;
+        }
+        if (!sorting) { /* the last ones: candidates are walked in full, too */
+            nc -= tc;
+            if (lane >= tf && lane < tf + tc) {
+                e.x = q.c[nc + lane - tf].x;
+                e.y = q.c[nc + lane - tf].y;
+            }
+        }
+    }
+    __syncwarp();
+    if (lane == 0u) {
+        q.nc = nc;
+        q.nf = nf;
+        __threadfence_block();
+        atomicExch(&s.lock, 0u);
+    }
+    __syncwarp();
+    return v;
+}
+
+/* Tracks closed by a warp's walks, kept until 32 of them can be binned at
+ * once: a record's two divisions and its atomic would otherwise run for the
+ * one lane whose track ended.  32 lanes close at most 128 tracks in a group
+ * of four frames. */
+constexpr uint32_t kTrackBuf = 160; /* 31 left over, 128 more */
+
+struct TrackBuf {
+    uint32_t p[kTrackBuf], k[kTrackBuf]; /* proposal, frames */
+    float de[kTrackBuf];
+};
+
+/* adds the track (k, de) of proposal p of the lanes with `rec` */
+__device__ __forceinline__ void track_push_(TrackBuf& b, uint32_t& n, bool rec, uint32_t p, uint32_t k, float de)
+{
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, rec);
+    if (m) {
+        if (rec) {
+            const uint32_t at = n + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u));
+            b.p[at] = p;
+            b.k[at] = k;
+            b.de[at] = de;
+        }
+        n += __popc(m);
+    }
+}
+
+/* bins the last `m` <= 32 of the n tracks */
+__device__ __forceinline__ void track_flush_(const SimArgs& a, TrackBuf& b, uint32_t& n, uint32_t m)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    n -= m;
+    if (lane < m) {
+        const PropDev& prop = a.props[b.p[n + lane]];
+        const JobDev& job = a.jobs[prop.job];
+        record_out_<false>(job.four_delta_t, job.dde, job.B, job.R * job.B, 0u, a.hist + prop.hist_off, a.err, nullptr,
+                           b.k[n + lane], b.de[n + lane]);
+    }
+    __syncwarp();
+}
+
+/* Four frames of 32 walks in step, one straight line of code: the tracks'
+ * state is updated by selects, and only where some lane's track has closed
+ * are the four frames gone through again to collect it.  (Branches on
+ * detection, as step_ has them, execute fewer instructions but leave each
+ * warp's next instruction waiting on the last; with the next group's normals
+ * drawn ahead this form lets 24 warps per SM do what 32 did, each walk takes
+ * less time and launches end sooner.)  CHECK: lanes whose particle has no
+ * frame s0 + t stay as they are. */
+template <bool CHECK>
+__device__ __forceinline__ void group_warp_(const ItemCtx& c, TrackBuf& b, uint32_t& nb, Walker& w, uint32_t p,
+                                            uint32_t s0, const float* nn)
+{
+    const uint32_t k0 = w.k;
+    const float de0 = w.de;
+    bool det[4], on[4], closed = false;
+    float dd[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        on[t] = !CHECK || s0 + (uint32_t)t < w.F;
+        const float dx = nn[3 * t], dy = nn[3 * t + 1];
+        const float x = wrap_(__fadd_rn(w.x, dx), c.hlx, 2.0f * c.hlx);
+        const float y = wrap_(__fadd_rn(w.y, dy), c.hly, 2.0f * c.hly);
+        const float z = wrap_(__fadd_rn(w.z, nn[3 * t + 2]), c.hlz, 2.0f * c.hlz);
+        det[t] = fabsf(z) <= w.haz && fabsf(x) <= c.hax && fabsf(y) <= c.hay;
+        dd[t] = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+        if (on[t]) {
+            w.x = x;
+            w.y = y;
+            w.z = z;
+            closed |= !det[t] && w.k >= c.kmin;
+            w.de = det[t] && w.k != 0u ? __fadd_rn(w.de, dd[t]) : 0.0f; /* from the track's second frame on */
+            w.k = det[t] ? w.k + 1u : 0u;
+        }
+    }
+    if (__any_sync(0xFFFFFFFFu, closed)) {
+        uint32_t k = k0;
+        float de = de0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            track_push_(b, nb, on[t] && !det[t] && k >= c.kmin, p, k, de);
+            if (on[t]) {
+                de = det[t] && k != 0u ? __fadd_rn(de, dd[t]) : 0.0f;
+                k = det[t] ? k + 1u : 0u;
+            }
+        }
+    }
+}
+
+/* Frames 1 .. F-1 of a warp's 32 particles (lanes without one have F = 0),
+ * and their last tracks. */
+__device__ __forceinline__ void walk_warp_(const SimArgs& a, const ItemCtx& c, TrackBuf& b, uint32_t& nb, Walker& q,
+                                           uint32_t p)
+{
+    const uint32_t f_max = __reduce_max_sync(0xFFFFFFFFu, q.F);
+    const uint32_t f_min = __reduce_min_sync(0xFFFFFFFFu, q.F ? q.F : f_max); /* 0 where no lane has one */
+    uint32_t s0 = 1;
+    float nn[12];
+    if (f_max > 1u) group_normals_<false>(a, q, s0, nn);
+    for (; s0 + 3u < f_min; s0 += 4u) {
+        float nx[12];
+        group_normals_<false>(a, q, s0 + 4u, nx);
+        group_warp_<false>(c, b, nb, q, p, s0, nn);
+        while (nb >= 32u) track_flush_(a, b, nb, 32u);
+#pragma unroll
+        for (int i = 0; i < 12; ++i) nn[i] = nx[i];
+    }
+#pragma unroll 1
+    for (; s0 < f_max; s0 += 4u) {
+        group_warp_<true>(c, b, nb, q, p, s0, nn);
+        while (nb >= 32u) track_flush_(a, b, nb, 32u);
+        group_normals_<false>(a, q, s0 + 4u, nn);
+    }
+    track_push_(b, nb, q.F > 0u && q.k >= c.kmin, p, q.k, q.de);
+    while (nb >= 32u) track_flush_(a, b, nb, 32u);
+}
+
+/* a position's distance from its detection region, along one coordinate:
+ * from the near edge, or 0.8 of that from the next image's edge */
+__device__ __forceinline__ float screen_room_(float v, float half_l, float half_a)
+{
+    const float u = fabsf(v);
+    return fminf(u - half_a, 0.8f * (2.0f * half_l - half_a - u));
+}
+
+__device__ __forceinline__ float screen_margin_(float k, float half_l, uint32_t F)
+{
+    return (__uint2float_rn(F) + 8.0f) * (4.0e-4f * k + 1.0e-6f * half_l);
+}
+
+/* the coordinate along which q has the most room (0 x, 1 y, 2 z) */
+__device__ __forceinline__ uint32_t screen_axis_(const Walker& q, const ItemCtx& c, float& room, float& half_l)
+{
+    const float rx = screen_room_(q.x, c.hlx, c.hax), ry = screen_room_(q.y, c.hly, c.hay);
+    const float rz = screen_room_(q.z, c.hlz, q.haz);
+    uint32_t axis = 0u;
+    room = rx;
+    half_l = c.hlx;
+    if (ry > room) {
+        axis = 1u;
+        room = ry;
+        half_l = c.hly;
+    }
+    if (rz > room) {
+        axis = 2u;
+        room = rz;
+        half_l = c.hlz;
+    }
+    return axis;
+}
+
+/* Whether to screen q (q.sd holds k).  Any NaN or infinity says no. */
+__device__ __forceinline__ bool screen_wanted_(const Walker& q, const ItemCtx& c)
+{
+    float room, half_l;
+    screen_axis_(q, c, room, half_l);
+    const float reach = kScreenSigmas / kSqrt2Ln2 * q.sd * sqrtf(__uint2float_rn(q.F));
+    return q.F >= kScreenMinFrames && c.kmin >= 1u && q.sd > 0.0f && 6.0f * q.sd <= half_l &&
+           room > reach + screen_margin_(q.sd, half_l, q.F);
+}
+
+/* The screen walk: true if q is certainly never detected.  The coordinate's
+ * normals of a group's four steps (group_normals_: numbers 0..11 in step
+ * order x, y, z, pairs sine then cosine) by axis:
+ *   x  r0.xy sin, r0.zw cos, r1.zw sin, r2.xy cos
+ *   y  r0.xy cos, r1.xy sin, r1.zw cos, r2.zw sin
+ *   z  r0.zw sin, r1.xy cos, r2.xy sin, r2.zw cos
+ * and cos(t) is taken as sin(t + pi/2), so all lanes run the same code. */
+__device__ __forceinline__ bool screen_walk_(const Walker& q, const ItemCtx& c)
+{
+    float room, half_l;
+    const uint32_t axis = screen_axis_(q, c, room, half_l);
+    const bool ax = axis == 0u, az = axis == 2u;
+    const float pi = 3.14159265358979f;
+    const float off0 = axis == 1u ? -0.5f * pi : -pi, off1 = axis == 1u ? -pi : -0.5f * pi;
+    float S = 0.0f, lo = 0.0f, hi = 0.0f; /* displacement over k, its extremes */
+    const uint32_t f_max = __reduce_max_sync(0xFFFFFFFFu, q.F);
+    for (uint32_t s0 = 1u, blk = 2u; s0 < f_max; s0 += 4u, blk += 3u) {
+        /* without this the lanes of a warp, whose axes differ, do not stay
+         * together: 20% more warp instructions per screened particle */
+        __syncwarp();
+        const pcs_u4 r0 = pcs_draw_pre(q.ph, pcs_ctr_tag(PCS_STREAM_PARTICLE, blk));
+        const pcs_u4 r1 = pcs_draw_pre(q.ph, pcs_ctr_tag(PCS_STREAM_PARTICLE, blk + 1u));
+        const pcs_u4 r2 = pcs_draw_pre(q.ph, pcs_ctr_tag(PCS_STREAM_PARTICLE, blk + 2u));
+        const uint32_t ra[4] = {az ? r0.z : r0.x, ax ? r0.z : r1.x, az ? r2.x : r1.z, ax ? r2.x : r2.z};
+        const uint32_t rb[4] = {az ? r0.w : r0.y, ax ? r0.w : r1.y, az ? r2.y : r1.w, ax ? r2.y : r2.w};
+        float d[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float u = __fmaf_rn(__uint2float_rn(ra[i]), 2.3283064365386963e-10f, 1.1641532182693481e-10f);
+            const float t = __fmaf_rn(__uint2float_rn(rb[i]), 1.4629180792671596e-09f, (i & 1) ? off1 : off0);
+            S = __fmaf_rn(sqrt_ftz_(-lg2_ftz_(u)), sin_ftz_(t), S);
+            d[i] = S;
+        }
+        if (s0 < q.F) {
+            lo = fminf(fminf(lo, fminf(d[0], d[1])), fminf(d[2], d[3]));
+            hi = fmaxf(fmaxf(hi, fmaxf(d[0], d[1])), fmaxf(d[2], d[3]));
+        }
+    }
+    /* the interval between the region and its next image, seen from u0 >= 0 */
+    const float v0 = ax ? q.x : (az ? q.z : q.y), half_a = ax ? c.hax : (az ? q.haz : c.hay);
+    const float u0 = fabsf(v0), m = screen_margin_(q.sd, half_l, q.F);
+    const float down = v0 < 0.0f ? hi : -lo, up = v0 < 0.0f ? -lo : hi; /* both >= 0 */
+    return u0 - q.sd * down > half_a + m && u0 + q.sd * up < 2.0f * half_l - half_a - m;
+}
+
+} // namespace
+
+/* Registers: 80 a thread in CTAs of up to 256 threads (24 warps per SM; 64
+ * and 32 warps, or 128 and 16, were slower by 1-4%), 64 in CTAs of 1024. */
+template <uint32_t BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK <= 256u ? 3 : 1) k_simulate_walk(const __grid_constant__ SimArgs a)
+{
+    __shared__ ScreenQueue s_queue;
+    extern __shared__ TrackBuf s_tracks[]; /* one per warp */
+    TrackBuf& tracks = s_tracks[threadIdx.x / 32u];
+    uint32_t n_tracks = 0u;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t slices = (a.chunk + 31u) / 32u;
+    const uint32_t n_slices = *a.n_items * slices, warps = gridDim.x * (blockDim.x / 32u);
+    const bool screening = n_slices / warps >= kScreenSlices;
+    const uint32_t n_sort = n_slices - min(n_slices, warps / kScreenTail);
+    if (threadIdx.x == 0u) s_queue.lock = s_queue.nc = s_queue.nf = 0u;
+    __syncthreads();
+
+    bool more = true, sorting = screening; /* slices are left; they go into the queue */
+    uint32_t push = 0u;
+    uint2 e = make_uint2(0xFFFFFFFFu, 0u); /* this lane's particle: (proposal, particle) */
+    for (;;) {
+        __syncwarp();
+        Visit v = kVisitNone;
+        if (screening) v = queue_visit_(s_queue, e, push, sorting, a.err);
+        push = 0u;
+        if (v == kVisitAbort) break;
+        if (v == kVisitNone) {
+            if (!more) break;
+            uint32_t sl = 0u;
+            if (lane == 0u) sl = atomicAdd(a.queue_head, 1u);
+            sl = __shfl_sync(0xFFFFFFFFu, sl, 0);
+            if (sl >= n_slices) {
+                more = sorting = false;
+                continue;
+            }
+            if (sl >= n_sort) sorting = false;
+            const uint32_t item = sl / slices, part = sl - item * slices;
+            const uint32_t p = a.item_prop[item];
+            const PropDev& prop = a.props[p];
+            const uint32_t i0 = (item - prop.item_begin) * a.chunk;
+            const uint32_t n = i0 + part * 32u + lane;
+            e = make_uint2(n < min(i0 + a.chunk, prop.total_particles) ? p : 0xFFFFFFFFu, n);
+            v = sorting && a.jobs[prop.job].frames_max >= kScreenMinFrames ? kVisitSort : kVisitFull;
+        }
+        Walker q;
+        ItemCtx c;
+        q.n = e.y;
+        q.F = q.k = 0u;
+        q.de = 0.0f;
+        if (e.x != 0xFFFFFFFFu) {
+            const PropDev& prop = a.props[e.x];
+            const JobDev& job = a.jobs[prop.job];
+            c = item_ctx_(a, job, prop);
+            init_walker_<false, true>(a, c, job, prop, a.counts + prop.counts_off + job.V, e.y, prop.slot,
+                                      pcs_ctr_gen_trial(prop.gen, prop.trial), job.seed_lo, job.seed_hi, q);
+        } else { /* never detected, never recorded */
+            c.hlx = c.hly = c.hlz = 1.0f;
+            c.hax = c.hay = q.haz = -1.0f;
+            c.kmin = 0xFFFFFFFFu;
+            q.x = q.y = q.z = q.sd = 0.0f;
+            q.ph = pcs_philox_prepare(0u, 0u, 0u, 0u, 0u);
+        }
+        __syncwarp();
+        if (v == kVisitSort) {
+            if (e.x != 0xFFFFFFFFu) push = screen_wanted_(q, c) ? 1u : 2u;
+        } else if (v == kVisitScreen) {
+            if (!screen_walk_(q, c)) push = 2u;
+        } else {
+            walk_warp_(a, c, tracks, n_tracks, q, e.x);
+        }
+    }
+    if (n_tracks) track_flush_(a, tracks, n_tracks, n_tracks);
 }
 
 /* ----------------------------------------------------------------------- */
@@ -788,6 +1173,14 @@ int occupancy_(uint32_t block, size_t smem)
     return n;
 }
 
+/* the tile-less walk's build for `block` threads (64 registers each way) */
+auto walk_kernel_(uint32_t block) -> void (*)(SimArgs)
+{
+    return block <= 256u ? k_simulate_walk<256> : (block <= 512u ? k_simulate_walk<512> : k_simulate_walk<1024>);
+}
+
+size_t walk_smem_(uint32_t block) { return (block / 32u) * sizeof(TrackBuf); }
+
 template <bool AGG>
 cudaError_t launch_split_(const SimArgs& a, uint32_t grid, size_t smem, cudaStream_t st)
 {
@@ -815,6 +1208,8 @@ uint32_t split_tile_words_(uint32_t tile_words)
     const size_t cap = (220u * 1024u - sizeof(SplitShared)) / 4u;
     return (uint32_t)(tile_words < cap ? tile_words : cap);
 }
+
+bool walk_launch_(const SimLaunch& l, uint32_t tile_words) { return !l.replay && l.ppt == 1 && tile_words == 0u; }
 } // namespace
 
 cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_t st)
@@ -827,6 +1222,14 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
         return l.aggregate ? launch_split_<true>(a, l.grid, smem, st) : launch_split_<false>(a, l.grid, smem, st);
     }
     const SimArgs& a = a_in;
+    if (walk_launch_(l, a.tile_words)) {
+        const auto fn = walk_kernel_(l.block);
+        const size_t tracks = walk_smem_(l.block);
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tracks);
+        if (e != cudaSuccess) return e;
+        fn<<<l.grid, l.block, tracks, st>>>(a);
+        return cudaGetLastError();
+    }
     const size_t smem = (size_t)a.tile_words * 4u;
 #define PCS_SIM_CASE(P, R, G)                                                               \
     if (l.ppt == P && l.replay == R && l.aggregate == G) return launch_sim_<P, R, G>(a, l.grid, l.block, smem, st);
@@ -849,6 +1252,13 @@ int simulate_occupancy(const SimLaunch& l, uint32_t tile_words)
     if (l.split) {
         const size_t smem = (size_t)split_tile_words_(tile_words) * 4u + sizeof(SplitShared);
         return l.aggregate ? occupancy_split_<true>(smem) : occupancy_split_<false>(smem);
+    }
+    if (walk_launch_(l, tile_words)) {
+        int n = 0;
+        const auto fn = walk_kernel_(l.block);
+        const size_t tracks = walk_smem_(l.block);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tracks);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)l.block, tracks) == cudaSuccess ? n : 0;
     }
     const size_t smem = (size_t)tile_words * 4u;
 #define PCS_SIM_OCC(P, R, G) \
