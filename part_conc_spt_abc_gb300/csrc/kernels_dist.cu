@@ -257,8 +257,14 @@ __global__ void __launch_bounds__(1024, 1) k_distance(DistArgs a)
  * formed as the float whose bits are 0x4B400000 + s - o (1.5 * 2^23 + s - o,
  * exact in [2^23, 2^24)) minus 1.5 * 2^23: the same value the reference's
  * two conversions and subtraction give, in two instructions.
- * SSD: also accumulate the exact integer sum of squares (128-bit per lane);
- * the PMC rounds do not ask for it, the parity entry point does. */
+ * F64: also the distance accumulated in double, SSD: the exact integer sum of
+ * squares (128-bit).  Below 2^22 a lane's squares of a strip (at most 52 rows)
+ * sum to less than 2^50, so every partial sum of the reference's double chain
+ * is that integer exactly: one 32 x 32 + 64 bit multiply-add per cell and one
+ * conversion per strip give the same double.  GB300's FP64 rate is a small
+ * fraction of its FP32 rate: three FP64 operations and two conversions per
+ * cell set the pace before (a short round of 201 x 1000: 398 -> 136 us;
+ * 16 of 1001 x 256 with both sums and the prefix sums: 433 -> 114 us). */
 const uint32_t kStripThreads = 512;
 const uint32_t kBox = 32;                     /* rows and columns of a tensor-map box */
 const uint32_t kBoxBytes = kBox * kBox * 4u;  /* 4096 */
@@ -458,10 +464,10 @@ __device__ __forceinline__ void strip_fill_(const DistArgs& a, uint32_t p, uint3
 }
 
 /* one distance term, general form: the reference's conversions, and on
- * request the FP64 and exact integer sums and the prefix-sum output */
+ * request the FP64 and exact integer sums */
 template <bool F64, bool SSD>
 __device__ __forceinline__ void term_(uint32_t s, uint32_t o, float& a2, double& a2d, uint64_t& shi,
-                                      uint64_t& slo, uint32_t* cum, uint64_t at)
+                                      uint64_t& slo)
 {
     const float dd = __fsub_rn(__uint2float_rn(s), __uint2float_rn(o));
     a2 = __fadd_rn(a2, __fmul_rn(dd, dd));
@@ -473,13 +479,19 @@ __device__ __forceinline__ void term_(uint32_t s, uint32_t o, float& a2, double&
         const double d64 = __dsub_rn((double)s, (double)o);
         a2d = __dadd_rn(a2d, __dmul_rn(d64, d64));
     }
-    if (cum) cum[at] = s;
 }
 
 /* float(s) - float(o) for s, o < 2^22 (exact integer difference) */
 __device__ __forceinline__ float exact_diff_(uint32_t s, uint32_t o)
 {
     return __fsub_rn(__uint_as_float(0x4B400000u + s - o), 12582912.0f);
+}
+
+/* (s - o)^2 for s, o < 2^22: below 2^44 */
+__device__ __forceinline__ uint64_t square_(uint32_t s, uint32_t o)
+{
+    const int32_t d = (int32_t)(s - o);
+    return (uint64_t)((int64_t)d * d);
 }
 
 /* Cluster mode (k_distance_cluster), for launches where walking each
@@ -900,6 +912,10 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                 carry[r] = o.w;
             }
             __syncthreads();
+            /* the strip's prefix sums, a row segment of 128 bytes per warp (the
+             * lanes of phase B hold columns, whose cells lie B apart) */
+            if (cum && c0 + l < B)
+                for (uint32_t r = w; r < R; r += kStripThreads / 32u) cum[(uint64_t)r * B + c0 + l] = T[sw_(r, l)];
             /* phase B: columns c0 + 2w and c0 + 2w + 1; lane l reads rows
              * l, l + 32, ..., all congruent to l mod 8, so its swizzled
              * offset within a row is fixed */
@@ -911,8 +927,9 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                 float a2A = 0.0f, a2B = 0.0f;
                 double a2dA = 0.0, a2dB = 0.0;
                 /* the largest cumulative counts: the strip's and the observed histogram's last cells */
-                const bool exact = !F64 && !SSD && !cum && T[sw_(R - 1u, 31u)] < kExactBelow &&
+                const bool exact = T[sw_(R - 1u, 31u)] < kExactBelow &&
                                    __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
+                uint64_t iA = 0u, iB = 0u; /* exact sums of squares of the lane's rows */
                 if (exact && inB) {
                     const uint2* ref2 = reinterpret_cast<const uint2*>(refc);
 #pragma unroll 4
@@ -923,24 +940,39 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                         const float dB = exact_diff_(s.y, o.y);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
                         a2B = __fadd_rn(a2B, __fmul_rn(dB, dB));
+                        if (F64 || SSD) {
+                            iA += square_(s.x, o.x);
+                            iB += square_(s.y, o.y);
+                        }
                     }
                 } else if (exact) {
 #pragma unroll 4
                     for (uint32_t r = l; r < R; r += 32u) {
-                        const float dA = exact_diff_(Tl[r << 5], __ldg(refc + r));
+                        const uint32_t s = Tl[r << 5], o = __ldg(refc + r);
+                        const float dA = exact_diff_(s, o);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
+                        if (F64 || SSD) iA += square_(s, o);
                     }
                 } else {
                     for (uint32_t r = l; r < R; r += 32u) {
-                        const uint64_t at = (uint64_t)r * B + colA;
                         if (inB) {
                             const uint2 s = *reinterpret_cast<const uint2*>(Tl + (r << 5));
                             const uint2 o = __ldg(reinterpret_cast<const uint2*>(refc) + r);
-                            term_<F64, SSD>(s.x, o.x, a2A, a2dA, shi, slo, cum, at);
-                            term_<F64, SSD>(s.y, o.y, a2B, a2dB, shi, slo, cum, at + 1u);
+                            term_<F64, SSD>(s.x, o.x, a2A, a2dA, shi, slo);
+                            term_<F64, SSD>(s.y, o.y, a2B, a2dB, shi, slo);
                         } else {
-                            term_<F64, SSD>(Tl[r << 5], __ldg(refc + r), a2A, a2dA, shi, slo, cum, at);
+                            term_<F64, SSD>(Tl[r << 5], __ldg(refc + r), a2A, a2dA, shi, slo);
                         }
+                    }
+                }
+                if (exact) {
+                    if (F64) {
+                        a2dA = (double)iA;
+                        a2dB = (double)iB;
+                    }
+                    if (SSD) {
+                        add128_(shi, slo, 0u, iA);
+                        add128_(shi, slo, 0u, iB);
                     }
                 }
                 acc0 = __fadd_rn(acc0, a2A);
