@@ -700,10 +700,6 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         if (smem > 227u * 1024u) throw Error(PCS_ERR_UNSUPPORTED, "too many histogram rows for one CTA");
         cudaStream_t st = c.stream;
         DevTmp t;
-        std::vector<uint32_t> refT(RB);
-        for (uint32_t r = 0; r < rows; ++r)
-            for (uint32_t b = 0; b < bins; ++b)
-                refT[pcs_sat_t_index(r, b, rows, bins)] = ref_sat[(uint64_t)r * bins + b];
         uint32_t* d_hist = t.get<uint32_t>(count * RB);
         uint32_t* d_ref = t.get<uint32_t>(RB);
         uint32_t* d_refT = t.get<uint32_t>(RB);
@@ -711,34 +707,25 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         float* d_d32 = t.get<float>(count);
         double* d_d64 = dist_f64 ? t.get<double>(count) : nullptr;
         uint64_t* d_ssd = ssd ? t.get<uint64_t>(2ull * count) : nullptr;
-        JobDev jd{};
-        jd.R = rows;
-        jd.B = bins;
-        jd.ref_sat = d_ref;
-        jd.ref_sat_t = d_refT;
         TmapDev map;
-        jd.tmap_depth = encode_hist_tmap(&map, d_hist, rows, bins, count) ? count : 0u;
-        TmapDev* d_map = t.get<TmapDev>(1);
-        std::vector<PropDev> props(count);
-        for (uint32_t q = 0; q < count; ++q) {
-            std::memset(&props[q], 0, sizeof(PropDev));
-            props[q].hist_off = (uint64_t)q * RB;
-            props[q].hist_z = q;
-        }
-        JobDev* d_jobs = t.get<JobDev>(1);
-        PropDev* d_props = t.get<PropDev>(count);
-        uint32_t* d_n = t.get<uint32_t>(1);
+        DistSetup setup{};
+        setup.ref = d_ref;
+        setup.ref_t = d_refT;
+        setup.job = t.get<JobDev>(1);
+        setup.map = t.get<TmapDev>(1);
+        setup.props = t.get<PropDev>(count);
+        setup.n_props = t.get<uint32_t>(1);
+        setup.rows = rows;
+        setup.bins = bins;
+        setup.count = count;
+        setup.map_depth = encode_hist_tmap(&map, d_hist, rows, bins, count) ? count : 0u;
         PCS_CUDA(cudaMemcpyAsync(d_hist, hist, count * RB * 4, cudaMemcpyHostToDevice, st));
         PCS_CUDA(cudaMemcpyAsync(d_ref, ref_sat, RB * 4, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_refT, refT.data(), RB * 4, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_jobs, &jd, sizeof jd, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_map, &map, sizeof map, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_props, props.data(), sizeof(PropDev) * count, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_n, &count, 4, cudaMemcpyHostToDevice, st));
+        PCS_CUDA(launch_distance_setup(setup, map, st));
         DistArgs d{};
-        d.jobs = d_jobs;
-        d.props = d_props;
-        d.n_props = d_n;
+        d.jobs = setup.job;
+        d.props = setup.props;
+        d.n_props = setup.n_props;
         d.hist = d_hist;
         d.cum_out = d_cum;
         d.dist_f32 = d_d32;
@@ -746,7 +733,7 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         d.ssd = d_ssd;
         d.err = c.err.as<uint32_t>();
         d.max_rows = rows;
-        d.tmaps = d_map;
+        d.tmaps = setup.map;
         const uint32_t cl = (d_cum || d_d64 || d_ssd) ? 0u : distance_cluster_size(rows, bins);
         PCS_CUDA(launch_distance(d, std::min<uint32_t>(count, (uint32_t)(distance_ctas_per_sm(rows) * c.sm_count)), st, cl));
         if (cum_out) PCS_CUDA(cudaMemcpyAsync(cum_out, d_cum, count * RB * 4, cudaMemcpyDeviceToHost, st));

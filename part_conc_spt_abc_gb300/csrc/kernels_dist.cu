@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1129,6 +1130,69 @@ static cudaError_t cluster_fit_(cudaLaunchConfig_t& cfg, uint32_t cl, size_t sme
     std::lock_guard<std::mutex> g(mu);
     cache[key] = fit;
     return cudaSuccess;
+}
+
+/* Device-side set-up of a standalone distance launch: the descriptors of
+ * `count` consecutive histograms sharing one job, and the observed
+ * histogram's column-major copy (pairs of columns interleaved,
+ * pcs_sat_t_index) through tiles of 32 rows x 64 columns in shared memory,
+ * read in 256-byte rows and written in 256-byte runs of a pair (done cell by
+ * cell on the host it took 0.4 ms for 1001 x 256). */
+constexpr uint32_t kPropWords = sizeof(PropDev) / 4u;
+
+__global__ void __launch_bounds__(256) k_distance_setup(DistSetup d, const __grid_constant__ TmapDev map)
+{
+    __shared__ uint32_t s_t[32][65];
+    const uint32_t tid = threadIdx.x;
+    const uint32_t R = d.rows, B = d.bins;
+    if (blockIdx.x == 0u && tid == 0u) {
+        JobDev j;
+        memset(&j, 0, sizeof j);
+        j.R = R;
+        j.B = B;
+        j.ref_sat = d.ref;
+        j.ref_sat_t = d.ref_t;
+        j.tmap_depth = d.map_depth;
+        *d.job = j;
+        *d.map = map;
+        /* the map, for the tensor copies of the kernel that follows (which acquires it) */
+        asm volatile("fence.proxy.tensormap::generic.release.gpu;\n" ::: "memory");
+        *d.n_props = d.count;
+        if (d.err) *d.err = 0u;
+    }
+    /* the histograms' descriptors, word by word across the threads */
+    for (uint64_t i = (uint64_t)blockIdx.x * 256u + tid; i < (uint64_t)d.count * kPropWords; i += (uint64_t)gridDim.x * 256u) {
+        const uint32_t q = (uint32_t)(i / kPropWords), k = (uint32_t)(i % kPropWords);
+        const uint64_t off = (uint64_t)q * R * B;
+        uint32_t v = 0u;
+        if (k == offsetof(PropDev, hist_z) / 4u) v = q;
+        if (k == offsetof(PropDev, hist_off) / 4u) v = (uint32_t)off;
+        if (k == offsetof(PropDev, hist_off) / 4u + 1u) v = (uint32_t)(off >> 32);
+        reinterpret_cast<uint32_t*>(d.props)[i] = v;
+    }
+    const uint32_t tc = (B + 63u) / 64u, tr = (R + 31u) / 32u;
+    for (uint64_t t = blockIdx.x; t < (uint64_t)tc * tr; t += gridDim.x) {
+        const uint32_t r0 = (uint32_t)(t / tc) * 32u, c0 = (uint32_t)(t % tc) * 64u;
+        for (uint32_t i = tid; i < 2048u; i += 256u) {
+            const uint32_t r = r0 + i / 64u, c = c0 + i % 64u;
+            if (r < R && c < B) s_t[i / 64u][i % 64u] = d.ref[(uint64_t)r * B + c];
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < 2048u; i += 256u) {
+            const uint32_t k = i % 64u, x = 2u * (i / 64u) + (k & 1u);
+            const uint32_t r = r0 + k / 2u, c = c0 + x;
+            if (r < R && c < B) d.ref_t[pcs_sat_t_index(r, c, R, B)] = s_t[k / 2u][x];
+        }
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaStream_t st)
+{
+    const uint64_t tiles = (uint64_t)((d.bins + 63u) / 64u) * ((d.rows + 31u) / 32u);
+    const uint64_t blocks = std::max<uint64_t>(tiles, ((uint64_t)d.count * kPropWords + 1023u) / 1024u);
+    k_distance_setup<<<(unsigned)std::min<uint64_t>(blocks, 4096u), 256, 0, st>>>(d, map);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl)

@@ -67,48 +67,6 @@ constexpr size_t kScratchBytes = kHeaderBytes + kPropBytes + (size_t)PCS_NOALLOC
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
-/* Fills the scratch for one call: the histograms' tensor map (map_depth of
- * them; 0: none) and job descriptor, one descriptor per histogram (consecutive
- * R x B blocks of the caller's buffer), the proposal count, a cleared error
- * word, and the observed histogram's column-major copy (pairs of columns
- * interleaved, pcs_sat_t_index). */
-__global__ void k_noalloc_setup(const uint32_t* __restrict__ ref_sat, uint32_t rows, uint32_t bins,
-                                uint32_t count, const __grid_constant__ TmapDev map, uint32_t map_depth)
-{
-    NoallocHeader* h = reinterpret_cast<NoallocHeader*>(g_scratch);
-    PropDev* props = reinterpret_cast<PropDev*>(g_scratch + kHeaderBytes);
-    uint32_t* ref_t = reinterpret_cast<uint32_t*>(g_scratch + kHeaderBytes + kPropBytes);
-    const uint64_t cells = (uint64_t)rows * bins;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    if (tid == 0) {
-        JobDev j;
-        memset(&j, 0, sizeof j);
-        j.R = rows;
-        j.B = bins;
-        j.ref_sat = ref_sat;
-        j.ref_sat_t = ref_t;
-        j.tmap_depth = map_depth;
-        h->job = j;
-        h->map = map;
-        /* the map, for the tensor copies of the kernel that follows (which acquires it) */
-        asm volatile("fence.proxy.tensormap::generic.release.gpu;\n" ::: "memory");
-        h->n_props = count;
-        h->err = 0u;
-    }
-    for (uint64_t q = tid; q < count; q += stride) {
-        PropDev p;
-        memset(&p, 0, sizeof p);
-        p.hist_off = q * cells;
-        p.hist_z = (uint32_t)q;
-        props[q] = p;
-    }
-    for (uint64_t i = tid; i < cells; i += stride) {
-        const uint64_t r = i / bins, b = i % bins;
-        ref_t[pcs_sat_t_index((uint32_t)r, (uint32_t)b, rows, bins)] = ref_sat[i];
-    }
-}
-
 std::mutex g_mu;
 void* g_addr[64] = {};
 
@@ -158,22 +116,28 @@ extern "C" pcs_status pcs_scan_distance_noalloc(uint32_t* d_hist, const uint32_t
     if (e != cudaSuccess) return fail_(PCS_ERR_CUDA, std::string("scratch set-up: ") + cudaGetErrorString(e));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    const uint64_t cells = (uint64_t)rows * bins;
-    const uint32_t threads = 256;
-    uint64_t blocks = (cells + threads - 1) / threads;
-    if (blocks < (count + threads - 1) / threads) blocks = (count + threads - 1) / threads;
-    if (blocks > 4096) blocks = 4096;
-    TmapDev map;
-    const uint32_t depth = pcs::encode_hist_tmap(&map, d_hist, rows, bins, count) ? count : 0u;
-    k_noalloc_setup<<<(unsigned)blocks, threads, 0, st>>>(d_ref_sat, rows, bins, count, map, depth);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail_(PCS_ERR_CUDA, std::string("setup launch: ") + cudaGetErrorString(e));
-
     unsigned char* b = static_cast<unsigned char*>(base);
     NoallocHeader* h = reinterpret_cast<NoallocHeader*>(b);
+    PropDev* props = reinterpret_cast<PropDev*>(b + kHeaderBytes);
+    TmapDev map;
+    pcs::DistSetup setup{};
+    setup.ref = d_ref_sat;
+    setup.ref_t = reinterpret_cast<uint32_t*>(b + kHeaderBytes + kPropBytes);
+    setup.job = &h->job;
+    setup.map = &h->map;
+    setup.props = props;
+    setup.n_props = &h->n_props;
+    setup.err = &h->err;
+    setup.rows = rows;
+    setup.bins = bins;
+    setup.count = count;
+    setup.map_depth = pcs::encode_hist_tmap(&map, d_hist, rows, bins, count) ? count : 0u;
+    e = pcs::launch_distance_setup(setup, map, st);
+    if (e != cudaSuccess) return fail_(PCS_ERR_CUDA, std::string("setup launch: ") + cudaGetErrorString(e));
+
     pcs::DistArgs d{};
     d.jobs = &h->job;
-    d.props = reinterpret_cast<const PropDev*>(b + kHeaderBytes);
+    d.props = props;
     d.n_props = &h->n_props;
     d.hist = d_hist;
     d.cum_out = nullptr;

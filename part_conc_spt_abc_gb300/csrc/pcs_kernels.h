@@ -70,6 +70,21 @@ struct DistArgs {
     uint32_t max_rows;          /* rows of the carry array in shared memory */
     const TmapDev* tmaps;       /* nullable: per job (index of jobs), tensor maps over hist */
 };
+/* A standalone launch's tables, filled on the device (launch_distance_setup):
+ * one job of rows x bins, `count` consecutive histograms, the observed
+ * histogram `ref` copied to column-major ref_t. */
+struct DistSetup {
+    const uint32_t* ref;
+    uint32_t* ref_t;
+    JobDev* job;
+    TmapDev* map;
+    PropDev* props;    /* [count] */
+    uint32_t* n_props;
+    uint32_t* err;     /* nullable: cleared */
+    uint32_t rows, bins, count;
+    uint32_t map_depth; /* histograms the map spans (0: no map) */
+};
+cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaStream_t st);
 /* grid: CTAs at most (one histogram each).  cl > 1 (at least every job's
  * strips of 32 bins; 0 or 1: none) allows clusters of cl CTAs, one strip of
  * a histogram per CTA, which the launch takes where the histograms have at
