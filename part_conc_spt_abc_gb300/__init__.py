@@ -350,6 +350,12 @@ class ForwardRun:
     generation: int = 0
 
 
+def _components(values, fill: float):
+    """A per-component C array: the values, then `fill`."""
+    v = [float(x) for x in values[:MAX_COMPONENTS]]
+    return (C.c_float * MAX_COMPONENTS)(*v, *[fill] * (MAX_COMPONENTS - len(v)))
+
+
 def simulate_hist(ctx: Context, setup: ForwardSetup, runs, seed: int = 0, replay=None) -> np.ndarray:
     """Forward model of each run; returns uint32 [len(runs), R, B]."""
     if isinstance(runs, ForwardRun):
@@ -361,11 +367,10 @@ def simulate_hist(ctx: Context, setup: ForwardSetup, runs, seed: int = 0, replay
         parts = np.ascontiguousarray(r.particles, np.uint32)
         keep.append(parts)
         arr[i].particles = _p(parts, C.c_uint32)
-        for k in range(MAX_COMPONENTS):
-            arr[i].half_az[k] = float(r.half_az[k]) if k < len(r.half_az) else 0.0
-            arr[i].pre_comp_prob[k] = float(r.pre_comp_prob[k]) if k < len(r.pre_comp_prob) else 2.0
-            arr[i].sd_scale[k] = float(r.sd_scale[k]) if k < len(r.sd_scale) else 0.0
-            arr[i].sd_shape[k] = float(r.sd_shape[k]) if r.sd_shape is not None and k < len(r.sd_shape) else 0.0
+        arr[i].half_az = _components(r.half_az, 0.0)
+        arr[i].pre_comp_prob = _components(r.pre_comp_prob, 2.0)
+        arr[i].sd_scale = _components(r.sd_scale, 0.0)
+        arr[i].sd_shape = _components(r.sd_shape if r.sd_shape is not None else (), 0.0)
         arr[i].slot, arr[i].trial, arr[i].generation = r.slot, r.trial, r.generation
     rp = None
     if replay is not None:
@@ -375,7 +380,7 @@ def simulate_hist(ctx: Context, setup: ForwardSetup, runs, seed: int = 0, replay
         sig = np.ascontiguousarray(sig, np.float32) if sig is not None else None
         keep += [u, z, sig]
         rp = _lib.Replay(_p(u, C.c_float), _p(z, C.c_float), z.shape[1], _p(sig, C.c_float) if sig is not None else None)
-    out = np.zeros((len(runs), setup.rows, setup.de_bins), np.uint32)
+    out = np.empty((len(runs), setup.rows, setup.de_bins), np.uint32)  # every cell is written
     check(lib().pcs_simulate_hist(ctx.h, C.byref(s), arr, len(runs), seed, C.byref(rp) if rp is not None else None,
                                   _p(out, C.c_uint32)), "pcs_simulate_hist")
     return out
@@ -389,10 +394,10 @@ def scan_distance(ctx: Context, hist: np.ndarray, ref_sat: np.ndarray, want_cum:
         h = h[None]
     n, R, B = h.shape
     ref = np.ascontiguousarray(ref_sat, np.uint32)
-    cum = np.zeros_like(h) if want_cum else None
-    d32 = np.zeros(n, np.float32)
-    d64 = np.zeros(n, np.float64) if want_f64 else None
-    ssd = np.zeros((n, 2), np.uint64) if want_ssd else None
+    cum = np.empty_like(h) if want_cum else None  # every output is written whole
+    d32 = np.empty(n, np.float32)
+    d64 = np.empty(n, np.float64) if want_f64 else None
+    ssd = np.empty((n, 2), np.uint64) if want_ssd else None
     check(lib().pcs_scan_distance(ctx.h, _p(h, C.c_uint32), _p(ref, C.c_uint32), R, B, n,
                                   _p(cum, C.c_uint32) if cum is not None else None, _p(d32, C.c_float),
                                   _p(d64, C.c_double) if d64 is not None else None,
@@ -412,7 +417,7 @@ def observed_sat(ctx: Context, K, DE, rows: int, bins: int, ub_de: float, julia:
     path's conventions (rows = kmax for K = 1..kmax, ceil binning)."""
     K = np.ascontiguousarray(K, np.uint32)
     DE = np.ascontiguousarray(DE, np.float64)
-    out = np.zeros((rows, bins), np.uint32)
+    out = np.empty((rows, bins), np.uint32)  # every cell is written
     fn = lib().pcs_observed_sat_julia if julia else lib().pcs_observed_sat
     check(fn(ctx.h, _p(K, C.c_uint32), _p(DE, C.c_double), len(K), rows, bins, ub_de, _p(out, C.c_uint32)),
           "pcs_observed_sat")

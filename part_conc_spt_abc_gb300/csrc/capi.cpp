@@ -62,31 +62,39 @@ Job& J_(pcs_job* j)
     return *j->impl;
 }
 
-struct DevTmp {
-    std::vector<DevBuf*> bufs;
-    ~DevTmp()
-    {
-        for (auto* b : bufs) delete b;
-    }
-    template <class T>
-    T* get(size_t n)
-    {
-        DevBuf* b = new DevBuf();
-        bufs.push_back(b);
-        b->alloc(std::max<size_t>(n, 1) * sizeof(T));
-        return b->as<T>();
-    }
-};
-
-void check_err_word(Ctx& c)
+/* The end of a standalone call: waits for its work, then reports the device
+ * error word, which is read in the same wait. */
+void finish(Ctx& c, Lease& ws)
 {
-    uint32_t bits = 0;
-    PCS_CUDA(cudaMemcpy(&bits, c.err.p, 4, cudaMemcpyDeviceToHost));
-    if (bits) {
+    uint32_t word = 0;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(ws.stage(4));
+    if (!bits) bits = &word;
+    PCS_CUDA(cudaMemcpyAsync(bits, c.err.p, 4, cudaMemcpyDeviceToHost, c.stream));
+    PCS_CUDA(cudaStreamSynchronize(c.stream));
+    ws.done();
+    if (*bits) {
         PCS_CUDA(cudaMemset(c.err.p, 0, 16));
-        throw Error(PCS_ERR_DEVICE, "device error word 0x" + std::to_string(bits));
+        throw Error(PCS_ERR_DEVICE, "device error word 0x" + std::to_string(*bits));
     }
 }
+
+/* A small result: read into the pinned page where there is room (take()
+ * hands it on after finish()), else straight into the caller's memory. */
+struct Fetch {
+    void* to = nullptr;
+    char* staged = nullptr;
+    size_t bytes = 0;
+    Fetch(Ctx& c, Lease& ws, void* host, const void* dev, size_t n) : to(host), bytes(n)
+    {
+        if (!to) return;
+        staged = ws.stage(n);
+        PCS_CUDA(cudaMemcpyAsync(staged ? staged : to, dev, n, cudaMemcpyDeviceToHost, c.stream));
+    }
+    void take() const
+    {
+        if (to && staged) std::memcpy(to, staged, bytes);
+    }
+};
 
 } // namespace
 
@@ -491,6 +499,8 @@ pcs_status pcs_serve_step(pcs_ctx* ctx, uint32_t* active)
             const uint64_t need_total = c.mem_used + j->arena_bytes() + hist_b;
             const uint64_t need_b = j->arena_bytes() + (uint64_t)c.tune.capacity * j->R * j->B * 4ull;
             const bool over_cap = c.mem_cap && need_total > c.mem_cap;
+            if (!over_cap && need_b + (64ull << 20) > (uint64_t)free_b && c.release_workspace())
+                PCS_CUDA(cudaMemGetInfo(&free_b, &total_b));
             if (over_cap || need_b + (64ull << 20) > (uint64_t)free_b) {
                 if (used == 0) throw Error(PCS_ERR_OUT_OF_MEMORY, "job does not fit in device memory");
                 break;
@@ -564,7 +574,41 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
         if (RB > (1ull << 31)) throw Error(PCS_ERR_UNSUPPORTED, "histogram too large");
 
         cudaStream_t st = c.stream;
-        DevTmp t;
+        const uint32_t chunk = c.tune.chunk;
+        const uint64_t cstride = 2ull * V + 1ull;
+        uint64_t n_items = 0;
+        std::vector<uint32_t> totals(count);
+        for (uint32_t q = 0; q < count; ++q) {
+            need(runs[q].particles, "run.particles");
+            uint64_t total = 0;
+            for (uint32_t v = 0; v < V; ++v) total += runs[q].particles[v];
+            if (total > 0xFFFFFFFFull) throw Error(PCS_ERR_INVALID_ARGUMENT, "too many particles");
+            totals[q] = (uint32_t)total;
+            n_items += (total + chunk - 1) / chunk;
+        }
+        if (replay) {
+            need(replay->uniforms, "replay->uniforms");
+            need(replay->normals, "replay->normals");
+            if (replay->normal_stride + 1 < fmax) throw Error(PCS_ERR_INVALID_ARGUMENT, "replay normal_stride < frames - 1");
+            if (setup->model == PCS_MODEL_LOGNORMAL) need(replay->sigmas, "replay->sigmas");
+        }
+        /* the inputs, laid out alike on the host and on the device: one copy */
+        const size_t o_frames = Lease::need<JobDev>(1), o_ctl = o_frames + Lease::need<uint32_t>(V),
+                     o_props = o_ctl + Lease::need<uint32_t>(2), o_counts = o_props + Lease::need<PropDev>(count),
+                     o_items = o_counts + Lease::need<uint32_t>(count * cstride),
+                     in_bytes = o_items + Lease::need<uint32_t>(n_items);
+        const uint64_t rp_n = replay ? totals[0] : 0u, rp_steps = replay ? replay->normal_stride : 0u;
+        Lease ws(c, in_bytes + Lease::need<uint32_t>(count * RB) + Lease::need<float>(4 * rp_n) +
+                        Lease::need<float>(3 * rp_n * rp_steps) + Lease::need<float>(rp_n));
+        char* d_in = ws.get<char>(in_bytes);
+        uint32_t* d_hist = ws.get<uint32_t>(count * RB);
+        std::vector<char> pageable;
+        char* h_in = ws.stage(in_bytes);
+        if (!h_in) {
+            pageable.resize(in_bytes);
+            h_in = pageable.data();
+        }
+
         JobDev jd{};
         jd.half_lx = setup->half_lx;
         jd.half_ly = setup->half_ly;
@@ -582,18 +626,17 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
         jd.Z = setup->model == PCS_MODEL_DISCRETE_VARIABLE_DEPTH ? Cc : 1u;
         pcs_seed_masks(seed, &jd.seed_lo, &jd.seed_hi);
         jd.frames_max = fmax;
-        uint32_t* d_frames = t.get<uint32_t>(V);
-        PCS_CUDA(cudaMemcpyAsync(d_frames, setup->frames, V * 4u, cudaMemcpyHostToDevice, st));
-        jd.frames = d_frames;
-
-        const uint32_t chunk = c.tune.chunk;
-        const uint64_t cstride = 2ull * V + 1ull;
-        std::vector<PropDev> props(count);
-        std::vector<uint32_t> counts(count * cstride);
-        std::vector<uint32_t> item_prop;
+        jd.frames = reinterpret_cast<uint32_t*>(d_in + o_frames);
+        std::memcpy(h_in, &jd, sizeof jd);
+        std::memcpy(h_in + o_frames, setup->frames, V * 4u);
+        uint32_t* ctl = reinterpret_cast<uint32_t*>(h_in + o_ctl);
+        ctl[0] = (uint32_t)n_items;
+        ctl[1] = 0u;
+        PropDev* props = reinterpret_cast<PropDev*>(h_in + o_props);
+        uint32_t* items = reinterpret_cast<uint32_t*>(h_in + o_items);
+        uint32_t at = 0u;
         for (uint32_t q = 0; q < count; ++q) {
             const pcs_run& r = runs[q];
-            need(r.particles, "run.particles");
             PropDev& pd = props[q];
             std::memset(&pd, 0, sizeof pd);
             pd.job = 0;
@@ -607,64 +650,46 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
                 pd.sd_shape[i] = r.sd_shape[i];
             }
             uint64_t total = 0;
-            uint32_t* cnt = counts.data() + q * cstride;
+            uint32_t* cnt = reinterpret_cast<uint32_t*>(h_in + o_counts) + q * cstride;
             cnt[V] = 0;
             for (uint32_t v = 0; v < V; ++v) {
                 cnt[v] = r.particles[v];
                 total += r.particles[v];
                 cnt[V + 1 + v] = (uint32_t)total;
             }
-            if (total > 0xFFFFFFFFull) throw Error(PCS_ERR_INVALID_ARGUMENT, "too many particles");
-            pd.total_particles = (uint32_t)total;
+            pd.total_particles = totals[q];
             pd.counts_off = q * cstride;
             pd.hist_off = (uint64_t)q * RB;
-            pd.item_begin = (uint32_t)item_prop.size();
-            pd.item_count = (uint32_t)((total + chunk - 1) / chunk);
-            for (uint32_t i = 0; i < pd.item_count; ++i) item_prop.push_back(q);
+            pd.item_begin = at;
+            pd.item_count = (uint32_t)(((uint64_t)totals[q] + chunk - 1) / chunk);
+            std::fill_n(items + at, pd.item_count, q);
+            at += pd.item_count;
         }
-        if (replay) {
-            need(replay->uniforms, "replay->uniforms");
-            need(replay->normals, "replay->normals");
-            if (replay->normal_stride + 1 < fmax) throw Error(PCS_ERR_INVALID_ARGUMENT, "replay normal_stride < frames - 1");
-            if (setup->model == PCS_MODEL_LOGNORMAL) need(replay->sigmas, "replay->sigmas");
-        }
-        JobDev* d_jobs = t.get<JobDev>(1);
-        PropDev* d_props = t.get<PropDev>(count);
-        uint32_t* d_counts = t.get<uint32_t>(counts.size());
-        uint32_t* d_items = t.get<uint32_t>(item_prop.size());
-        uint32_t* d_ctl = t.get<uint32_t>(2);
-        uint32_t* d_hist = t.get<uint32_t>(count * RB);
-        uint32_t ctl[2] = {(uint32_t)item_prop.size(), 0u};
-        PCS_CUDA(cudaMemcpyAsync(d_jobs, &jd, sizeof jd, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_props, props.data(), sizeof(PropDev) * count, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_counts, counts.data(), counts.size() * 4, cudaMemcpyHostToDevice, st));
-        if (!item_prop.empty())
-            PCS_CUDA(cudaMemcpyAsync(d_items, item_prop.data(), item_prop.size() * 4, cudaMemcpyHostToDevice, st));
-        PCS_CUDA(cudaMemcpyAsync(d_ctl, ctl, 8, cudaMemcpyHostToDevice, st));
+        PCS_CUDA(cudaMemcpyAsync(d_in, h_in, in_bytes, cudaMemcpyHostToDevice, st));
         PCS_CUDA(cudaMemsetAsync(d_hist, 0, count * RB * 4, st));
 
         SimArgs a{};
-        a.jobs = d_jobs;
-        a.props = d_props;
-        a.counts = d_counts;
+        a.jobs = reinterpret_cast<JobDev*>(d_in);
+        a.props = reinterpret_cast<PropDev*>(d_in + o_props);
+        a.counts = reinterpret_cast<uint32_t*>(d_in + o_counts);
         a.hist = d_hist;
-        a.item_prop = d_items;
-        a.n_items = d_ctl;
-        a.queue_head = d_ctl + 1;
+        a.item_prop = reinterpret_cast<uint32_t*>(d_in + o_items);
+        a.n_items = reinterpret_cast<uint32_t*>(d_in + o_ctl);
+        a.queue_head = reinterpret_cast<uint32_t*>(d_in + o_ctl) + 1;
         a.chunk = chunk;
         a.err = c.err.as<uint32_t>();
         a.tile_words = tile_words_for(std::min<uint32_t>(c.tune.tile_rows, R), B);
         if (replay) {
-            const uint64_t n = props[0].total_particles;
-            float* du = t.get<float>(4 * n);
-            float* dn = t.get<float>((uint64_t)n * replay->normal_stride * 3);
+            const uint64_t n = rp_n;
+            float* du = ws.get<float>(4 * n);
+            float* dn = ws.get<float>(3 * n * rp_steps);
             PCS_CUDA(cudaMemcpyAsync(du, replay->uniforms, 16 * n, cudaMemcpyHostToDevice, st));
             PCS_CUDA(cudaMemcpyAsync(dn, replay->normals, 12ull * n * replay->normal_stride, cudaMemcpyHostToDevice, st));
             a.rp_uniforms = du;
             a.rp_normals = dn;
             a.rp_stride = replay->normal_stride;
             if (replay->sigmas) {
-                float* ds = t.get<float>(n);
+                float* ds = ws.get<float>(n);
                 PCS_CUDA(cudaMemcpyAsync(ds, replay->sigmas, 4 * n, cudaMemcpyHostToDevice, st));
                 a.rp_sigmas = ds;
             }
@@ -679,8 +704,7 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
         l.grid = (uint32_t)std::max(1, occ) * (uint32_t)c.sm_count;
         PCS_CUDA(launch_simulate(a, l, st));
         PCS_CUDA(cudaMemcpyAsync(hist_out, d_hist, count * RB * 4, cudaMemcpyDeviceToHost, st));
-        PCS_CUDA(cudaStreamSynchronize(st));
-        check_err_word(c);
+        finish(c, ws);
     });
 }
 
@@ -699,22 +723,25 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         const size_t smem = distance_smem_bytes(rows);
         if (smem > 227u * 1024u) throw Error(PCS_ERR_UNSUPPORTED, "too many histogram rows for one CTA");
         cudaStream_t st = c.stream;
-        DevTmp t;
-        uint32_t* d_hist = t.get<uint32_t>(count * RB);
-        uint32_t* d_ref = t.get<uint32_t>(RB);
-        uint32_t* d_refT = t.get<uint32_t>(RB);
-        uint32_t* d_cum = cum_out ? t.get<uint32_t>(count * RB) : nullptr;
-        float* d_d32 = t.get<float>(count);
-        double* d_d64 = dist_f64 ? t.get<double>(count) : nullptr;
-        uint64_t* d_ssd = ssd ? t.get<uint64_t>(2ull * count) : nullptr;
+        Lease ws(c, Lease::need<uint32_t>(count * RB) * (cum_out ? 2u : 1u) + 2u * Lease::need<uint32_t>(RB) +
+                        Lease::need<float>(count) + Lease::need<double>(count) + Lease::need<uint64_t>(2ull * count) +
+                        Lease::need<JobDev>(1) + Lease::need<TmapDev>(1) + Lease::need<PropDev>(count) +
+                        Lease::need<uint32_t>(1));
+        uint32_t* d_hist = ws.get<uint32_t>(count * RB);
+        uint32_t* d_ref = ws.get<uint32_t>(RB);
+        uint32_t* d_refT = ws.get<uint32_t>(RB);
+        uint32_t* d_cum = cum_out ? ws.get<uint32_t>(count * RB) : nullptr;
+        float* d_d32 = ws.get<float>(count);
+        double* d_d64 = dist_f64 ? ws.get<double>(count) : nullptr;
+        uint64_t* d_ssd = ssd ? ws.get<uint64_t>(2ull * count) : nullptr;
         TmapDev map;
         DistSetup setup{};
         setup.ref = d_ref;
         setup.ref_t = d_refT;
-        setup.job = t.get<JobDev>(1);
-        setup.map = t.get<TmapDev>(1);
-        setup.props = t.get<PropDev>(count);
-        setup.n_props = t.get<uint32_t>(1);
+        setup.job = ws.get<JobDev>(1);
+        setup.map = ws.get<TmapDev>(1);
+        setup.props = ws.get<PropDev>(count);
+        setup.n_props = ws.get<uint32_t>(1);
         setup.rows = rows;
         setup.bins = bins;
         setup.count = count;
@@ -737,11 +764,13 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         const uint32_t cl = (d_cum || d_d64 || d_ssd) ? 0u : distance_cluster_size(rows, bins);
         PCS_CUDA(launch_distance(d, std::min<uint32_t>(count, (uint32_t)(distance_ctas_per_sm(rows) * c.sm_count)), st, cl));
         if (cum_out) PCS_CUDA(cudaMemcpyAsync(cum_out, d_cum, count * RB * 4, cudaMemcpyDeviceToHost, st));
-        PCS_CUDA(cudaMemcpyAsync(dist_f32, d_d32, count * 4, cudaMemcpyDeviceToHost, st));
-        if (dist_f64) PCS_CUDA(cudaMemcpyAsync(dist_f64, d_d64, count * 8, cudaMemcpyDeviceToHost, st));
-        if (ssd) PCS_CUDA(cudaMemcpyAsync(ssd, d_ssd, 16ull * count, cudaMemcpyDeviceToHost, st));
-        PCS_CUDA(cudaStreamSynchronize(st));
-        check_err_word(c);
+        const Fetch f32(c, ws, dist_f32, d_d32, (size_t)count * 4);
+        const Fetch f64(c, ws, dist_f64, d_d64, (size_t)count * 8);
+        const Fetch fss(c, ws, ssd, d_ssd, (size_t)count * 16);
+        finish(c, ws);
+        f32.take();
+        f64.take();
+        fss.take();
     });
 }
 
@@ -754,19 +783,18 @@ pcs_status pcs_observed_sat(pcs_ctx* ctx, const uint32_t* K, const double* DE, s
         if (n && (!K || !DE)) throw Error(PCS_ERR_INVALID_ARGUMENT, "K/DE are NULL");
         if (rows == 0 || bins == 0) throw Error(PCS_ERR_INVALID_ARGUMENT, "rows and bins must be positive");
         cudaStream_t st = c.stream;
-        DevTmp t;
         const uint64_t RB = (uint64_t)rows * bins;
-        uint32_t* dK = t.get<uint32_t>(n);
-        double* dDE = t.get<double>(n);
-        uint32_t* dS = t.get<uint32_t>(RB);
+        Lease ws(c, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
+        uint32_t* dK = ws.get<uint32_t>(n);
+        double* dDE = ws.get<double>(n);
+        uint32_t* dS = ws.get<uint32_t>(RB);
         if (n) {
             PCS_CUDA(cudaMemcpyAsync(dK, K, n * 4, cudaMemcpyHostToDevice, st));
             PCS_CUDA(cudaMemcpyAsync(dDE, DE, n * 8, cudaMemcpyHostToDevice, st));
         }
         PCS_CUDA(launch_observed_sat(dK, dDE, n, rows, bins, ub_de, dS, nullptr, c.err.as<uint32_t>(), st));
         PCS_CUDA(cudaMemcpyAsync(sat_out, dS, RB * 4, cudaMemcpyDeviceToHost, st));
-        PCS_CUDA(cudaStreamSynchronize(st));
-        check_err_word(c);
+        finish(c, ws);
     });
 }
 
@@ -779,19 +807,18 @@ pcs_status pcs_observed_sat_julia(pcs_ctx* ctx, const uint32_t* K, const double*
         if (n && (!K || !DE)) throw Error(PCS_ERR_INVALID_ARGUMENT, "K/DE are NULL");
         if (kmax == 0 || bins == 0) throw Error(PCS_ERR_INVALID_ARGUMENT, "kmax and bins must be positive");
         cudaStream_t st = c.stream;
-        DevTmp t;
         const uint64_t RB = (uint64_t)kmax * bins;
-        uint32_t* dK = t.get<uint32_t>(n);
-        double* dDE = t.get<double>(n);
-        uint32_t* dS = t.get<uint32_t>(RB);
+        Lease ws(c, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
+        uint32_t* dK = ws.get<uint32_t>(n);
+        double* dDE = ws.get<double>(n);
+        uint32_t* dS = ws.get<uint32_t>(RB);
         if (n) {
             PCS_CUDA(cudaMemcpyAsync(dK, K, n * 4, cudaMemcpyHostToDevice, st));
             PCS_CUDA(cudaMemcpyAsync(dDE, DE, n * 8, cudaMemcpyHostToDevice, st));
         }
         PCS_CUDA(launch_observed_sat_julia(dK, dDE, n, kmax, bins, ub_de, dS, c.err.as<uint32_t>(), st));
         PCS_CUDA(cudaMemcpyAsync(sat_out, dS, RB * 4, cudaMemcpyDeviceToHost, st));
-        PCS_CUDA(cudaStreamSynchronize(st));
-        check_err_word(c);
+        finish(c, ws);
     });
 }
 
@@ -801,10 +828,10 @@ pcs_status pcs_debug_particle_stream(pcs_ctx* ctx, uint64_t seed, uint32_t slot,
     return guard([&] {
         Ctx& c = C_(ctx);
         need(out, "out");
-        DevTmp t;
-        uint32_t* d = t.get<uint32_t>(4);
-        PCS_CUDA(launch_debug_stream(seed, slot, generation, trial, particle, block, d, c.stream));
-        PCS_CUDA(cudaMemcpyAsync(out, d, 16, cudaMemcpyDeviceToHost, c.stream));
+        DevBuf d;
+        d.alloc(16);
+        PCS_CUDA(launch_debug_stream(seed, slot, generation, trial, particle, block, d.as<uint32_t>(), c.stream));
+        PCS_CUDA(cudaMemcpyAsync(out, d.p, 16, cudaMemcpyDeviceToHost, c.stream));
         PCS_CUDA(cudaStreamSynchronize(c.stream));
     });
 }

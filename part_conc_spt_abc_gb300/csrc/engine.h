@@ -49,6 +49,45 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+struct Ctx;
+
+/* Memory that the standalone entry points keep between calls: device memory
+ * up to kKeep bytes (allocating and freeing nine buffers took 30-40 us of a
+ * 90 us call) and a pinned page for small transfers.  One call at a time
+ * holds it (Lease); a call that finds it taken by another thread, or needs
+ * more, allocates its own for the call.  Given back at pcs_close, and when
+ * an allocation of the context's jobs fails (Ctx::alloc). */
+struct Workspace {
+    static const size_t kKeep = 64ull << 20, kPinned = 64ull << 10;
+    std::mutex mu;
+    DevBuf dev;
+    char* pinned = nullptr;
+};
+
+class Lease {
+public:
+    /* bytes: the sum of need<T>(n) over the get<T>(n) that follow */
+    Lease(Ctx& c, size_t bytes);
+    ~Lease();
+    Lease(const Lease&) = delete;
+    Lease& operator=(const Lease&) = delete;
+    template <class T> static size_t need(size_t n) { return (n * sizeof(T) + 255u) / 256u * 256u; }
+    template <class T> T* get(size_t n) { return static_cast<T*>(take(need<T>(n))); }
+    /* pinned memory for `n` bytes of this call, or NULL (none left, or taken) */
+    char* stage(size_t n);
+    /* the call's work on the stream has completed */
+    void done() { done_ = true; }
+
+private:
+    void* take(size_t bytes);
+    Ctx& c_;
+    std::unique_lock<std::mutex> held_;
+    DevBuf own_;
+    char* base_ = nullptr;
+    size_t size_ = 0, used_ = 0, staged_ = 0;
+    bool done_ = false;
+};
+
 struct Tuning {
     uint32_t block = 256;
     uint32_t ppt = 1;
@@ -84,6 +123,7 @@ struct Ctx {
     DevBuf sim_tasks;        /* slab-split task counter (u64, cumulative) */
     DevBuf logfact;          /* [kLogFactEntries] log(k!) from the host's lgamma */
     uint64_t sim_tasks_base = 0;
+    Workspace ws;
     uint32_t* h_err = nullptr;
     RoundBufs rb;
     JobPmcDev* h_status = nullptr; /* pinned mirror of the pmc table */
@@ -106,6 +146,11 @@ struct Ctx {
 
     explicit Ctx(int dev, int inflight);
     ~Ctx();
+
+    /* b.alloc(n); if that fails, once more with the workspace given back */
+    void alloc(DevBuf& b, size_t n);
+    /* frees the workspace's device memory; false if there is none or a call holds it */
+    bool release_workspace();
 
     /* round machinery */
     void ensure_round_buffers(uint32_t v_max, uint32_t max_rows, uint32_t max_n, uint64_t rb_max);
