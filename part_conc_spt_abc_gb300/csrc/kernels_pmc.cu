@@ -41,32 +41,59 @@ namespace pcs {
 
 namespace {
 
-__device__ uint32_t job_of_(const RoundDev* rd, uint32_t q)
+/* the job whose range of the round's proposals holds q (a warp's lanes look
+ * at two jobs each) */
+__device__ __forceinline__ uint32_t job_of_(const RoundDev* rd, uint32_t q, uint32_t lane)
 {
-    uint32_t j = 0;
-    for (uint32_t i = 1; i < rd->n_jobs; ++i)
-        if (rd->job_base[i] <= q && rd->job_count[i] > 0) j = i;
-    /* job_base is non-decreasing; pick the last job whose range contains q */
-    for (uint32_t i = 0; i < rd->n_jobs; ++i)
-        if (q >= rd->job_base[i] && q < rd->job_base[i] + rd->job_count[i]) return i;
-    return j;
+    static_assert(kMaxRoundJobs <= 64u, "two jobs per lane");
+    const uint32_t n = rd->n_jobs;
+    uint32_t found = 0u;
+#pragma unroll
+    for (uint32_t h = 0; h < 2u; ++h) {
+        const uint32_t i = lane + 32u * h;
+        if (i < n && q >= rd->job_base[i] && q - rd->job_base[i] < rd->job_count[i]) found |= 1u << h;
+    }
+    const unsigned m0 = __ballot_sync(0xFFFFFFFFu, found & 1u), m1 = __ballot_sync(0xFFFFFFFFu, found & 2u);
+    return m0 ? (uint32_t)__ffs(m0) - 1u : (m1 ? 31u + (uint32_t)__ffs(m1) : 0u);
 }
 
 } // namespace
 
 /* ----------------------------------------------------------------------- */
-__global__ void k_round_plan(PmcArgs a)
+/* One thread per job computes the job's share (divisions and dependent loads
+ * of 64 jobs side by side instead of one after another: 4 jobs 20 -> 9 us);
+ * thread 0 adds up what depends on the jobs before. */
+__global__ void __launch_bounds__(kMaxRoundJobs) k_round_plan(PmcArgs a)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ double s_planned[kMaxRoundJobs], s_key[kMaxRoundJobs];
+    __shared__ uint64_t s_rb[kMaxRoundJobs], s_hbase[kMaxRoundJobs];
+    __shared__ uint32_t s_pend[kMaxRoundJobs], s_k[kMaxRoundJobs], s_base[kMaxRoundJobs], s_cnt[kMaxRoundJobs];
+    __shared__ uint8_t s_ord[kMaxRoundJobs], s_spec[kMaxRoundJobs];
+    __shared__ uint32_t s_kmax;
+    __shared__ double s_fill;
+    const uint32_t j = threadIdx.x;
     RoundDev* rd = a.round;
-    uint64_t total_pending = 0;
-    for (uint32_t j = 0; j < rd->n_jobs; ++j) {
-        const JobPmcDev& pm = a.pmc[j];
-        if (!pm.done) total_pending += pm.pending_count;
+    const uint32_t nj = min(rd->n_jobs, kMaxRoundJobs);
+    const bool have = j < nj;
+    const JobPmcDev& pm = a.pmc[have ? j : 0u];
+    const bool live = have && !pm.done;
+    const uint32_t pend = live ? pm.pending_count : 0u, gen = pm.generation;
+    const double accepted = (double)pm.accepted_gen, trials = (double)pm.trials;
+    const double sims = (double)pm.simulations, steps = (double)pm.particle_steps;
+    s_pend[j] = pend;
+    s_rb[j] = have ? (uint64_t)a.jobs[j].R * a.jobs[j].B : 0u;
+    const double fmax_j = (double)max(have ? a.jobs[j].frames_max : 1u, 1u);
+    __syncthreads();
+    if (j == 0u) {
+        uint64_t total_pending = 0;
+        for (uint32_t i = 0; i < nj; ++i) total_pending += s_pend[i];
+        uint32_t k = total_pending ? (uint32_t)(rd->capacity / total_pending) : 1u;
+        if (k < 1u) k = 1u;
+        if (k > rd->max_spec) k = rd->max_spec;
+        s_kmax = k;
     }
-    uint32_t k = total_pending ? (uint32_t)(rd->capacity / total_pending) : 1u;
-    if (k < 1u) k = 1u;
-    if (k > rd->max_spec) k = rd->max_spec;
+    __syncthreads();
+    const uint32_t k = s_kmax;
     /* trials per pending slot: enough to fill the round, but not many more
      * than ~0.3 / (acceptance rate so far), so that few trials are simulated
      * after a slot's first acceptance -- unless the round's proposals would
@@ -74,99 +101,92 @@ __global__ void k_round_plan(PmcArgs a)
      * launch; at the end of a generation few slots are left and the GPU
      * would idle), in which case the slots get proportionally more trials,
      * up to k.  Particles per proposal are estimated from the job's history. */
-    uint32_t kjs[kMaxRoundJobs];
-    double planned = 0.0;
-    uint64_t pend_spec = 0;
-    for (uint32_t j = 0; j < rd->n_jobs && j < kMaxRoundJobs; ++j) {
-        const JobPmcDev& pm = a.pmc[j];
-        uint32_t kj = k;
-        if (pm.generation == 0u) {
-            kj = 1u; /* prior pass: one simulation per slot */
-        } else {
-            const double pacc = ((double)pm.accepted_gen + 1.0) / ((double)pm.trials + 2.0);
-            const double kw = ceil(0.3 / pacc);
-            if (kw < (double)kj) kj = (uint32_t)(kw < 1.0 ? 1.0 : kw);
-            if (!pm.done) pend_spec += pm.pending_count;
-        }
-        kjs[j] = kj;
-        if (!pm.done) {
-            /* particles per proposal so far (steps over the longest video) */
-            const double ppp = pm.simulations ? (double)pm.particle_steps / (double)pm.simulations /
-                                                    (double)max(a.jobs[j].frames_max, 1u)
-                                              : (double)rd->fill;
-            planned += (double)pm.pending_count * kj * ppp;
-        }
+    const double pacc = (accepted + 1.0) / (trials + 2.0);
+    uint32_t kj = k;
+    if (gen == 0u) {
+        kj = 1u; /* prior pass: one simulation per slot */
+    } else {
+        const double kw = ceil(0.3 / pacc);
+        if (kw < (double)kj) kj = (uint32_t)(kw < 1.0 ? 1.0 : kw);
     }
-    if (rd->fill && planned < (double)rd->fill && pend_spec > 0) {
-        const double f = planned > 0.0 ? (double)rd->fill / planned : (double)k;
-        for (uint32_t j = 0; j < rd->n_jobs && j < kMaxRoundJobs; ++j)
-            if (a.pmc[j].generation > 0u && !a.pmc[j].done)
-                kjs[j] = (uint32_t)min((double)k, fmax((double)kjs[j], ceil((double)kjs[j] * f)));
-    }
+    /* particles per proposal so far (steps over the longest video) */
+    const double spp = steps / sims;
+    const double ppp = pm.simulations ? spp / fmax_j : (double)rd->fill;
+    s_planned[j] = (double)pend * kj * ppp;
+    s_spec[j] = live && gen > 0u && pend > 0u;
     /* the order in which jobs take the round's capacity: admission order, or
      * (order == 1) jobs in their prior pass first, then the least estimated
      * remaining work first -- (pending slots + slots of the generations left)
      * x particle-steps per proposal / acceptance rate -- which lets short
      * jobs finish early instead of waiting behind long ones */
-    uint32_t ord[kMaxRoundJobs];
-    double key[kMaxRoundJobs];
-    const uint32_t nj = min(rd->n_jobs, kMaxRoundJobs);
-    for (uint32_t j = 0; j < nj; ++j) {
-        const JobPmcDev& pm = a.pmc[j];
-        double kv = (double)j;
-        if (rd->order == 1u && pm.generation > 0u && !pm.done) {
-            const double pacc = ((double)pm.accepted_gen + 1.0) / ((double)pm.trials + 2.0);
-            const double spp = pm.simulations ? (double)pm.particle_steps / (double)pm.simulations : 1.0;
-            const double gens_left =
-                pm.max_generations ? fmax(0.0, (double)pm.max_generations - (double)pm.iterations) : 8.0;
-            kv = 1e6 + ((double)pm.pending_count + (double)pm.N * gens_left) * spp / pacc;
-        }
-        key[j] = kv;
-        uint32_t x = j;
-        while (x > 0 && key[ord[x - 1]] > kv) {
-            ord[x] = ord[x - 1];
-            --x;
-        }
-        ord[x] = j;
+    double kv = (double)j;
+    if (rd->order == 1u && gen > 0u && live) {
+        const double gens_left =
+            pm.max_generations ? fmax(0.0, (double)pm.max_generations - (double)pm.iterations) : 8.0;
+        kv = 1e6 + ((double)pend + (double)pm.N * gens_left) * (pm.simulations ? spp : 1.0) / pacc;
     }
-    for (uint32_t j = nj; j < rd->n_jobs; ++j) {
-        rd->job_base[j] = 0u;
-        rd->job_count[j] = 0u;
-        rd->job_k[j] = 1u;
-        rd->job_hist_base[j] = 0u;
-    }
-    uint32_t base = 0;
-    uint64_t hbase = 0, cells = 0;
-    for (uint32_t o = 0; o < nj; ++o) {
-        const uint32_t j = ord[o];
-        const JobPmcDev& pm = a.pmc[j];
-        const uint32_t kj = kjs[j];
-        uint64_t want = pm.done ? 0u : (uint64_t)pm.pending_count * kj;
-        uint64_t room = rd->capacity - base;
-        const uint64_t rb = (uint64_t)a.jobs[j].R * a.jobs[j].B;
-        if (rb) {
-            /* each job's histograms start at a multiple of R x B words, so
-             * one tensor map (B x R x histograms over the whole area) reaches
-             * every histogram of the job */
-            hbase = (hbase + rb - 1u) / rb * rb;
-            const uint64_t hroom = hbase < rd->hist_cap ? (rd->hist_cap - hbase) / rb : 0u;
-            if (hroom < room) room = hroom;
+    s_key[j] = kv;
+    s_ord[j] = (uint8_t)j;
+    __syncthreads();
+    if (j == 0u) {
+        double planned = 0.0;
+        bool spec = false;
+        for (uint32_t i = 0; i < nj; ++i) {
+            if (s_pend[i]) planned += s_planned[i];
+            spec |= s_spec[i] != 0u;
         }
-        uint64_t cnt = want < room ? want : room;
-        cnt -= cnt % kj; /* whole slots only */
-        rd->job_base[j] = base;
-        rd->job_k[j] = kj;
-        rd->job_count[j] = (uint32_t)cnt;
-        rd->job_hist_base[j] = hbase;
-        base += (uint32_t)cnt;
-        hbase += cnt * rb;
-        cells += cnt * rb;
+        /* the factor of a round to be topped up, else 0 */
+        s_fill = rd->fill && planned < (double)rd->fill && spec
+                     ? (planned > 0.0 ? (double)rd->fill / planned : (double)k)
+                     : 0.0;
     }
-    rd->n_props = base;
-    rd->n_items = 0u;
-    rd->queue_head = 0u;
-    rd->round_steps = 0ull;
-    rd->round_cells = cells;
+    uint32_t rank = 0u; /* of this job's key, equal keys in admission order */
+    for (uint32_t i = 0; i < nj; ++i) rank += s_key[i] < kv || (s_key[i] == kv && i < j) ? 1u : 0u;
+    if (have) s_ord[rank] = (uint8_t)j;
+    __syncthreads();
+    if (s_fill > 0.0 && gen > 0u && live)
+        kj = (uint32_t)min((double)k, fmax((double)kj, ceil((double)kj * s_fill)));
+    s_k[j] = have ? kj : 1u;
+    __syncthreads();
+    if (j == 0u) {
+        uint32_t base = 0;
+        uint64_t hbase = 0, cells = 0;
+        for (uint32_t o = 0; o < nj; ++o) {
+            const uint32_t i = s_ord[o];
+            const uint32_t ki = s_k[i];
+            uint64_t want = (uint64_t)s_pend[i] * ki;
+            uint64_t room = rd->capacity - base;
+            const uint64_t rb = s_rb[i];
+            if (rb) {
+                /* each job's histograms start at a multiple of R x B words, so
+                 * one tensor map (B x R x histograms over the whole area) reaches
+                 * every histogram of the job */
+                hbase = (hbase + rb - 1u) / rb * rb;
+                const uint64_t hroom = hbase < rd->hist_cap ? (rd->hist_cap - hbase) / rb : 0u;
+                if (hroom < room) room = hroom;
+            }
+            uint32_t cnt = (uint32_t)(want < room ? want : room);
+            cnt -= cnt % ki; /* whole slots only */
+            s_base[i] = base;
+            s_cnt[i] = cnt;
+            s_hbase[i] = hbase;
+            base += cnt;
+            hbase += cnt * rb;
+            cells += cnt * rb;
+        }
+        rd->n_props = base;
+        rd->n_items = 0u;
+        rd->queue_head = 0u;
+        rd->round_steps = 0ull;
+        rd->round_cells = cells;
+    }
+    __syncthreads();
+    if (j < rd->n_jobs) {
+        rd->job_base[j] = have ? s_base[j] : 0u;
+        rd->job_k[j] = s_k[j];
+        rd->job_count[j] = have ? s_cnt[j] : 0u;
+        rd->job_hist_base[j] = have ? s_hbase[j] : 0u;
+    }
 }
 
 /* ----------------------------------------------------------------------- */
@@ -213,16 +233,31 @@ __device__ __forceinline__ uint32_t warp_pick_(const double* wcum, uint32_t N, d
  * constants are computed once and the lanes draw the per-video counts in
  * parallel (each count has its own Philox counter) and scan them into the
  * video prefix.  Every value is the one pcs_build_theta / pcs_build_args /
- * pcs_draw_counts compute (same functions, same operation order). */
-constexpr uint32_t kProposeWarps = 8;
+ * pcs_draw_counts compute (same functions, same operation order).
+ *
+ * Bound by FP64 (a warp instruction occupies an SM's FP64 unit for about 16
+ * cycles), so a round's warps are spread over all SMs: warp w of CTA b takes
+ * proposal w x CTAs + b.  Eight consecutive proposals per CTA left the 213
+ * proposals of configuration 0's average round on 27 SMs.  The parameters
+ * and the descriptor are put together in shared memory and written by the
+ * whole warp, not in each lane's local memory. */
+constexpr uint32_t kProposeWarps = 4;
+
+struct ProposeWarp {
+    double th[PCS_MAX_P], nrm[PCS_MAX_P];
+    CompArgs ca[PCS_MAX_C];
+    PropDev pd;
+};
 
 __global__ void __launch_bounds__(32 * kProposeWarps) k_propose(PmcArgs a)
 {
+    __shared__ ProposeWarp s_warp[kProposeWarps];
     RoundDev* rd = a.round;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t q = blockIdx.x * kProposeWarps + (threadIdx.x >> 5);
+    const uint32_t q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     if (q >= rd->n_props) return; /* whole warp */
-    const uint32_t j = job_of_(rd, q);
+    ProposeWarp& w = s_warp[threadIdx.x >> 5];
+    const uint32_t j = job_of_(rd, q, lane);
     JobPmcDev& pm = a.pmc[j];
     const JobDev& jd = a.jobs[j];
     const uint32_t k = rd->job_k[j];
@@ -235,53 +270,37 @@ __global__ void __launch_bounds__(32 * kProposeWarps) k_propose(PmcArgs a)
     const uint32_t P = pm.P;
     const uint32_t gt = pcs_ctr_gen_trial(gen, trial);
 
-    /* parameters: lane p holds parameter p */
-    double th_l = 0.0;
+    /* parameters: lane p computes parameter p */
     if (gen == 0u) {
-        if (lane < P) th_l = pm.theta[(uint64_t)slot * P + lane];
+        if (lane < P) w.th[lane] = pm.theta[(uint64_t)slot * P + lane];
     } else {
         const pcs_u4 r = pcs_draw(0u, pcs_ctr_tag(PCS_STREAM_PICK, 0u), slot, gt, k0, k1);
         const uint32_t parent = warp_pick_(pm.wcum, pm.N, pcs_u01_53(r.x, r.y), lane);
         const double* tp = pm.theta + (uint64_t)parent * P;
-        double n0 = 0.0, n1 = 0.0;
         if (2u * lane < P) {
             const pcs_u4 rr = pcs_draw(lane, pcs_ctr_tag(PCS_STREAM_PERTURB, 0u), slot, gt, k0, k1);
-            pcs_normal2(rr, n0, n1);
+            pcs_normal2(rr, w.nrm[2u * lane], w.nrm[2u * lane + 1u]);
         }
-        double nrm[PCS_MAX_P];
-        for (uint32_t i = 0; i < P; ++i) { /* P is the same on every lane */
-            const double a0 = __shfl_sync(0xFFFFFFFFu, n0, i >> 1);
-            const double a1 = __shfl_sync(0xFFFFFFFFu, n1, i >> 1);
-            nrm[i] = (i & 1u) ? a1 : a0;
-        }
-        if (lane < P) th_l = pcs_perturb_one(pm, tp, pm.factor, nrm, lane);
+        __syncwarp();
+        if (lane < P) w.th[lane] = pcs_perturb_one(pm, tp, pm.factor, w.nrm, lane);
+        __syncwarp();
+        if (lane == 0u) pcs_sort_components(pm, w.th);
     }
-    double th[PCS_MAX_P];
-    for (uint32_t i = 0; i < P; ++i) th[i] = __shfl_sync(0xFFFFFFFFu, th_l, i);
-    if (gen != 0u) pcs_sort_components(pm, th);
+    __syncwarp();
 
     /* per-component arguments: lane c computes component c */
-    CompArgs ca_l;
-    ca_l.powc = 0.0;
-    ca_l.sd_scale = ca_l.sd_shape = 0.0f;
-    if (lane < pm.C) ca_l = pcs_comp_args(pm, th, lane);
-    CompArgs ca[PCS_MAX_C];
-    for (uint32_t i = 0; i < pm.C; ++i) {
-        ca[i].powc = __shfl_sync(0xFFFFFFFFu, ca_l.powc, i);
-        ca[i].sd_scale = __shfl_sync(0xFFFFFFFFu, ca_l.sd_scale, i);
-        ca[i].sd_shape = __shfl_sync(0xFFFFFFFFu, ca_l.sd_shape, i);
-    }
-    PropDev pd;
-    pd.job = j;
-    pd.slot = slot;
-    pd.trial = trial;
-    pd.gen = gen;
-    pd.hist_z = 0u;
-    const double lambda = pcs_assemble_args(pm, th, ca, gen, pd);
+    if (lane < pm.C) w.ca[lane] = pcs_comp_args(pm, w.th, lane);
+    __syncwarp();
+    double lambda = 0.0;
     if (lane == 0u) {
-        double* out = a.theta_prop + (uint64_t)q * PCS_MAX_P;
-        for (uint32_t p = 0; p < P; ++p) out[p] = th[p];
+        w.pd.job = j;
+        w.pd.slot = slot;
+        w.pd.trial = trial;
+        w.pd.gen = gen;
+        lambda = pcs_assemble_args(pm, w.th, w.ca, gen, w.pd);
     }
+    lambda = __shfl_sync(0xFFFFFFFFu, lambda, 0);
+    if (lane < P) a.theta_prop[(uint64_t)q * PCS_MAX_P + lane] = w.th[lane];
 
     PoissonSetup ps = pcs_poisson_setup(lambda);
     ps.logfact = a.logfact;
@@ -309,19 +328,22 @@ __global__ void __launch_bounds__(32 * kProposeWarps) k_propose(PmcArgs a)
         run += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
     for (int d = 16; d >= 1; d >>= 1) steps += __shfl_xor_sync(0xFFFFFFFFu, steps, d);
-    if (lane != 0u) return;
-    const uint64_t total = run;
-    if (total > 0xFFFFFFFFull) atomicOr(a.err, PCS_ERRBIT_COUNTS);
-    pd.total_particles = (uint32_t)min(total, (uint64_t)0xFFFFFFFFu);
-    pd.counts_off = coff;
-    pd.hist_off = rd->job_hist_base[j] + (uint64_t)local * ((uint64_t)jd.R * jd.B);
-    /* the job's histograms start at a multiple of R x B words (k_round_plan) */
-    pd.hist_z = (uint32_t)(pd.hist_off / max(1ull, (unsigned long long)jd.R * jd.B));
-    pd.item_count = (pd.total_particles + rd->chunk - 1u) / rd->chunk;
-    pd.item_begin = 0u;
-    a.props[q] = pd;
-    atomicAdd((unsigned long long*)&pm.particle_steps, (unsigned long long)steps);
-    atomicAdd(&a.round->round_steps, (unsigned long long)steps);
+    if (lane == 0u) {
+        const uint64_t total = run, rb = (uint64_t)jd.R * jd.B;
+        if (total > 0xFFFFFFFFull) atomicOr(a.err, PCS_ERRBIT_COUNTS);
+        w.pd.total_particles = (uint32_t)min(total, (uint64_t)0xFFFFFFFFu);
+        w.pd.counts_off = coff;
+        w.pd.hist_off = rd->job_hist_base[j] + (uint64_t)local * rb;
+        /* the job's histograms start at a multiple of R x B words (k_round_plan) */
+        w.pd.hist_z = (uint32_t)(w.pd.hist_off / max(1ull, (unsigned long long)rb));
+        w.pd.item_count = (w.pd.total_particles + rd->chunk - 1u) / rd->chunk;
+        w.pd.item_begin = 0u;
+        atomicAdd((unsigned long long*)&pm.particle_steps, (unsigned long long)steps);
+        atomicAdd(&a.round->round_steps, (unsigned long long)steps);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < sizeof(PropDev) / 4u; i += 32u)
+        reinterpret_cast<uint32_t*>(a.props + q)[i] = reinterpret_cast<const uint32_t*>(&w.pd)[i];
 }
 
 /* ----------------------------------------------------------------------- */
@@ -372,6 +394,7 @@ __global__ void __launch_bounds__(1024) k_accept(PmcArgs a)
 {
     __shared__ uint32_t s_keep, s_exhausted;
     __shared__ unsigned long long s_trials, s_acc;
+    __shared__ double s_sure, s_never;
     const uint32_t j = blockIdx.x;
     RoundDev* rd = a.round;
     if (j >= rd->n_jobs) return;
@@ -389,45 +412,74 @@ __global__ void __launch_bounds__(1024) k_accept(PmcArgs a)
         s_trials = 0ull;
         s_acc = 0ull;
         pm.gen_ended = 0u;
+        const double edge = exp10(pm.gamma); /* one warp's FP64, not the block's */
+        s_sure = edge * (1.0 - 1e-11);
+        s_never = edge * (1.0 + 1e-11);
     }
     __syncthreads();
-    /* decide every pending slot; kept slots go to scratch (as u32 bits) */
+    /* decide every pending slot; kept slots go to scratch (as u32 bits).  A
+     * group of lanes (as many as the trials per slot, at most a warp) looks at
+     * a slot's trials side by side: at a generation's end few slots have many
+     * trials each.  log10(d) <= gamma is decided by d against 10^gamma but for
+     * a margin far above both functions' errors, in which log10 is taken: on
+     * this GPU's FP64 rate it would otherwise set the pace for every trial. */
     uint32_t* keep_list = reinterpret_cast<uint32_t*>(pm.scratch);
-    for (uint32_t i = threadIdx.x; i < npend; i += blockDim.x) {
-        const uint32_t slot = pm.pending[i];
-        bool acc_ok = false;
-        if (i < nprop_slots) {
-            uint32_t first = k;
-            double dsel = 0.0;
-            for (uint32_t r = 0; r < k; ++r) {
+    uint32_t g = 1u;
+    while (g < 32u && g < k) g <<= 1;
+    const uint32_t lane = threadIdx.x & 31u, gl = lane & (g - 1u), g0 = lane & ~(g - 1u);
+    const unsigned gmask = g == 32u ? 0xFFFFFFFFu : (1u << g) - 1u;
+    const bool prior = pm.generation == 0u, f64 = a.use_f64_distance && a.dist_f64;
+    const double gamma = pm.gamma, sure = s_sure, never = s_never;
+    unsigned long long trials = 0ull, accepted = 0ull;
+    for (uint32_t i0 = 0; i0 < npend; i0 += blockDim.x / g) {
+        const uint32_t i = i0 + threadIdx.x / g;
+        const bool in = i < npend && i < nprop_slots;
+        const uint32_t slot = i < npend ? pm.pending[i] : 0u;
+        uint32_t first = k;
+        for (uint32_t r0 = 0; r0 < k; r0 += g) {
+            const uint32_t r = r0 + gl;
+            bool ok = false;
+            if (in && first == k && r < k) {
                 const uint32_t q = base + i * k + r;
-                const double df = a.use_f64_distance && a.dist_f64 ? a.dist_f64[q] : (double)a.dist_f32[q];
-                const double d = log10(df);
-                if (pm.generation == 0u || d <= pm.gamma) {
-                    first = r;
-                    dsel = d;
-                    break;
-                }
+                const double df = f64 ? a.dist_f64[q] : (double)a.dist_f32[q];
+                ok = prior || df <= sure || (!(df >= never) && log10(df) <= gamma);
             }
-            if (first < k) {
+            const unsigned m = (__ballot_sync(0xFFFFFFFFu, ok) >> g0) & gmask;
+            if (m) first = r0 + (uint32_t)__ffs(m) - 1u;
+            if (!__any_sync(0xFFFFFFFFu, in && first == k)) break;
+        }
+        if (in && first < k) {
+            const uint32_t q = base + i * k + first;
+            for (uint32_t p = gl; p < P; p += g)
+                pm.theta_new[(uint64_t)slot * P + p] = a.theta_prop[(uint64_t)q * PCS_MAX_P + p];
+        }
+        if (i < npend && gl == 0u) {
+            if (in && first < k) {
                 const uint32_t q = base + i * k + first;
-                for (uint32_t p = 0; p < P; ++p)
-                    pm.theta_new[(uint64_t)slot * P + p] = a.theta_prop[(uint64_t)q * PCS_MAX_P + p];
-                pm.dist_new[slot] = dsel;
+                pm.dist_new[slot] = log10(f64 ? a.dist_f64[q] : (double)a.dist_f32[q]);
                 pm.accepted[slot] = 1u;
-                acc_ok = true;
-                atomicAdd(&s_trials, (unsigned long long)(first + 1u));
-                atomicAdd(&s_acc, 1ull);
+                trials += first + 1u;
+                accepted += 1u;
             } else {
-                pm.next_trial[slot] += k;
-                atomicAdd(&s_trials, (unsigned long long)k);
-                /* the trial ordinal has 20 bits in the random-stream counter:
-                 * a slot that exhausts them ends the generation like the
-                 * trial cap does (converged) */
-                if (pm.next_trial[slot] + rd->max_spec >= (1u << 20)) s_exhausted = 1u;
+                if (in) {
+                    pm.next_trial[slot] += k;
+                    trials += k;
+                    /* the trial ordinal has 20 bits in the random-stream counter:
+                     * a slot that exhausts them ends the generation like the
+                     * trial cap does (converged) */
+                    if (pm.next_trial[slot] + rd->max_spec >= (1u << 20)) s_exhausted = 1u;
+                }
+                keep_list[atomicAdd(&s_keep, 1u)] = slot;
             }
         }
-        if (!acc_ok) keep_list[atomicAdd(&s_keep, 1u)] = slot;
+    }
+    for (int d = 16; d >= 1; d >>= 1) {
+        trials += __shfl_xor_sync(0xFFFFFFFFu, trials, d);
+        accepted += __shfl_xor_sync(0xFFFFFFFFu, accepted, d);
+    }
+    if (lane == 0u && trials) {
+        atomicAdd(&s_trials, trials);
+        atomicAdd(&s_acc, accepted);
     }
     __syncthreads();
     const uint32_t nk = s_keep;
@@ -974,7 +1026,7 @@ static void launch_sat_sums_(uint32_t rows, uint32_t bins, uint32_t* sat, uint32
 /* ----------------------------------------------------------------------- */
 cudaError_t launch_round_plan(const PmcArgs& a, cudaStream_t st)
 {
-    k_round_plan<<<1, 32, 0, st>>>(a);
+    k_round_plan<<<1, kMaxRoundJobs, 0, st>>>(a);
     return cudaGetLastError();
 }
 
