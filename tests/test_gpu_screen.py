@@ -44,6 +44,8 @@ CASES = {
     "long-steps": (0, 2, 55, 2, 12.0, 2.0, (100.0, 80.0, 10.0), (50.0, 40.0)),
     "no-steps": (0, 1, 56, 2, 0.0, 2.0, (100.0, 80.0, 10.0), (50.0, 40.0)),
     "edge": (0, 1, 48, 2, 2.5, 2.0, (100.0, 80.0, 10.0), (98.0, 79.0)),
+    "box-edge": (0, 1, 90, 2, 0.8, 4.0, (20.0, 19.0, 10.0), (1.0, 0.5)),  # groups with and without x, y wraps
+    "tiny-steps": (0, 1, 64, 2, 1e-6, 4.0, (100.0, 80.0, 10.0), (99.0, 79.0)),  # steps near one rounding of x
     "short": (0, 2, 47, 2, 0.4, 2.0, (100.0, 80.0, 10.0), (50.0, 40.0)),
     "one-step": (2, 1, 2, 1, 0.4, 2.0, (100.0, 80.0, 10.0), (50.0, 40.0)),
     "one-frame": (2, 1, 1, 1, 0.4, 2.0, (100.0, 80.0, 10.0), (50.0, 40.0)),
