@@ -760,6 +760,8 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         d.ssd = d_ssd;
         d.err = c.err.as<uint32_t>();
         d.max_rows = rows;
+        d.max_bins = bins;
+        d.max_count = d.min_count = count;
         d.tmaps = setup.map;
         const uint32_t cl = (d_cum || d_d64 || d_ssd) ? 0u : distance_cluster_size(rows, bins);
         PCS_CUDA(launch_distance(d, std::min<uint32_t>(count, (uint32_t)(distance_ctas_per_sm(rows) * c.sm_count)), st, cl));

@@ -670,6 +670,9 @@ void Ctx::enqueue_round()
     d.ssd = nullptr;
     d.err = a.err;
     d.max_rows = rb.max_rows;
+    d.max_bins = rb_max_b_;
+    d.max_count = rb.capacity;
+    d.min_count = 1u; /* the round's number is the device's */
     d.tmaps = rb.tmaps.as<TmapDev>();
     const uint32_t cl = d.dist_f64 ? 0u : distance_cluster_size(rb.max_rows, rb_max_b_);
     PCS_CUDA(cudaEventRecordWithFlags(ev_dist0, stream, cudaEventRecordExternal));

@@ -75,6 +75,10 @@ __device__ __forceinline__ double reduce0_(double v)
     return v;
 }
 
+/* what the row kernel leaves as the distance of a histogram that the kernel
+ * launched after it shall take: a quiet NaN that no sum of squares is */
+const uint32_t kRedo = 0x7FC5EED0u;
+
 __device__ __forceinline__ void add128_(uint64_t& hi, uint64_t& lo, uint64_t bhi, uint64_t blo)
 {
     uint64_t n = lo + blo;
@@ -85,7 +89,7 @@ __device__ __forceinline__ void add128_(uint64_t& hi, uint64_t& lo, uint64_t bhi
 } // namespace
 
 template <bool F64>
-__global__ void __launch_bounds__(1024, 1) k_distance(DistArgs a)
+__global__ void __launch_bounds__(1024, 1) k_distance(DistArgs a, uint32_t redo)
 {
     extern __shared__ uint32_t s_mem[];
     uint32_t* carry = s_mem;            /* [max_rows] */
@@ -99,6 +103,7 @@ __global__ void __launch_bounds__(1024, 1) k_distance(DistArgs a)
     const uint32_t M = *a.n_props;
 
     for (uint32_t p = blockIdx.x; p < M; p += gridDim.x) {
+        if (redo && __float_as_uint(a.dist_f32[p]) != kRedo) continue; /* the row kernel's */
         const uint32_t job = a.props[p].job;
         const uint64_t hoff = a.props[p].hist_off;
         const uint32_t R = a.jobs[job].R, B = a.jobs[job].B;
@@ -770,8 +775,405 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
     strip_cluster_(a, db, cl, M, tiles, tile_words, zero, carry, P2, part2, s_tot, s_col, s_K, s_mbar, &s_abort);
 }
 
+/* Row kernel: a CTA takes one histogram at a time, a warp 128 of its columns
+ * (lane l columns 4l..4l+3), and the rows stream past.  Rows come in blocks of
+ * 8 through a ring of three blocks per warp in shared memory, filled two
+ * blocks ahead by each lane's own cp.async (16 bytes where the rows are
+ * 16-byte aligned, else cell by cell), so no lane waits for another's copy.
+ * A lane keeps its columns' running sums; one warp scan per row (eight rows'
+ * step by step together) turns them into the row's 2-D prefix sums.  With
+ * more than 128 columns the warps exchange each row's last prefix sum once
+ * per block (one CTA barrier).  The reference's per-lane sums, one for every
+ * (row mod 32, column) of a strip of 32 columns, live in shared memory as
+ * [32][128] floats per warp, one 16-byte read and write per row and lane; at
+ * the end the strips' are added in order and the reference's trees follow.
+ *
+ * 62 warp instructions per 128 cells, where the strip kernel, passing over
+ * its tile three times, has about 150; of 8 warps per SM (shared memory: 28 KB
+ * each, 64 KB of loads in flight) the two per scheduler issue in 31 % of the
+ * cycles, between waits for shared memory, scans and the observed cells.
+ * 1024 of 301 x 128: 88 us (strips) -> 51 us.  One lane per column instead
+ * (7 KB per warp, 32 warps per SM) has 48 instructions per 32 cells: 86 us.
+ * A walk down few rows at a time costs a fixed 90 ns per row, so few
+ * histograms of few columns stay with the strips (use_rows_).
+ *
+ * Where every value of a block of rows is below 2^22 the differences are
+ * exact integers (see k_distance_strip); other blocks take the reference's
+ * conversions.  F64 needs exact differences and an exact sum of squares
+ * below 2^53, where the reference's chain of double additions is exact in any
+ * order.  Whether that holds is known when the last row has passed: a
+ * histogram for which it does not is left as it was (with F64 the zeroing
+ * waits for the verdict) with kRedo as its distance, and the strip kernel
+ * launched after it takes it. */
+const uint32_t kRowsBlock = 8u, kRowsRing = 3u, kRowsWarps = 8u;
+const uint32_t kRowsAccBytes = 32u * 128u * 4u, kRowsRingBytes = kRowsRing * kRowsBlock * 512u;
+const uint32_t kRowsWarpBytes = kRowsAccBytes + kRowsRingBytes;
+
+/* 16 bytes where `valid`, else zeros, without reading src */
+__device__ __forceinline__ void cp_async16z_(void* dst, const void* src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32_(dst)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
+/* a warp's inclusive scans of eight values, step by step together */
+__device__ __forceinline__ void warp_scan8_(uint32_t* t)
+{
+#define PCS_SCAN_STEP(d)                                                                                       \
+    _Pragma("unroll") for (uint32_t i = 0; i < kRowsBlock; ++i)                                                 \
+        asm volatile("{\n\t.reg .u32 u;\n\t.reg .pred p;\n\tshfl.sync.up.b32 u|p, %0, " #d                     \
+                     ", 0x0, 0xffffffff;\n\t@p add.u32 %0, %0, u;\n\t}\n"                                       \
+                     : "+r"(t[i]));
+    PCS_SCAN_STEP(1)
+    PCS_SCAN_STEP(2)
+    PCS_SCAN_STEP(4)
+    PCS_SCAN_STEP(8)
+    PCS_SCAN_STEP(16)
+#undef PCS_SCAN_STEP
+}
+
+/* One warp's walk down its 128 columns of a histogram. */
+template <bool F64, bool SSD, bool VEC>
+struct RowsWalk {
+    const uint32_t* hist; /* this lane's first column (or column 0), row 0 */
+    const uint32_t* next; /* the same, the next row to fill (16-byte rows) */
+    const uint32_t* ref;  /* of the next row of the observed histogram */
+    uint32_t* gone;       /* the next row to zero */
+    uint32_t* cum;        /* or null */
+    uint4* ring;          /* [3][8] steps of 32 */
+    float4* acc;          /* [32] steps of 32 */
+    uint32_t (*P)[kRowsWarps][kRowsBlock];
+    uint32_t R, B, nc, w, l, NP;
+    uint4 col, o[kRowsBlock];
+    bool high;            /* a value of 2^22 or more has passed */
+    uint64_t hi, lo;      /* exact sum of squares */
+
+    /* this lane's copies of block b (one group); rows and columns past the last arrive as zeros */
+    __device__ __forceinline__ void fill(uint32_t b)
+    {
+        uint4* to = ring + (b % kRowsRing) * (kRowsBlock * 32u);
+        const bool full = (b + 1u) * kRowsBlock <= R;
+        if (VEC && full) {
+            if (nc) {
+#pragma unroll
+                for (uint32_t i = 0; i < kRowsBlock; ++i, next += B) cp_async16z_(to + i * 32u, next, true);
+            }
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i) {
+                const uint32_t r = b * kRowsBlock + i;
+                const uint32_t* from = hist + (uint64_t)min(r, R - 1u) * B;
+                if (VEC) {
+                    cp_async16z_(to + i * 32u, from, r < R && nc != 0u);
+                } else {
+#pragma unroll
+                    for (uint32_t x = 0; x < 4u; ++x)
+                        cp_async4_(reinterpret_cast<uint32_t*>(to + i * 32u) + x, from + (x < nc ? x : 0u), r < R && x < nc);
+                }
+            }
+        }
+        cp_async_commit_();
+    }
+
+    /* the observed histogram's cells at q in this lane's columns */
+    __device__ __forceinline__ uint4 observed(const uint32_t* q) const
+    {
+        if (VEC) return __ldg(reinterpret_cast<const uint4*>(q));
+        return make_uint4(__ldg(q), __ldg(q + (1u < nc ? 1u : 0u)), __ldg(q + (2u < nc ? 2u : 0u)), __ldg(q + (3u < nc ? 3u : 0u)));
+    }
+
+    /* those of block b; rows past the last take the last row's */
+    __device__ __forceinline__ void observe(uint32_t b)
+    {
+        if ((b + 1u) * kRowsBlock <= R) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i, ref += B) o[i] = observed(ref);
+        } else if (b * kRowsBlock < R) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i) {
+                o[i] = observed(ref);
+                if (b * kRowsBlock + i + 1u < R) ref += B;
+            }
+        }
+    }
+
+    /* one row's cells zeroed, as K_distance does */
+    __device__ __forceinline__ void zero_row()
+    {
+        if (VEC) {
+            if (nc) __stcs(reinterpret_cast<uint4*>(gone), make_uint4(0u, 0u, 0u, 0u));
+        } else {
+            if (nc > 0u) __stcs(gone, 0u);
+            if (nc > 1u) __stcs(gone + 1, 0u);
+            if (nc > 2u) __stcs(gone + 2, 0u);
+            if (nc > 3u) __stcs(gone + 3, 0u);
+        }
+        gone += B;
+    }
+
+    /* the rows' terms added to the sums (columns past the last too: they are not read) */
+    template <bool FULL, typename Diff>
+    __device__ __forceinline__ void terms(uint32_t b, const uint4* s, float4* v, Diff diff) const
+    {
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) {
+            if (!FULL && b * kRowsBlock + i >= R) break;
+            const float dx = diff(s[i].x, o[i].x), dy = diff(s[i].y, o[i].y);
+            const float dz = diff(s[i].z, o[i].z), dw = diff(s[i].w, o[i].w);
+            v[i].x = __fadd_rn(v[i].x, __fmul_rn(dx, dx));
+            v[i].y = __fadd_rn(v[i].y, __fmul_rn(dy, dy));
+            v[i].z = __fadd_rn(v[i].z, __fmul_rn(dz, dz));
+            v[i].w = __fadd_rn(v[i].w, __fmul_rn(dw, dw));
+        }
+    }
+
+    __device__ __forceinline__ void wide_square_(uint32_t s, uint32_t o)
+    {
+        const uint64_t d = s >= o ? s - o : o - s;
+        add128_(hi, lo, 0u, d * d);
+    }
+
+    template <bool FULL>
+    __device__ __forceinline__ void block(uint32_t b)
+    {
+        fill(b + 2u);
+        cp_async_wait_<2>();
+        const uint4* in = ring + (b % kRowsRing) * (kRowsBlock * 32u);
+        uint4 s[kRowsBlock];
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) {
+            const uint4 v = in[i * 32u];
+            col.x += v.x;
+            col.y += v.y;
+            col.z += v.z;
+            col.w += v.w;
+            s[i].x = col.x;
+            s[i].y = col.x + col.y;
+            s[i].z = s[i].y + col.z;
+            s[i].w = s[i].z + col.w;
+            if (!F64 && (FULL || b * kRowsBlock + i < R)) zero_row();
+        }
+        uint32_t t[kRowsBlock];
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) t[i] = s[i].w;
+        warp_scan8_(t);
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) {
+            const uint32_t before = t[i] - s[i].w;
+            s[i].x += before;
+            s[i].y += before;
+            s[i].z += before;
+            s[i].w = t[i];
+        }
+        if (NP > 1u) {
+            uint32_t (*Pb)[kRowsBlock] = P[b & 1u];
+            if (l == 31u) {
+#pragma unroll
+                for (uint32_t i = 0; i < kRowsBlock; ++i) Pb[w][i] = s[i].w;
+            }
+            __syncthreads();
+            uint32_t left = 0u;
+            for (uint32_t j = 0; j < w; ++j) left += Pb[j][l & (kRowsBlock - 1u)];
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i) {
+                const uint32_t add = __shfl_sync(0xFFFFFFFFu, left, i);
+                s[i].x += add;
+                s[i].y += add;
+                s[i].z += add;
+                s[i].w += add;
+            }
+        }
+        float4* at = acc + (b & 3u) * (kRowsBlock * 32u);
+        float4 v[kRowsBlock];
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) v[i] = at[i * 32u];
+        /* counts grow down the rows: the block's largest are its last row's */
+        const uint4 sl = s[kRowsBlock - 1u], ol = o[kRowsBlock - 1u];
+        const bool exact = !__any_sync(0xFFFFFFFFu, (sl.w | ol.x | ol.y | ol.z | ol.w) >= kExactBelow);
+        if (!exact) high = true;
+        if (F64 || exact) {
+            terms<FULL>(b, s, v, [](uint32_t t, uint32_t q) { return exact_diff_(t, q); });
+        } else {
+            terms<FULL>(b, s, v, [](uint32_t t, uint32_t q) { return __fsub_rn(__uint2float_rn(t), __uint2float_rn(q)); });
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) at[i * 32u] = v[i];
+        if (F64 || SSD) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i) {
+                if (!FULL && b * kRowsBlock + i >= R) break;
+                if (F64 || exact) {
+                    if (VEC || nc > 0u) lo += square_(s[i].x, o[i].x);
+                    if (VEC || nc > 1u) lo += square_(s[i].y, o[i].y);
+                    if (VEC || nc > 2u) lo += square_(s[i].z, o[i].z);
+                    if (VEC || nc > 3u) lo += square_(s[i].w, o[i].w);
+                } else {
+                    if (VEC || nc > 0u) wide_square_(s[i].x, o[i].x);
+                    if (VEC || nc > 1u) wide_square_(s[i].y, o[i].y);
+                    if (VEC || nc > 2u) wide_square_(s[i].z, o[i].z);
+                    if (VEC || nc > 3u) wide_square_(s[i].w, o[i].w);
+                }
+            }
+        }
+        observe(b + 1u);
+        if (cum) {
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsBlock; ++i) {
+                const uint32_t r = b * kRowsBlock + i;
+                if (r < R && nc) {
+                    uint32_t* q = cum + (uint64_t)r * B;
+                    if (VEC) {
+                        __stcs(reinterpret_cast<uint4*>(q), s[i]);
+                    } else {
+                        q[0] = s[i].x;
+                        if (nc > 1u) q[1] = s[i].y;
+                        if (nc > 2u) q[2] = s[i].z;
+                        if (nc > 3u) q[3] = s[i].w;
+                    }
+                }
+            }
+        }
+    }
+
+    __device__ __forceinline__ void walk()
+    {
+        if (VEC && !nc) /* filled by no copy */
+#pragma unroll
+            for (uint32_t i = 0; i < kRowsRing * kRowsBlock; ++i) ring[i * 32u] = make_uint4(0u, 0u, 0u, 0u);
+        next = hist;
+        fill(0u);
+        fill(1u);
+        observe(0u);
+#pragma unroll
+        for (uint32_t k = 0; k < 32u; ++k) acc[k * 32u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        col = make_uint4(0u, 0u, 0u, 0u);
+        high = false;
+        hi = lo = 0u;
+        uint32_t b = 0u;
+        for (; (b + 1u) * kRowsBlock <= R; ++b) block<true>(b);
+        if (b * kRowsBlock < R) block<false>(b);
+        cp_async_wait_<0>();
+    }
+};
+
+/* histogram p by the CTA's warps; false: left as it was */
+template <bool F64, bool SSD, bool VEC>
+__device__ __forceinline__ bool rows_hist_(const DistArgs& a, uint32_t p, const JobDev& jd, uint32_t* hist,
+                                           unsigned char* s_rows, uint32_t (*s_P)[kRowsWarps][kRowsBlock],
+                                           uint64_t* s_hi, uint64_t* s_lo)
+{
+    RowsWalk<F64, SSD, VEC> k;
+    k.w = threadIdx.x >> 5;
+    k.l = threadIdx.x & 31u;
+    k.NP = blockDim.x >> 5;
+    k.R = jd.R;
+    k.B = jd.B;
+    const uint32_t c = 128u * k.w + 4u * k.l, w = k.w, l = k.l, NP = k.NP;
+    k.nc = c < k.B ? min(k.B - c, 4u) : 0u;
+    const uint32_t c1 = k.nc ? c : 0u;
+    k.hist = k.gone = hist + c1;
+    k.ref = jd.ref_sat + c1;
+    k.cum = a.cum_out ? a.cum_out + a.props[p].hist_off + c1 : nullptr;
+    k.acc = reinterpret_cast<float4*>(s_rows + w * kRowsWarpBytes) + l;
+    k.ring = reinterpret_cast<uint4*>(s_rows + w * kRowsWarpBytes + kRowsAccBytes) + l;
+    k.P = s_P;
+    k.walk();
+
+    uint64_t hi = k.nc ? k.hi : 0u, lo = k.nc ? k.lo : 0u;
+    if (F64 || SSD) {
+        for (uint32_t d = 16; d >= 1; d >>= 1) {
+            const uint64_t ohi = __shfl_down_sync(0xFFFFFFFFu, hi, d);
+            const uint64_t olo = __shfl_down_sync(0xFFFFFFFFu, lo, d);
+            if (l + d < 32u) add128_(hi, lo, ohi, olo);
+        }
+        if (l == 0u) {
+            s_hi[w] = hi;
+            s_lo[w] = lo;
+        }
+    }
+    const bool over = __syncthreads_or(k.high) != 0;
+    if (F64 || SSD) {
+        hi = lo = 0u;
+        for (uint32_t j = 0; j < NP; ++j) add128_(hi, lo, s_hi[j], s_lo[j]);
+    }
+    if (F64) {
+        if (over || hi != 0u || (lo >> 53) != 0u) return false;
+#pragma unroll 8
+        for (uint32_t r = 0; r < k.R; ++r) k.zero_row();
+    }
+    /* (logical warp l, lane i): its strips' sums in order; then the trees */
+    float* sums = reinterpret_cast<float*>(s_rows + kRowsAccBytes); /* [32][33], over warp 0's ring */
+    const uint32_t ns = (k.B + 31u) / 32u;
+    for (uint32_t i = w; i < 32u; i += NP) {
+        float v = 0.0f;
+        for (uint32_t j = 0; j < ns; ++j)
+            if (32u * j + l < k.B)
+                v = __fadd_rn(v, reinterpret_cast<const float*>(s_rows + (j >> 2) * kRowsWarpBytes)[i * 128u + (j & 3u) * 32u + l]);
+        sums[l * 33u + i] = v;
+    }
+    __syncthreads();
+    if (w == 0u) {
+        float v[32];
+#pragma unroll
+        for (uint32_t i = 0; i < 32u; ++i) v[i] = sums[l * 33u + i];
+#pragma unroll
+        for (uint32_t d = 16; d >= 1; d >>= 1)
+#pragma unroll
+            for (uint32_t i = 0; i < d; ++i) v[i] = __fadd_rn(v[i], v[i + d]);
+        const float fin = reduce0_(v[0]);
+        if (l == 0u) {
+            a.dist_f32[p] = fin;
+            if (F64 && a.dist_f64) a.dist_f64[p] = (double)lo;
+            if (SSD && a.ssd) {
+                a.ssd[2 * (uint64_t)p] = hi;
+                a.ssd[2 * (uint64_t)p + 1] = lo;
+            }
+        }
+    }
+    return true;
+}
+
 template <bool F64, bool SSD>
-__global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t db)
+__global__ void __launch_bounds__(32 * kRowsWarps) k_distance_rows(DistArgs a)
+{
+    extern __shared__ __align__(128) unsigned char s_rows[]; /* per warp: float sums [32][128], ring [3][8][128] */
+    __shared__ uint32_t s_P[2][kRowsWarps][kRowsBlock];      /* each warp's last prefix sum of a row */
+    __shared__ uint64_t s_hi[kRowsWarps], s_lo[kRowsWarps];
+    const uint32_t M = *a.n_props;
+    for (uint32_t p = blockIdx.x; p < M; p += gridDim.x) {
+        const JobDev& jd = a.jobs[a.props[p].job];
+        uint32_t* hist = a.hist + a.props[p].hist_off;
+        bool done = false;
+        if (jd.R > a.max_rows || jd.B > 4u * blockDim.x) {
+            if (threadIdx.x == 0u) {
+                atomicOr(a.err, PCS_ERRBIT_ROWS);
+                a.dist_f32[p] = __int_as_float(0x7fc00000);
+            }
+            done = true;
+        } else {
+            const uintptr_t at = reinterpret_cast<uintptr_t>(hist) | reinterpret_cast<uintptr_t>(jd.ref_sat) |
+                                 reinterpret_cast<uintptr_t>(a.cum_out ? a.cum_out + a.props[p].hist_off : nullptr);
+            if (((jd.B * 4u) & 15u) == 0u && (at & 15u) == 0u)
+                done = rows_hist_<F64, SSD, true>(a, p, jd, hist, s_rows, s_P, s_hi, s_lo);
+            else
+                done = rows_hist_<F64, SSD, false>(a, p, jd, hist, s_rows, s_P, s_hi, s_lo);
+        }
+        if (!done && threadIdx.x == 0u) a.dist_f32[p] = __uint_as_float(kRedo);
+        __syncthreads(); /* the sums are read */
+    }
+}
+
+/* the first histogram from p on in this CTA's sequence that is the strip
+ * kernel's: all of them, or (redo) those that the row kernel left */
+__device__ __forceinline__ uint32_t strip_next_(const DistArgs& a, uint32_t p, uint32_t M, uint32_t redo)
+{
+    if (redo)
+        while (p < M && __float_as_uint(a.dist_f32[p]) != kRedo) p += gridDim.x;
+    return p;
+}
+
+template <bool F64, bool SSD>
+__global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t db, uint32_t redo)
 {
     extern __shared__ __align__(16) uint32_t s_mem[];
     const uint32_t tile_words = strip_cap_rows(a.max_rows) * 32u;
@@ -791,7 +1193,7 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
     const uint32_t tid = threadIdx.x;
     const uint32_t w = tid >> 5, l = tid & 31u;
     const uint32_t M = *a.n_props;
-    uint32_t p = blockIdx.x;
+    uint32_t p = strip_next_(a, blockIdx.x, M, redo);
     if (p >= M) return;
     if (tid == 0) {
         mbar_init_(&s_mbar[0], kStripThreads);
@@ -819,7 +1221,7 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
         /* the (proposal, strip) after this one */
         uint32_t pn = p, cn = c0 + 32u;
         if (!ok || cn >= B) {
-            pn = p + gridDim.x;
+            pn = strip_next_(a, p + gridDim.x, M, redo);
             cn = 0u;
         }
         const bool has_next = pn < M;
@@ -1195,8 +1597,57 @@ cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaSt
     return cudaGetLastError();
 }
 
+static const size_t kSmemPerSm = 228u * 1024u; /* of which 1 KB per resident CTA is not the CTA's */
+
+/* Rows or strips.  The row kernel takes one walk down the rows (10 us + 90 ns
+ * per row) for any number of columns and histograms until its warps fill the
+ * SMs; the strip kernels take 2.2 us + 9.5 ns per row for every strip (or
+ * cluster's histogram) that a CTA (cluster slot) has in turn.  The lines
+ * cross at 5 turns for 33 rows, 7 for 201 and 8.5 for 1001.  Measured, strips
+ * -> rows in us: 4 turns (201 x 100 x 213) 21.9 -> 24.5, 8 turns (201 x 100 x
+ * 608) 40.9 -> 27.1 and (201 x 256 x 100) 33.3 -> 26.4, 32 turns (201 x 1000
+ * x 152) 122 -> 52; clusters at 6 turns (1001 x 256 x 76) 83 -> 102, at 8
+ * (x 120) 115 -> 104, at 21 (x 304) 281 -> 131; 16 turns (301 x 128 x 1024)
+ * 89.6 -> 51.1.
+ * With double sums the walk zeroes in a second pass and a launch for the
+ * histograms left over follows: 8 turns (1001 x 256 x 152) 116 -> 138, 16
+ * (x 304) 228 -> 166, 32 (201 x 1000 x 20) 126 -> 63.
+ * Where rows are not 16-byte aligned the lanes copy cell by cell: 8 turns
+ * (201 x 255 x 100) 39.4 -> 43, 10 (51 x 31 x 3000) 44.6 -> 57, 12 (201 x 99
+ * x 912) 75.9 -> 57.8, 32 (201 x 999 x 38) 145 -> 90.
+ * Histograms too tall for a strip in shared memory (above 1664 rows), whose
+ * kernel works through blocks of rows: 2 turns (1800 x 40 x 2) 154 -> 157,
+ * 4 (x 200) 836 -> 146, 16 (1800 x 256 x 200) 5409 -> 195. */
+static bool use_rows_(const DistArgs& a, uint32_t turns)
+{
+    uint32_t from = 8u;
+    if (a.dist_f64) from += 4u;
+    if (a.max_bins & 3u) from += 4u;
+    if (!use_strip(a.max_rows, 0u)) from = 3u;
+    return a.max_bins <= 128u * kRowsWarps && turns >= from;
+}
+
+static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st)
+{
+    void (*k)(DistArgs);
+    if (a.dist_f64) k = a.ssd ? k_distance_rows<true, true> : k_distance_rows<true, false>;
+    else k = a.ssd ? k_distance_rows<false, true> : k_distance_rows<false, false>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRowsWarps * kRowsWarpBytes));
+    if (e != cudaSuccess) return e;
+    const uint32_t warps = (a.max_bins + 127u) / 128u;
+    const size_t smem = (size_t)warps * kRowsWarpBytes;
+    const uint32_t per_sm = std::max<uint32_t>(1u, (uint32_t)(kSmemPerSm / (smem + 2048u)));
+    k<<<std::min(a.max_count, per_sm * sms), 32u * warps, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl)
 {
+    int dev = 0, n_sm = 0;
+    cudaError_t e0 = cudaGetDevice(&dev);
+    if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (e0 != cudaSuccess) return e0;
+    const uint32_t sms = (uint32_t)n_sm, strips = (a.max_bins + 31u) / 32u;
     if (cl > 1u && (a.dist_f64 || a.ssd || a.cum_out || !use_strip(a.max_rows, cl) || cl > kMaxDistCluster)) cl = 0u;
     if (cl > 1u) {
         /* clusters of cl CTAs where the histograms are tall, or where every
@@ -1221,29 +1672,37 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
         e = cluster_fit_(cfg, cl, smem, fit);
         if (e != cudaSuccess) return e;
         if (fit > 0 && (strip_cap_rows(a.max_rows) >= kClusterRowsMin || grid <= (uint32_t)fit)) {
+            if (use_rows_(a, (a.min_count + (uint32_t)fit - 1u) / (uint32_t)fit)) return launch_rows_(a, sms, st);
             cfg.gridDim = dim3(std::min<uint32_t>(grid, (uint32_t)fit) * cl);
             return cudaLaunchKernelEx(&cfg, k_distance_cluster, a, strip_db(a.max_rows, cl) ? 1u : 0u, cl);
         }
         cl = 0u;
     }
     const size_t smem = distance_smem_bytes(a.max_rows, 0u);
+    if (smem > 227u * 1024u) return cudaErrorInvalidValue;
+    const uint32_t slots = sms * (use_strip(a.max_rows, 0u) && 2u * (smem + 4096u) <= kSmemPerSm ? 2u : 1u);
+    const bool rows = use_rows_(a, strips * ((std::max(1u, a.min_count) + slots - 1u) / slots));
+    if (rows) {
+        const cudaError_t e = launch_rows_(a, sms, st);
+        if (e != cudaSuccess || !a.dist_f64) return e;
+    }
     if (use_strip(a.max_rows, 0u)) {
-        void (*k)(DistArgs, uint32_t);
+        void (*k)(DistArgs, uint32_t, uint32_t);
         if (a.dist_f64) k = a.ssd ? k_distance_strip<true, true> : k_distance_strip<true, false>;
         else k = a.ssd ? k_distance_strip<false, true> : k_distance_strip<false, false>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u);
+        k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u, rows ? 1u : 0u);
         return cudaGetLastError();
     }
     if (a.dist_f64) {
         cudaError_t e = cudaFuncSetAttribute(k_distance<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        k_distance<true><<<grid, 1024, smem, st>>>(a);
+        k_distance<true><<<grid, 1024, smem, st>>>(a, rows ? 1u : 0u);
     } else {
         cudaError_t e = cudaFuncSetAttribute(k_distance<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        k_distance<false><<<grid, 1024, smem, st>>>(a);
+        k_distance<false><<<grid, 1024, smem, st>>>(a, 0u);
     }
     return cudaGetLastError();
 }

@@ -146,6 +146,8 @@ extern "C" pcs_status pcs_scan_distance_noalloc(uint32_t* d_hist, const uint32_t
     d.ssd = nullptr;
     d.err = &h->err;
     d.max_rows = rows;
+    d.max_bins = bins;
+    d.max_count = d.min_count = count;
     d.tmaps = &h->map;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);

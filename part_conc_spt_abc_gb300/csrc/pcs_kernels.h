@@ -68,6 +68,9 @@ struct DistArgs {
     uint64_t* ssd;              /* [M][2] nullable: exact integer sum (hi, lo) */
     uint32_t* err;
     uint32_t max_rows;          /* rows of the carry array in shared memory */
+    uint32_t max_bins;          /* bins of the widest histogram */
+    uint32_t max_count;         /* histograms at most */
+    uint32_t min_count;         /* histograms at least, as far as the host knows */
     const TmapDev* tmaps;       /* nullable: per job (index of jobs), tensor maps over hist */
 };
 /* A standalone launch's tables, filled on the device (launch_distance_setup):
