@@ -1499,10 +1499,10 @@ int distance_ctas_per_sm(uint32_t max_rows, uint32_t cl)
     const size_t smem = distance_smem_bytes(max_rows, cl);
     int n = 0;
     if (use_strip(max_rows, cl)) {
-        cudaFuncSetAttribute(k_distance_strip<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(k_distance_strip<false, false>);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance_strip<false, false>, (int)kStripThreads, smem);
     } else {
-        cudaFuncSetAttribute(k_distance<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(k_distance<false>);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance<false>, 1024, smem);
     }
     return n > 0 ? n : 1;
@@ -1632,7 +1632,7 @@ static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st
     void (*k)(DistArgs);
     if (a.dist_f64) k = a.ssd ? k_distance_rows<true, true> : k_distance_rows<true, false>;
     else k = a.ssd ? k_distance_rows<false, true> : k_distance_rows<false, false>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRowsWarps * kRowsWarpBytes));
+    const cudaError_t e = allow_smem(k);
     if (e != cudaSuccess) return e;
     const uint32_t warps = (a.max_bins + 127u) / 128u;
     const size_t smem = (size_t)warps * kRowsWarpBytes;
@@ -1654,7 +1654,7 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
          * histogram of the launch has a cluster to itself; as many clusters
          * as fit at once, at most one per histogram slot */
         const size_t smem = distance_smem_bytes(a.max_rows, cl);
-        cudaError_t e = cudaFuncSetAttribute(k_distance_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(k_distance_cluster);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -1690,17 +1690,17 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
         void (*k)(DistArgs, uint32_t, uint32_t);
         if (a.dist_f64) k = a.ssd ? k_distance_strip<true, true> : k_distance_strip<true, false>;
         else k = a.ssd ? k_distance_strip<false, true> : k_distance_strip<false, false>;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(k);
         if (e != cudaSuccess) return e;
         k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u, rows ? 1u : 0u);
         return cudaGetLastError();
     }
     if (a.dist_f64) {
-        cudaError_t e = cudaFuncSetAttribute(k_distance<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(k_distance<true>);
         if (e != cudaSuccess) return e;
         k_distance<true><<<grid, 1024, smem, st>>>(a, rows ? 1u : 0u);
     } else {
-        cudaError_t e = cudaFuncSetAttribute(k_distance<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(k_distance<false>);
         if (e != cudaSuccess) return e;
         k_distance<false><<<grid, 1024, smem, st>>>(a, 0u);
     }

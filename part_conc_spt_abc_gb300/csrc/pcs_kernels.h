@@ -56,6 +56,18 @@ cudaError_t launch_debug_stream(uint64_t seed, uint32_t slot, uint32_t gen, uint
                                 uint32_t particle, uint32_t block, uint32_t* d_out,
                                 cudaStream_t st);
 
+/* Dynamic shared memory for a kernel, as much as a CTA may have.  The limit
+ * belongs to the kernel and not to the launch: set to each launch's own size,
+ * threads launching different sizes would lower it under one another. */
+template <typename F>
+inline cudaError_t allow_smem(F* fn)
+{
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227u * 1024u - fa.sharedSizeBytes));
+}
+
 /* ---------------- scan + distance (kernels_dist.cu) ---------------- */
 struct DistArgs {
     const JobDev* jobs;

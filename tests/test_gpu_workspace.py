@@ -45,7 +45,11 @@ def test_several_threads(pcs, ctx):
     def work(k):
         for i in range(3 * len(calls)):
             j = (i * 5 + k) % len(calls)
-            if not np.array_equal(calls[j](), want[j]):
+            try:
+                same = np.array_equal(calls[j](), want[j])
+            except Exception as e:  # noqa: BLE001 -- a thread's exception would be lost
+                same, j = False, (j, repr(e))
+            if not same:
                 wrong.append((k, j))
 
     threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
