@@ -574,9 +574,16 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
         if (RB > (1ull << 31)) throw Error(PCS_ERR_UNSUPPORTED, "histogram too large");
 
         cudaStream_t st = c.stream;
-        const uint32_t chunk = c.tune.chunk;
+        SimLaunch l{};
+        l.block = c.tune.block;
+        l.ppt = replay ? 1 : (int)c.tune.ppt;
+        l.replay = replay != nullptr;
+        l.aggregate = c.tune.aggregate == 1u;
+        l.split = !replay && c.split_walk();
+        const uint32_t tile_words = tile_words_for(std::min<uint32_t>(c.tune.tile_rows, R), B);
+        uint32_t chunk = c.tune.chunk;
         const uint64_t cstride = 2ull * V + 1ull;
-        uint64_t n_items = 0;
+        uint64_t n_items = 0, n_few = 0;
         std::vector<uint32_t> totals(count);
         for (uint32_t q = 0; q < count; ++q) {
             need(runs[q].particles, "run.particles");
@@ -585,6 +592,12 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
             if (total > 0xFFFFFFFFull) throw Error(PCS_ERR_INVALID_ARGUMENT, "too many particles");
             totals[q] = (uint32_t)total;
             n_items += (total + chunk - 1) / chunk;
+            n_few += (total + kFewChunk - 1) / kFewChunk;
+        }
+        if (simulate_few(l, tile_words, setup->kmin, n_few)) {
+            chunk = kFewChunk;
+            n_items = n_few;
+            l.few_items = (uint32_t)n_few;
         }
         if (replay) {
             need(replay->uniforms, "replay->uniforms");
@@ -678,7 +691,7 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
         a.queue_head = reinterpret_cast<uint32_t*>(d_in + o_ctl) + 1;
         a.chunk = chunk;
         a.err = c.err.as<uint32_t>();
-        a.tile_words = tile_words_for(std::min<uint32_t>(c.tune.tile_rows, R), B);
+        a.tile_words = tile_words;
         if (replay) {
             const uint64_t n = rp_n;
             float* du = ws.get<float>(4 * n);
@@ -694,14 +707,7 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
                 a.rp_sigmas = ds;
             }
         }
-        SimLaunch l{};
-        l.block = c.tune.block;
-        l.ppt = replay ? 1 : (int)c.tune.ppt;
-        l.replay = replay != nullptr;
-        l.aggregate = c.tune.aggregate == 1u;
-        l.split = !replay && c.split_walk();
-        int occ = simulate_occupancy(l, a.tile_words);
-        l.grid = (uint32_t)std::max(1, occ) * (uint32_t)c.sm_count;
+        if (!l.few_items) l.grid = (uint32_t)std::max(1, simulate_occupancy(l, a.tile_words)) * (uint32_t)c.sm_count;
         PCS_CUDA(launch_simulate(a, l, st));
         PCS_CUDA(cudaMemcpyAsync(hist_out, d_hist, count * RB * 4, cudaMemcpyDeviceToHost, st));
         finish(c, ws);

@@ -8,10 +8,11 @@
  * particles) pulled from a device counter, so proposals with uneven Poisson
  * particle counts pack densely onto all SMs.  Per particle the walk state
  * lives in registers.  k_simulate_walk, the default, records tracks by global
- * atomics and screens out the particles that are never detected; k_simulate
- * (a tile of histogram rows privatised in shared memory, several walkers per
- * thread, replayed draws) walks an item per CTA, and k_simulate_split is the
- * slab-split walk.
+ * atomics and screens out the particles that are never detected;
+ * k_simulate_few spreads the particles of small standalone calls over four or
+ * eight lanes each; k_simulate (a tile of histogram rows privatised in shared
+ * memory, several walkers per thread, replayed draws) walks an item per CTA,
+ * and k_simulate_split is the slab-split walk.
  *
  * Arithmetic contract: the walk, DE and binning use explicit round-to-nearest
  * intrinsics (__fmul_rn/__fadd_rn/__fdiv_rn) in the reference's evaluation
@@ -891,6 +892,131 @@ __global__ void __launch_bounds__(BLOCK, BLOCK <= 256u ? 3 : 1) k_simulate_walk(
 }
 
 /* ----------------------------------------------------------------------- */
+/* Few particles (k_simulate_few): L lanes per particle, 4 or 8.
+ *
+ * A launch of a few slices per scheduler takes as long as one walk's chain of
+ * Philox rounds, Box-Muller and steps, group after group, whatever its size.
+ * Here lane j of a particle's L draws the normals of frames 4j .. 4j+3 of a
+ * block of 4L, and then walks one coordinate (lane 0 x, 1 y, the others z)
+ * through all of them, the steps transposed through shared memory; the next
+ * block's normals are drawn meanwhile.  Each lane keeps a bit per frame for
+ * its coordinate lying in the detection region; two exchanges give the frames
+ * that find the particle, and only where there are any does the first lane
+ * extend and close tracks.  Every value is computed as in the other walks:
+ * the histogram is the same, count for count.
+ *
+ * Only the z coordinate's steps are repeated, so with 4 lanes a particle's
+ * frames take ~1.3 times the issue slots of a walk by one lane, with 8 ~1.5
+ * times; a group of four frames takes a lone warp 0.23 us (0.18) and not 0.8.
+ * Measured, k_simulate_walk -> 4 lanes -> 8 lanes in us, 200 frames: 2560
+ * particles 45 -> 22.8 -> 18.1, 8000 54 -> 25.9 -> 24.8, 16000 56 -> 29.3 ->
+ * 34.3, 48000 77 -> 54, 64000 77 -> 69, 96000 79 -> 93; 1000 frames: 2560
+ * 202 -> 75 -> 58, 8000 239 -> 87 -> 75, 64000 354 -> 281, 96000 354 -> 388;
+ * 50 frames: 2560 16.9 -> 11.0 -> 10.8, 64000 26.4 -> 26.8.  Hence the lines:
+ * 8 lanes to 8192 particles, 4 lanes to 65536.  The host has to know the
+ * number: standalone calls only. */
+constexpr uint32_t kFewItems = 65536u / kFewChunk, kFewItems8 = 8192u / kFewChunk;
+constexpr uint32_t kFewThreads = 64;
+
+/* frames s0 .. s0+nv-1 of the particle's track (bit t of `det`: found in frame s0 + t) */
+__device__ __forceinline__ void few_tracks_(const ItemCtx& c, uint32_t det, uint32_t nv, const float* dd, uint32_t& k, float& de)
+{
+    uint32_t f = 0u;
+    while (f < nv) {
+        uint32_t rest = det >> f;
+        if (!(rest & 1u)) { /* closed, up to the next frame that finds it */
+            if (k >= c.kmin) record_out_<false>(c.four_dt, c.dde, c.B, c.RB, 0u, c.hist, c.err, nullptr, k, de);
+            k = 0u;
+            de = 0.0f;
+            if (!rest) break;
+            f += (uint32_t)__ffs(rest) - 1u;
+            rest = det >> f;
+        }
+        const uint32_t end = min(f + (uint32_t)__clz((int)__brev(~rest)), nv);
+        if (k == 0u) { /* from the track's second frame on */
+            k = 1u;
+            ++f;
+        }
+        k += end - f;
+#pragma unroll 4
+        for (; f < end; ++f) de = __fadd_rn(de, dd[f]);
+    }
+}
+
+template <uint32_t L>
+__global__ void __launch_bounds__(kFewThreads, 12) k_simulate_few(const __grid_constant__ SimArgs a)
+{
+    /* a particle's x, y, z steps and squared displacements of a block's
+     * frames: rows of 4L + 4, free of bank conflicts either way */
+    constexpr uint32_t kParticles = 32u / L, kFrames = 4u * L, kRow = kFrames + 4u;
+    __shared__ __align__(16) float s_steps[kFewThreads / 32u][kParticles * 4u * kRow];
+    const uint32_t lane = threadIdx.x & 31u, j = lane % L;
+    const uint32_t slices = (a.chunk + kParticles - 1u) / kParticles;
+    const uint32_t sl = blockIdx.x * (kFewThreads / 32u) + (threadIdx.x >> 5);
+    const uint32_t item = sl / slices, part = sl - item * slices;
+    if (item >= *a.n_items) return; /* whole warp */
+    const PropDev& prop = a.props[a.item_prop[item]];
+    const JobDev& job = a.jobs[prop.job];
+    const uint32_t i0 = (item - prop.item_begin) * a.chunk;
+    const uint32_t n = i0 + part * kParticles + lane / L;
+    const bool real = part * kParticles + lane / L < a.chunk && n < prop.total_particles;
+    if (!__any_sync(0xFFFFFFFFu, real)) return;
+    const ItemCtx c = item_ctx_(a, job, prop);
+    Walker q;
+    q.F = q.k = 0u;
+    q.x = q.y = q.z = q.sd = q.haz = 0.0f;
+    if (real) {
+        init_walker_<false, true>(a, c, job, prop, a.counts + prop.counts_off + job.V, n, prop.slot,
+                                  pcs_ctr_gen_trial(prop.gen, prop.trial), job.seed_lo, job.seed_hi, q);
+    } else {
+        q.ph = pcs_philox_prepare(0u, 0u, 0u, 0u, 0u);
+    }
+    float v = j == 0u ? q.x : (j == 1u ? q.y : q.z);
+    const float half_l = j == 0u ? c.hlx : (j == 1u ? c.hly : c.hlz);
+    const float half_a = j == 0u ? c.hax : (j == 1u ? c.hay : q.haz);
+    float* mine = s_steps[threadIdx.x >> 5] + lane / L * 4u * kRow;
+    const float* walk = mine + min(j, 2u) * kRow;
+    uint32_t k = j == 0u ? q.k : 0u;
+    float de = 0.0f;
+    const uint32_t f_max = __reduce_max_sync(0xFFFFFFFFu, q.F);
+    float nn[12];
+    group_normals_<false>(a, q, 1u + 4u * j, nn);
+    for (uint32_t s0 = 1u; s0 < f_max; s0 += kFrames) {
+        __syncwarp(); /* the block before is read */
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            *reinterpret_cast<float4*>(mine + x * (int)kRow + 4u * j) = make_float4(nn[x], nn[3 + x], nn[6 + x], nn[9 + x]);
+        float dd[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            dd[t] = __fadd_rn(__fmul_rn(nn[3 * t], nn[3 * t]), __fmul_rn(nn[3 * t + 1], nn[3 * t + 1]));
+        *reinterpret_cast<float4*>(mine + 3u * kRow + 4u * j) = make_float4(dd[0], dd[1], dd[2], dd[3]);
+        __syncwarp();
+        group_normals_<false>(a, q, s0 + kFrames + 4u * j, nn); /* past the last frame: not used */
+        uint32_t in = 0u;
+#pragma unroll
+        for (uint32_t g = 0; g < L; ++g) {
+            const float4 d = *reinterpret_cast<const float4*>(walk + 4u * g);
+            const float step[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (uint32_t t = 0; t < 4u; ++t) {
+                v = wrap_(__fadd_rn(v, step[t]), half_l, 2.0f * half_l);
+                in |= fabsf(v) <= half_a ? 1u << (4u * g + t) : 0u;
+            }
+        }
+        in &= __shfl_xor_sync(0xFFFFFFFFu, in, 1);
+        in &= __shfl_xor_sync(0xFFFFFFFFu, in, 2); /* all three coordinates', in lanes 0 .. 3 */
+        const uint32_t nv = q.F > s0 ? min(q.F - s0, kFrames) : 0u;
+        in &= nv < 32u ? (1u << nv) - 1u : 0xFFFFFFFFu;
+        /* the vote keeps the warp together where no lane has any */
+        if (__any_sync(0xFFFFFFFFu, j == 0u && (in | k) != 0u)) {
+            if (j == 0u) few_tracks_(c, in, nv, mine + 3u * kRow, k, de);
+            __syncwarp();
+        }
+    }
+    if (j == 0u && q.F > 0u && k >= c.kmin) record_out_<false>(c.four_dt, c.dde, c.B, c.RB, 0u, c.hist, c.err, nullptr, k, de);
+}
+
 /* The slab-split walk (k_simulate_split).
  *
  * Same model as k_simulate, fewer draws: a particle can only be detected
@@ -1233,6 +1359,15 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
         return l.aggregate ? launch_split_<true>(a, l.grid, smem, st) : launch_split_<false>(a, l.grid, smem, st);
     }
     const SimArgs& a = a_in;
+    if (l.few_items) {
+        if (a.chunk != kFewChunk) return cudaErrorInvalidValue;
+        const uint32_t per = kFewThreads / 32u;
+        if (l.few_items <= kFewItems8)
+            k_simulate_few<8><<<(l.few_items * (kFewChunk / 4u) + per - 1u) / per, kFewThreads, 0, st>>>(a);
+        else
+            k_simulate_few<4><<<(l.few_items * (kFewChunk / 8u) + per - 1u) / per, kFewThreads, 0, st>>>(a);
+        return cudaGetLastError();
+    }
     if (walk_launch_(l, a.tile_words)) {
         const auto fn = walk_kernel_(l.block);
         const size_t tracks = walk_smem_(l.block);
@@ -1256,6 +1391,13 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
     PCS_SIM_CASE(1, true, true)
 #undef PCS_SIM_CASE
     return cudaErrorInvalidValue;
+}
+
+bool simulate_few(const SimLaunch& l, uint32_t tile_words, uint32_t kmin, uint64_t items)
+{
+    /* kmin 0 records an empty track for every frame that does not find the
+     * particle, which the runs of few_tracks_ do not see */
+    return !l.split && walk_launch_(l, tile_words) && kmin >= 1u && items <= kFewItems;
 }
 
 int simulate_occupancy(const SimLaunch& l, uint32_t tile_words)

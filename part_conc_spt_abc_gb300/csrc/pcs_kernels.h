@@ -46,12 +46,16 @@ struct SimLaunch {
     bool replay;
     bool aggregate;
     bool split; /* slab-split walk (k_simulate_split: 256 threads, 1 particle each, no replay) */
+    uint32_t few_items; /* the number of items of kFewChunk particles where simulate_few says so, else 0 */
 };
 
 cudaError_t launch_simulate(const SimArgs& a, const SimLaunch& l, cudaStream_t st);
 /* largest CTA the forward model's build for `ppt` walkers per thread launches */
 __host__ __device__ constexpr uint32_t sim_max_block(int ppt) { return ppt == 1 ? 1024u : (ppt == 2 ? 512u : 256u); }
 int simulate_occupancy(const SimLaunch& l, uint32_t tile_words);
+/* whether a launch of `items` items of kFewChunk particles is one for k_simulate_few */
+constexpr uint32_t kFewChunk = 32;
+bool simulate_few(const SimLaunch& l, uint32_t tile_words, uint32_t kmin, uint64_t items);
 cudaError_t launch_debug_stream(uint64_t seed, uint32_t slot, uint32_t gen, uint32_t trial,
                                 uint32_t particle, uint32_t block, uint32_t* d_out,
                                 cudaStream_t st);
