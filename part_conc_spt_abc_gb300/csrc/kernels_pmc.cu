@@ -741,171 +741,287 @@ __device__ void start_generation_(JobPmcDev& pm)
     pm.gen_ended = 0u;
 }
 
-/* finalize: one block per job whose generation ended this round */
-constexpr uint32_t kWcumChunk = 1024;
+/* block_sum_ of K values at once, to s_out: the same sums in the same order,
+ * with one pair of barriers, the second stages by K warps.  Threads from n
+ * on hold zeros, so warps past n only write theirs (FP64 runs at one warp
+ * instruction per ~16 cycles and SM: 32 warps' trees take 2600 cycles). */
+template <uint32_t K>
+__device__ void block_sums_(const double* v, uint32_t n, double (*s_part)[32], double* s_out)
+{
+    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u, nw = blockDim.x >> 5;
+    static_assert(K <= 32u, "a warp per value");
+    __syncthreads(); /* s_part and s_out are read */
+#pragma unroll
+    for (uint32_t k = 0; k < K; ++k) {
+        double t = v[k];
+        if (32u * w < n)
+            for (int d = 16; d >= 1; d >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, d);
+        if (l == 0u) s_part[k][w] = t;
+    }
+    __syncthreads();
+    if (w < K) {
+        double t = l < nw ? s_part[w][l] : 0.0;
+        for (int d = 16; d >= 1; d >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, d);
+        if (l == 0u) s_out[w] = t;
+    }
+    __syncthreads();
+}
 
-__global__ void __launch_bounds__(1024) k_finalize(PmcArgs a)
+/* finalize: a cluster of 8 CTAs per job whose generation ended this round.
+ * What does not depend on one another runs at the same time: CTA 0 has the
+ * weights and their cumulative sums (a serial chain), CTAs 1-6 the
+ * perturbation factor's moments, CTA 7 the next epsilon (selection), the
+ * population's commit and the slots' reset.  The moments with weights start
+ * when the weights are there (one cluster barrier); after the last barrier
+ * CTA 0 factorises the covariance and starts the next generation.  Bound by
+ * chains of FP64 operations (a dependent addition every ~60 cycles, a warp
+ * instruction per ~16 cycles and SM).  In one CTA, one after another: N = 256,
+ * P = 4 52 us, N = 840, P = 7 119 us, N = 1024, P = 7 with the covariance
+ * 195 us; here 22, 48 and 76
+ * us (rounds' PMC kernels of a job: configuration 0 1.63 -> 1.29 ms,
+ * configuration 1 1.57 -> 1.06 ms, four served jobs 2.30 -> 1.65 ms). */
+constexpr uint32_t kWcumChunk = 1024;
+constexpr uint32_t kFinCtas = 8, kFinMoments = 6; /* CTAs per cluster; of these for the moments */
+
+__device__ __forceinline__ void fin_cluster_sync_()
+{
+    __syncwarp(); /* the barrier is the whole warp's */
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+/* s_wc[0 .. m) and acc become cumulative sums, by one thread in order; eight
+ * values are read ahead of the chain (a load behind a store to the same array
+ * waits for it: 110 cycles per value) */
+__device__ __forceinline__ void wcum_chain_(double* s_wc, uint32_t m, double& acc)
+{
+    constexpr uint32_t U = 8;
+    double v[U];
+    uint32_t i = 0;
+    if (m >= U)
+#pragma unroll
+        for (uint32_t t = 0; t < U; ++t) v[t] = s_wc[t];
+    for (; i + U <= m; i += U) {
+        double nx[U];
+#pragma unroll
+        for (uint32_t t = 0; t < U; ++t) nx[t] = s_wc[min(i + U + t, m - 1u)];
+#pragma unroll
+        for (uint32_t t = 0; t < U; ++t) {
+            acc += v[t];
+            s_wc[i + t] = acc;
+        }
+#pragma unroll
+        for (uint32_t t = 0; t < U; ++t) v[t] = nx[t];
+    }
+    for (; i < m; ++i) {
+        acc += s_wc[i];
+        s_wc[i] = acc;
+    }
+}
+
+/* pm.w: the new population's normalised weights */
+__device__ __forceinline__ void fin_weights_(JobPmcDev& pm, double* s_red)
+{
+    const uint32_t N = pm.N, tid = threadIdx.x, bd = blockDim.x;
+    double s = 0.0;
+    if (pm.weighting == 0u) {
+        double mx = -INFINITY;
+        for (uint32_t i = tid; i < N; i += bd) mx = fmax(mx, pm.scratch[i]);
+        mx = block_max_(mx, s_red);
+        for (uint32_t i = tid; i < N; i += bd) {
+            const double e = exp(pm.scratch[i] - mx);
+            pm.scratch[i] = e;
+            s += e;
+        }
+    } else {
+        /* inverse-distance-squared (:872-887) */
+        for (uint32_t i = tid; i < N; i += bd) {
+            const double d = pm.dist_new[i];
+            const double wv = 1.0 / (d * d);
+            pm.scratch[i] = wv;
+            s += wv;
+        }
+    }
+    s = block_sum_(s, s_red);
+    for (uint32_t i = tid; i < N; i += bd) pm.w[i] = pm.scratch[i] / s;
+    __syncthreads();
+}
+
+/* cumulative weights (partial_sum, :222): one thread adds them in the
+ * reference's order, from a shared-memory copy of each 1024-weight chunk */
+__device__ __forceinline__ void fin_wcum_(JobPmcDev& pm, double* s_wc)
+{
+    const uint32_t N = pm.N, tid = threadIdx.x, bd = blockDim.x;
+    double acc = 0.0; /* thread 0's running sum across chunks */
+    for (uint32_t base = 0; base < N; base += kWcumChunk) {
+        const uint32_t m = min(kWcumChunk, N - base);
+        for (uint32_t i = tid; i < m; i += bd) s_wc[i] = pm.w[base + i];
+        __syncthreads();
+        if (tid == 0) wcum_chain_(s_wc, m, acc);
+        __syncthreads();
+        for (uint32_t i = tid; i < m; i += bd) pm.wcum[base + i] = s_wc[i];
+        __syncthreads();
+    }
+}
+
+/* compute_tau_ (:733-749) of parameters first, first + kFinMoments, ...:
+ * tau = sqrt(2 var), uncorrected 1/N variance */
+__device__ __forceinline__ void fin_tau_(JobPmcDev& pm, const double* theta, uint32_t first, double (*s_part)[32], double* s_out)
+{
+    const uint32_t N = pm.N, P = pm.P, tid = threadIdx.x, bd = blockDim.x;
+    for (uint32_t p = first; p < P; p += kFinMoments) {
+        double s = 0.0;
+        for (uint32_t i = tid; i < N; i += bd) s += theta[(uint64_t)i * P + p];
+        block_sums_<1>(&s, N, s_part, s_out);
+        const double mean = s_out[0] / (double)N;
+        double v = 0.0;
+        for (uint32_t i = tid; i < N; i += bd) {
+            const double x = theta[(uint64_t)i * P + p] - mean;
+            v += x * x;
+        }
+        block_sums_<1>(&v, N, s_part, s_out);
+        for (uint32_t q = tid; q < P; q += bd)
+            pm.factor[p * P + q] = q == p ? sqrt(2.0 * (s_out[0] / (double)N)) : 0.0;
+    }
+}
+
+/* 2 x weighted covariance (Beaumont et al. 2009), entries first, first +
+ * kFinMoments, ... of the lower triangle row by row, into pm.factor */
+__device__ __forceinline__ void fin_covariance_(JobPmcDev& pm, const double* theta, uint32_t first, double (*s_part)[32],
+                                                double* s_out, double* s_mean)
+{
+    const uint32_t N = pm.N, P = pm.P, tid = threadIdx.x, bd = blockDim.x;
+    constexpr uint32_t K = 4;
+    for (uint32_t p0 = 0; p0 < P; p0 += K) { /* every CTA has all the means */
+        double s[K] = {0.0, 0.0, 0.0, 0.0};
+        for (uint32_t i = tid; i < N; i += bd) {
+            const double wi = pm.w[i];
+#pragma unroll
+            for (uint32_t k = 0; k < K; ++k)
+                if (p0 + k < P) s[k] += wi * theta[(uint64_t)i * P + p0 + k];
+        }
+        block_sums_<K>(s, N, s_part, s_out);
+        if (tid < K && p0 + tid < P) s_mean[p0 + tid] = s_out[tid];
+    }
+    __syncthreads();
+    const uint32_t pairs = P * (P + 1u) / 2u;
+    for (uint32_t e0 = first; e0 < pairs; e0 += K * kFinMoments) {
+        double s[K] = {0.0, 0.0, 0.0, 0.0};
+        uint32_t pk[K], qk[K];
+#pragma unroll
+        for (uint32_t k = 0; k < K; ++k) {
+            const uint32_t e = min(e0 + k * kFinMoments, pairs - 1u);
+            uint32_t p = 0;
+            while ((p + 1u) * (p + 2u) / 2u <= e) ++p;
+            pk[k] = p;
+            qk[k] = e - p * (p + 1u) / 2u;
+        }
+        for (uint32_t i = tid; i < N; i += bd) {
+            const double* t = theta + (uint64_t)i * P;
+            const double wi = pm.w[i];
+#pragma unroll
+            for (uint32_t k = 0; k < K; ++k)
+                if (e0 + k * kFinMoments < pairs) s[k] += wi * (t[pk[k]] - s_mean[pk[k]]) * (t[qk[k]] - s_mean[qk[k]]);
+        }
+        block_sums_<K>(s, N, s_part, s_out);
+        if (tid < K && e0 + tid * kFinMoments < pairs) {
+            const uint32_t e = e0 + tid * kFinMoments;
+            uint32_t p = 0;
+            while ((p + 1u) * (p + 2u) / 2u <= e) ++p;
+            const uint32_t q = e - p * (p + 1u) / 2u;
+            pm.factor[p * P + q] = pm.factor[q * P + p] = 2.0 * s_out[tid];
+        }
+    }
+}
+
+/* pm.factor, a covariance, becomes its lower Cholesky factor (one thread) */
+__device__ void fin_cholesky_(JobPmcDev& pm, double* s_cov)
+{
+    const uint32_t P = pm.P;
+    for (uint32_t x = 0; x < P * P; ++x) {
+        s_cov[x] = pm.factor[x];
+        pm.factor[x] = 0.0;
+    }
+    for (uint32_t c = 0; c < P; ++c) {
+        if (pm.fixed[c]) continue;
+        double d = s_cov[c * P + c];
+        for (uint32_t t = 0; t < c; ++t)
+            if (!pm.fixed[t]) d -= pm.factor[c * P + t] * pm.factor[c * P + t];
+        const double lv = sqrt(fmax(d, 1e-300));
+        pm.factor[c * P + c] = lv;
+        for (uint32_t r = c + 1; r < P; ++r) {
+            if (pm.fixed[r]) continue;
+            double s = s_cov[r * P + c];
+            for (uint32_t t = 0; t < c; ++t)
+                if (!pm.fixed[t]) s -= pm.factor[r * P + t] * pm.factor[c * P + t];
+            pm.factor[r * P + c] = s / lv;
+        }
+    }
+}
+
+__global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(1024) k_finalize(PmcArgs a)
 {
     __shared__ double s_red[32];
     __shared__ double s_wc[kWcumChunk];
-    __shared__ double s_sel;
+    __shared__ double s_part[4][32], s_out[4];
     __shared__ double s_mean[PCS_MAX_P];
     __shared__ double s_cov[PCS_MAX_P * PCS_MAX_P];
     __shared__ SelectShared s_select;
-    const uint32_t j = blockIdx.x;
-    RoundDev* rd = a.round;
-    if (j >= rd->n_jobs) return;
-    JobPmcDev& pm = a.pmc[j];
-    if (pm.done || !pm.gen_ended) return;
-    const uint32_t N = pm.N, P = pm.P;
-    const uint32_t tid = threadIdx.x, bd = blockDim.x;
-
-    bool commit = true;
-    if (pm.generation == 0u) {
-        /* prior pass: gamma_0 from the median distance (compute_initial_gamma_ :819-829) */
-        const uint32_t target = (pm.schedule == 1u) ? min(N - 1u, (uint32_t)floor(pm.quantile * N)) : N / 2u;
-        const double g0 = select_rank_(pm.dist_new, N, target, s_select);
-        if (tid == 0) pm.gamma = g0;
-        /* the reference keeps the prior population as drawn; the quantile
-         * schedule keeps its distances as the generation-0 distances */
-        for (uint32_t i = tid; i < N; i += bd) pm.dist[i] = (pm.schedule == 1u) ? pm.dist_new[i] : 0.0;
-        commit = false;
-    } else if ((double)pm.trials >= (double)pm.avg_trials * (double)pm.N) {
-        /* trial cap: converged, discard this generation (:425-428) */
-        if (tid == 0) {
-            pm.converged = 1u;
-            pm.done = 1u;
-        }
-        return;
-    }
-
-    if (commit) {
-        /* weights */
-        if (pm.weighting == 0u) {
-            double mx = -INFINITY;
-            for (uint32_t i = tid; i < N; i += bd) mx = fmax(mx, pm.scratch[i]);
-            mx = block_max_(mx, s_red);
-            double s = 0.0;
-            for (uint32_t i = tid; i < N; i += bd) {
-                const double e = exp(pm.scratch[i] - mx);
-                pm.scratch[i] = e;
-                s += e;
+    const uint32_t rank = blockIdx.x % kFinCtas, tid = threadIdx.x, bd = blockDim.x;
+    const uint32_t n_jobs = a.round->n_jobs;
+    for (uint32_t j = blockIdx.x / kFinCtas; j < n_jobs; j += gridDim.x / kFinCtas) {
+        JobPmcDev& pm = a.pmc[j];
+        if (pm.done || !pm.gen_ended) continue;
+        const uint32_t N = pm.N, P = pm.P;
+        /* generation 0: the prior pass's population stays as it was drawn */
+        const bool commit = pm.generation != 0u, covariance = pm.perturbation != 0u;
+        if (commit && (double)pm.trials >= (double)pm.avg_trials * (double)pm.N) {
+            /* trial cap: converged, discard this generation (:425-428); the
+             * other CTAs pass the job by whether they see this or not */
+            if (rank == 0u && tid == 0) {
+                pm.converged = 1u;
+                pm.done = 1u;
             }
-            s = block_sum_(s, s_red);
-            for (uint32_t i = tid; i < N; i += bd) pm.w[i] = pm.scratch[i] / s;
+            continue;
+        }
+        const double* theta = commit ? pm.theta_new : pm.theta;
+        double gamma = pm.gamma; /* CTA 0: the old one */
+        if (rank == 0u) {
+            if (commit) fin_weights_(pm, s_red);
+            if (covariance) fin_cluster_sync_();
+            fin_wcum_(pm, s_wc);
+        } else if (rank <= kFinMoments) {
+            if (covariance) {
+                fin_cluster_sync_(); /* the weights */
+                fin_covariance_(pm, theta, rank - 1u, s_part, s_out, s_mean);
+            } else {
+                fin_tau_(pm, theta, rank - 1u, s_part, s_out);
+            }
         } else {
-            /* inverse-distance-squared (:872-887) */
-            double s = 0.0;
+            if (covariance) fin_cluster_sync_();
+            /* gamma_0 from the median distance (compute_initial_gamma_
+             * :819-829), or the next epsilon of the quantile schedule */
+            if (!commit || pm.schedule == 1u) {
+                const uint32_t target = pm.schedule == 1u ? min(N - 1u, (uint32_t)floor(pm.quantile * N)) : N / 2u;
+                gamma = select_rank_(pm.dist_new, N, target, s_select);
+            }
+            /* commit the new population (:434-450); the quantile schedule
+             * keeps the prior pass's distances as the generation-0 distances */
+            if (commit)
+                for (uint64_t i = tid; i < (uint64_t)N * P; i += bd) pm.theta[i] = pm.theta_new[i];
             for (uint32_t i = tid; i < N; i += bd) {
-                const double d = pm.dist_new[i];
-                const double wv = 1.0 / (d * d);
-                pm.scratch[i] = wv;
-                s += wv;
-            }
-            s = block_sum_(s, s_red);
-            for (uint32_t i = tid; i < N; i += bd) pm.w[i] = pm.scratch[i] / s;
-        }
-        /* commit the new population (:434-450) */
-        for (uint64_t i = tid; i < (uint64_t)N * P; i += bd) pm.theta[i] = pm.theta_new[i];
-        for (uint32_t i = tid; i < N; i += bd) pm.dist[i] = pm.dist_new[i];
-        __syncthreads();
-    }
-
-    /* cumulative weights (partial_sum, :222): one thread adds them in the
-     * reference's order, from a shared-memory copy of each 1024-weight chunk
-     * (a chain through global memory would wait for every load in turn) */
-    {
-        double acc = 0.0; /* thread 0's running sum across chunks */
-        for (uint32_t base = 0; base < N; base += kWcumChunk) {
-            const uint32_t m = min(kWcumChunk, N - base);
-            for (uint32_t i = tid; i < m; i += bd) s_wc[i] = pm.w[base + i];
-            __syncthreads();
-            if (tid == 0) {
-                for (uint32_t i = 0; i < m; ++i) {
-                    acc += s_wc[i];
-                    s_wc[i] = acc;
-                }
-            }
-            __syncthreads();
-            for (uint32_t i = tid; i < m; i += bd) pm.wcum[base + i] = s_wc[i];
-            __syncthreads();
-        }
-    }
-    /* perturbation factor from the (new) committed population */
-    if (pm.perturbation == 0u) {
-        /* compute_tau_ (:733-749): tau = sqrt(2 var), uncorrected 1/N variance */
-        for (uint32_t p = 0; p < P; ++p) {
-            double s = 0.0;
-            for (uint32_t i = tid; i < N; i += bd) s += pm.theta[(uint64_t)i * P + p];
-            s = block_sum_(s, s_red);
-            const double mean = s / (double)N;
-            double v = 0.0;
-            for (uint32_t i = tid; i < N; i += bd) {
-                const double x = pm.theta[(uint64_t)i * P + p] - mean;
-                v += x * x;
-            }
-            v = block_sum_(v, s_red);
-            if (tid == 0) {
-                for (uint32_t q = 0; q < P; ++q) pm.factor[p * P + q] = 0.0;
-                pm.factor[p * P + p] = sqrt(2.0 * (v / (double)N));
+                pm.dist[i] = commit || pm.schedule == 1u ? pm.dist_new[i] : 0.0;
+                pm.pending[i] = i;
+                pm.next_trial[i] = 0u;
+                pm.accepted[i] = 0u;
             }
         }
-    } else {
-        /* 2 x weighted covariance and its Cholesky factor (Beaumont et al. 2009) */
-        for (uint32_t p = 0; p < P; ++p) {
-            double s = 0.0;
-            for (uint32_t i = tid; i < N; i += bd) s += pm.w[i] * pm.theta[(uint64_t)i * P + p];
-            s = block_sum_(s, s_red);
-            if (tid == 0) s_mean[p] = s;
+        fin_cluster_sync_();
+        if (rank == 0u && tid == 0 && covariance) fin_cholesky_(pm, s_cov);
+        if (rank == kFinCtas - 1u && tid == 0) {
+            pm.gamma = gamma;
+            start_generation_(pm);
         }
-        __syncthreads();
-        for (uint32_t p = 0; p < P; ++p)
-            for (uint32_t q = 0; q <= p; ++q) {
-                double s = 0.0;
-                for (uint32_t i = tid; i < N; i += bd) {
-                    const double* t = pm.theta + (uint64_t)i * P;
-                    s += pm.w[i] * (t[p] - s_mean[p]) * (t[q] - s_mean[q]);
-                }
-                s = block_sum_(s, s_red);
-                if (tid == 0) s_cov[p * P + q] = s_cov[q * P + p] = 2.0 * s;
-            }
-        __syncthreads();
-        if (tid == 0) {
-            for (uint32_t x = 0; x < P * P; ++x) pm.factor[x] = 0.0;
-            for (uint32_t c = 0; c < P; ++c) {
-                if (pm.fixed[c]) continue;
-                double d = s_cov[c * P + c];
-                for (uint32_t t = 0; t < c; ++t)
-                    if (!pm.fixed[t]) d -= pm.factor[c * P + t] * pm.factor[c * P + t];
-                const double lv = sqrt(fmax(d, 1e-300));
-                pm.factor[c * P + c] = lv;
-                for (uint32_t r = c + 1; r < P; ++r) {
-                    if (pm.fixed[r]) continue;
-                    double s = s_cov[r * P + c];
-                    for (uint32_t t = 0; t < c; ++t)
-                        if (!pm.fixed[t]) s -= pm.factor[r * P + t] * pm.factor[c * P + t];
-                    pm.factor[r * P + c] = s / lv;
-                }
-            }
-        }
-    }
-    __syncthreads();
-
-    /* epsilon for the next generation */
-    if (pm.schedule == 1u && pm.generation > 0u) {
-        const uint32_t target = min(N - 1u, (uint32_t)floor(pm.quantile * N));
-        const double eps = select_rank_(pm.dist, N, target, s_select);
-        if (tid == 0) s_sel = eps;
-        __syncthreads();
-    }
-    if (tid == 0) {
-        if (pm.schedule == 1u && pm.generation > 0u) pm.gamma = s_sel;
-        start_generation_(pm);
-    }
-    for (uint32_t i = tid; i < N; i += bd) {
-        pm.pending[i] = i;
-        pm.next_trial[i] = 0u;
-        pm.accepted[i] = 0u;
+        __syncthreads(); /* s_cov, s_out and the rest are free */
     }
 }
 
@@ -1053,7 +1169,7 @@ cudaError_t launch_finalize(const PmcArgs& a, uint32_t n_jobs, uint32_t max_n, c
     /* grids for one job's points; the kernels stride over the round's jobs */
     k_whiten<<<(2u * max_n + 255) / 256, 256, 0, st>>>(a);
     k_kernel_sum<<<(max_n * 32u + 255) / 256, 256, 0, st>>>(a);
-    k_finalize<<<n_jobs, 1024, 0, st>>>(a);
+    k_finalize<<<(n_jobs + kFinCtas - 1u) / kFinCtas * kFinCtas, 1024, 0, st>>>(a);
     return cudaGetLastError();
 }
 
