@@ -627,6 +627,9 @@ void Ctx::enqueue_round()
     a.err = err.as<uint32_t>();
     a.logfact = logfact.as<double>();
     a.logfact_n = kLogFactEntries;
+    a.h_pmc = h_status;
+    a.h_round = h_round_out;
+    a.h_err = h_err;
     a.use_f64_distance = 0u;
     for (Job* j : table)
         if (j && j->p.distance_double) a.use_f64_distance = 1u;
@@ -684,9 +687,6 @@ void Ctx::enqueue_round()
     PCS_CUDA(launch_accept(a, kMaxRoundJobs, stream));
     PCS_CUDA(launch_finalize(a, kMaxRoundJobs, rb.max_n, stream));
     PCS_CUDA(cudaEventRecordWithFlags(ev_pmc1, stream, cudaEventRecordExternal));
-    PCS_CUDA(cudaMemcpyAsync(h_status, rb.pmc.p, sizeof(JobPmcDev) * kMaxRoundJobs, cudaMemcpyDeviceToHost, stream));
-    PCS_CUDA(cudaMemcpyAsync(h_err, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-    PCS_CUDA(cudaMemcpyAsync(h_round_out, rb.round.p, sizeof(RoundDev), cudaMemcpyDeviceToHost, stream));
 }
 
 void Ctx::run_round(double* ms_out)

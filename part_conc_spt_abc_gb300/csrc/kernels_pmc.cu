@@ -958,6 +958,18 @@ __device__ void fin_cholesky_(JobPmcDev& pm, double* s_cov)
     }
 }
 
+/* x, as this CTA's threads left it, to pinned host memory: the host reads it
+ * when the round has ended (three copies behind the kernel took 10 us a round;
+ * this takes 2.5) */
+template <typename T>
+__device__ __forceinline__ void report_(T& host, const T& x)
+{
+    static_assert(sizeof(T) % 4u == 0u, "words");
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < sizeof(T) / 4u; i += blockDim.x)
+        reinterpret_cast<volatile uint32_t*>(&host)[i] = reinterpret_cast<const volatile uint32_t*>(&x)[i];
+}
+
 __global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(1024) k_finalize(PmcArgs a)
 {
     __shared__ double s_red[32];
@@ -970,16 +982,23 @@ __global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(1024) k_final
     const uint32_t n_jobs = a.round->n_jobs;
     for (uint32_t j = blockIdx.x / kFinCtas; j < n_jobs; j += gridDim.x / kFinCtas) {
         JobPmcDev& pm = a.pmc[j];
-        if (pm.done || !pm.gen_ended) continue;
+        if (pm.done || !pm.gen_ended) {
+            if (rank == kFinCtas - 1u) report_(a.h_pmc[j], pm);
+            continue;
+        }
         const uint32_t N = pm.N, P = pm.P;
         /* generation 0: the prior pass's population stays as it was drawn */
         const bool commit = pm.generation != 0u, covariance = pm.perturbation != 0u;
         if (commit && (double)pm.trials >= (double)pm.avg_trials * (double)pm.N) {
             /* trial cap: converged, discard this generation (:425-428); the
              * other CTAs pass the job by whether they see this or not */
-            if (rank == 0u && tid == 0) {
-                pm.converged = 1u;
-                pm.done = 1u;
+            if (rank == kFinCtas - 1u) {
+                __syncthreads(); /* the CTA has read them */
+                if (tid == 0) {
+                    pm.converged = 1u;
+                    pm.done = 1u;
+                }
+                report_(a.h_pmc[j], pm);
             }
             continue;
         }
@@ -1017,11 +1036,18 @@ __global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(1024) k_final
         }
         fin_cluster_sync_();
         if (rank == 0u && tid == 0 && covariance) fin_cholesky_(pm, s_cov);
-        if (rank == kFinCtas - 1u && tid == 0) {
-            pm.gamma = gamma;
-            start_generation_(pm);
+        if (rank == kFinCtas - 1u) {
+            if (tid == 0) {
+                pm.gamma = gamma;
+                start_generation_(pm);
+            }
+            report_(a.h_pmc[j], pm);
         }
         __syncthreads(); /* s_cov, s_out and the rest are free */
+    }
+    if (blockIdx.x == 0u) { /* no kernel from here on changes these */
+        report_(*a.h_round, *a.round);
+        report_(*a.h_err, *a.err);
     }
 }
 

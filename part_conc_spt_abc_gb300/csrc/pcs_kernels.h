@@ -205,6 +205,10 @@ struct PmcArgs {
     uint32_t use_f64_distance;
     uint32_t logfact_n;       /* entries of logfact */
     const double* logfact;    /* nullable: log(k!) for k < logfact_n, for the Poisson sampler */
+    /* what the host reads after a round, in pinned host memory (k_finalize) */
+    JobPmcDev* h_pmc;
+    RoundDev* h_round;
+    uint32_t* h_err;
 };
 
 /* entries of the device log-factorial table (covers 1e5 particles per video) */
