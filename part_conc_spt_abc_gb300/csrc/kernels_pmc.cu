@@ -227,7 +227,7 @@ __device__ __forceinline__ uint32_t warp_pick_(const double* wcum, uint32_t N, d
     return lo < N ? lo : N - 1u;
 }
 
-/* One warp per proposal.  The FP64 work is spread over the lanes: lane i
+/* Two warps per proposal.  The FP64 work is spread over the lanes: lane i
  * draws perturbation normal pair i, lane p perturbs and reflects parameter p,
  * lane c computes component c's arguments (10^log10c, step sd); the Poisson
  * constants are computed once and the lanes draw the per-video counts in
@@ -235,28 +235,49 @@ __device__ __forceinline__ uint32_t warp_pick_(const double* wcum, uint32_t N, d
  * video prefix.  Every value is the one pcs_build_theta / pcs_build_args /
  * pcs_draw_counts compute (same functions, same operation order).
  *
- * Bound by FP64 (a warp instruction occupies an SM's FP64 unit for about 16
- * cycles), so a round's warps are spread over all SMs: warp w of CTA b takes
- * proposal w x CTAs + b.  Eight consecutive proposals per CTA left the 213
- * proposals of configuration 0's average round on 27 SMs.  The parameters
- * and the descriptor are put together in shared memory and written by the
- * whole warp, not in each lane's local memory. */
-constexpr uint32_t kProposeWarps = 4;
+ * Bound by one proposal's chain of FP64 operations (a dependent one every ~60
+ * cycles, a warp instruction per ~16 cycles and SM), so what is independent
+ * goes side by side: warp 0 draws the normals' radii, perturbs and sorts, and
+ * has the concentrations, the Poisson constants and the counts; warp 1 picks
+ * the parent, draws the normals' angles, and has the step sds, the logarithm
+ * of the Poisson mean and the descriptor.  (One warp for all of it: 33000
+ * cycles, 25.7 us a launch; two: 21.4.)  A round's warps are spread over all
+ * SMs: pair w of CTA b takes proposal w x CTAs + b.  The parameters and the
+ * descriptor are put together in shared memory and written by a whole warp,
+ * not in each lane's local memory. */
+constexpr uint32_t kProposePairs = 2;
 
-struct ProposeWarp {
-    double th[PCS_MAX_P], nrm[PCS_MAX_P];
+struct ProposePair {
+    double th[PCS_MAX_P], nrm[PCS_MAX_P], sn[PCS_MAX_P / 2 + 1], cs[PCS_MAX_P / 2 + 1];
+    double lambda, loglam;
     CompArgs ca[PCS_MAX_C];
     PropDev pd;
+    uint32_t parent;
 };
 
-__global__ void __launch_bounds__(32 * kProposeWarps) k_propose(PmcArgs a)
+/* a pair's barriers: 0 both wait; 1 warp 1 waits for warp 0, 2 warp 0 for warp 1 */
+__device__ __forceinline__ void pair_sync_(uint32_t pair, uint32_t which)
 {
-    __shared__ ProposeWarp s_warp[kProposeWarps];
+    __syncwarp();
+    asm volatile("bar.sync %0, 64;\n" ::"r"(1u + 3u * pair + which) : "memory");
+}
+
+__device__ __forceinline__ void pair_arrive_(uint32_t pair, uint32_t which)
+{
+    __syncwarp();
+    __threadfence_block();
+    asm volatile("bar.arrive %0, 64;\n" ::"r"(1u + 3u * pair + which) : "memory");
+}
+
+__global__ void __launch_bounds__(64 * kProposePairs) k_propose(PmcArgs a)
+{
+    __shared__ ProposePair s_pair[kProposePairs];
     RoundDev* rd = a.round;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    if (q >= rd->n_props) return; /* whole warp */
-    ProposeWarp& w = s_warp[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, pair = threadIdx.x >> 6;
+    const bool first = (threadIdx.x & 32u) == 0u; /* warp 0 of the pair */
+    const uint32_t q = pair * gridDim.x + blockIdx.x;
+    if (q >= rd->n_props) return; /* both warps */
+    ProposePair& w = s_pair[pair];
     const uint32_t j = job_of_(rd, q, lane);
     JobPmcDev& pm = a.pmc[j];
     const JobDev& jd = a.jobs[j];
@@ -272,105 +293,135 @@ __global__ void __launch_bounds__(32 * kProposeWarps) k_propose(PmcArgs a)
 
     /* parameters: lane p computes parameter p */
     if (gen == 0u) {
-        if (lane < P) w.th[lane] = pm.theta[(uint64_t)slot * P + lane];
+        if (first && lane < P) w.th[lane] = pm.theta[(uint64_t)slot * P + lane];
     } else {
-        const pcs_u4 r = pcs_draw(0u, pcs_ctr_tag(PCS_STREAM_PICK, 0u), slot, gt, k0, k1);
-        const uint32_t parent = warp_pick_(pm.wcum, pm.N, pcs_u01_53(r.x, r.y), lane);
-        const double* tp = pm.theta + (uint64_t)parent * P;
-        if (2u * lane < P) {
-            const pcs_u4 rr = pcs_draw(lane, pcs_ctr_tag(PCS_STREAM_PERTURB, 0u), slot, gt, k0, k1);
-            pcs_normal2(rr, w.nrm[2u * lane], w.nrm[2u * lane + 1u]);
+        pcs_u4 rr = {0u, 0u, 0u, 0u};
+        if (2u * lane < P) rr = pcs_draw(lane, pcs_ctr_tag(PCS_STREAM_PERTURB, 0u), slot, gt, k0, k1);
+        double rad = 0.0;
+        if (first) {
+            if (2u * lane < P) rad = pcs_normal_radius(rr);
+        } else {
+            const pcs_u4 r = pcs_draw(0u, pcs_ctr_tag(PCS_STREAM_PICK, 0u), slot, gt, k0, k1);
+            const uint32_t parent = warp_pick_(pm.wcum, pm.N, pcs_u01_53(r.x, r.y), lane);
+            if (lane == 0u) w.parent = parent;
+            if (2u * lane < P) pcs_normal_angle(rr, w.sn[lane], w.cs[lane]);
         }
-        __syncwarp();
-        if (lane < P) w.th[lane] = pcs_perturb_one(pm, tp, pm.factor, w.nrm, lane);
-        __syncwarp();
-        if (lane == 0u) pcs_sort_components(pm, w.th);
+        pair_sync_(pair, 0u);
+        if (first) {
+            if (2u * lane < P) {
+                w.nrm[2u * lane] = rad * w.sn[lane];
+                if (2u * lane + 1u < PCS_MAX_P) w.nrm[2u * lane + 1u] = rad * w.cs[lane];
+            }
+            __syncwarp();
+            const double* tp = pm.theta + (uint64_t)w.parent * P;
+            if (lane < P) w.th[lane] = pcs_perturb_one(pm, tp, pm.factor, w.nrm, lane);
+            __syncwarp();
+            if (lane == 0u) pcs_sort_components(pm, w.th);
+        }
     }
-    __syncwarp();
+    pair_sync_(pair, 0u);
 
     /* per-component arguments: lane c computes component c */
-    if (lane < pm.C) w.ca[lane] = pcs_comp_args(pm, w.th, lane);
-    __syncwarp();
-    double lambda = 0.0;
-    if (lane == 0u) {
-        w.pd.job = j;
-        w.pd.slot = slot;
-        w.pd.trial = trial;
-        w.pd.gen = gen;
-        lambda = pcs_assemble_args(pm, w.th, w.ca, gen, w.pd);
-    }
-    lambda = __shfl_sync(0xFFFFFFFFu, lambda, 0);
-    if (lane < P) a.theta_prop[(uint64_t)q * PCS_MAX_P + lane] = w.th[lane];
-
-    PoissonSetup ps = pcs_poisson_setup(lambda);
-    ps.logfact = a.logfact;
-    ps.logfact_n = a.logfact_n;
     const uint64_t coff = (uint64_t)q * (2u * rd->v_max + 1u);
-    uint32_t* cnt = a.counts + coff;
-    uint32_t* pre = cnt + jd.V;
-    uint64_t run = 0, steps = 0;
-    if (lane == 0u) pre[0] = 0u;
-    for (uint32_t v0 = 0; v0 < jd.V; v0 += 32u) {
-        const uint32_t v = v0 + lane;
-        uint32_t c = 0u;
-        if (v < jd.V) {
-            c = pcs_poisson_draw(ps, v, slot, gt, k0, k1);
-            cnt[v] = c;
-            steps += (uint64_t)c * jd.frames[v];
+    if (first) {
+        if (lane < pm.C) w.ca[lane].powc = pcs_comp_power(pm, w.th, lane);
+        __syncwarp();
+        const double lambda = pcs_lambda(pm, w.ca);
+        if (lane == 0u) w.lambda = lambda;
+        pair_arrive_(pair, 1u);
+        if (lane < P) a.theta_prop[(uint64_t)q * PCS_MAX_P + lane] = w.th[lane];
+
+        PoissonSetup ps = pcs_poisson_setup<false>(lambda);
+        ps.logfact = a.logfact;
+        ps.logfact_n = a.logfact_n;
+        pair_sync_(pair, 2u);
+        if (pcs_poisson_takes_log(lambda)) pcs_poisson_set_log(ps, w.loglam);
+        uint32_t* cnt = a.counts + coff;
+        uint32_t* pre = cnt + jd.V;
+        uint64_t run = 0, steps = 0;
+        if (lane == 0u) pre[0] = 0u;
+        for (uint32_t v0 = 0; v0 < jd.V; v0 += 32u) {
+            const uint32_t v = v0 + lane;
+            uint32_t c = 0u;
+            if (v < jd.V) {
+                c = pcs_poisson_draw(ps, v, slot, gt, k0, k1);
+                cnt[v] = c;
+                steps += (uint64_t)c * jd.frames[v];
+            }
+            uint64_t incl = c;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if ((int)lane >= d) incl += t;
+            }
+            const uint64_t tot = run + incl;
+            if (v < jd.V) pre[v + 1] = (uint32_t)(tot < 0xFFFFFFFFull ? tot : 0xFFFFFFFFull);
+            run += __shfl_sync(0xFFFFFFFFu, incl, 31);
         }
-        uint64_t incl = c;
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if ((int)lane >= d) incl += t;
+        for (int d = 16; d >= 1; d >>= 1) steps += __shfl_xor_sync(0xFFFFFFFFu, steps, d);
+        if (lane == 0u) {
+            const uint64_t total = run;
+            if (total > 0xFFFFFFFFull) atomicOr(a.err, PCS_ERRBIT_COUNTS);
+            w.pd.total_particles = (uint32_t)min(total, (uint64_t)0xFFFFFFFFu);
+            w.pd.item_count = (w.pd.total_particles + rd->chunk - 1u) / rd->chunk;
+            w.pd.item_begin = 0u;
+            atomicAdd((unsigned long long*)&pm.particle_steps, (unsigned long long)steps);
+            atomicAdd(&a.round->round_steps, (unsigned long long)steps);
         }
-        const uint64_t tot = run + incl;
-        if (v < jd.V) pre[v + 1] = (uint32_t)(tot < 0xFFFFFFFFull ? tot : 0xFFFFFFFFull);
-        run += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    } else {
+        if (lane < pm.C) pcs_comp_sd(pm, w.th, lane, w.ca[lane]);
+        pair_sync_(pair, 1u); /* the concentrations and the mean */
+        if (lane == 0u && pcs_poisson_takes_log(w.lambda)) w.loglam = log(w.lambda);
+        pair_arrive_(pair, 2u);
+        if (lane == 0u) {
+            const uint64_t rb = (uint64_t)jd.R * jd.B;
+            w.pd.job = j;
+            w.pd.slot = slot;
+            w.pd.trial = trial;
+            w.pd.gen = gen;
+            pcs_assemble_args(pm, w.th, w.ca, gen, w.pd);
+            w.pd.counts_off = coff;
+            w.pd.hist_off = rd->job_hist_base[j] + (uint64_t)local * rb;
+            /* the job's histograms start at a multiple of R x B words (k_round_plan) */
+            w.pd.hist_z = (uint32_t)(w.pd.hist_off / max(1ull, (unsigned long long)rb));
+        }
     }
-    for (int d = 16; d >= 1; d >>= 1) steps += __shfl_xor_sync(0xFFFFFFFFu, steps, d);
-    if (lane == 0u) {
-        const uint64_t total = run, rb = (uint64_t)jd.R * jd.B;
-        if (total > 0xFFFFFFFFull) atomicOr(a.err, PCS_ERRBIT_COUNTS);
-        w.pd.total_particles = (uint32_t)min(total, (uint64_t)0xFFFFFFFFu);
-        w.pd.counts_off = coff;
-        w.pd.hist_off = rd->job_hist_base[j] + (uint64_t)local * rb;
-        /* the job's histograms start at a multiple of R x B words (k_round_plan) */
-        w.pd.hist_z = (uint32_t)(w.pd.hist_off / max(1ull, (unsigned long long)rb));
-        w.pd.item_count = (w.pd.total_particles + rd->chunk - 1u) / rd->chunk;
-        w.pd.item_begin = 0u;
-        atomicAdd((unsigned long long*)&pm.particle_steps, (unsigned long long)steps);
-        atomicAdd(&a.round->round_steps, (unsigned long long)steps);
-    }
-    __syncwarp();
-    for (uint32_t i = lane; i < sizeof(PropDev) / 4u; i += 32u)
-        reinterpret_cast<uint32_t*>(a.props + q)[i] = reinterpret_cast<const uint32_t*>(&w.pd)[i];
+    pair_sync_(pair, 0u);
+    if (first)
+        for (uint32_t i = lane; i < sizeof(PropDev) / 4u; i += 32u)
+            reinterpret_cast<uint32_t*>(a.props + q)[i] = reinterpret_cast<const uint32_t*>(&w.pd)[i];
 }
 
 /* ----------------------------------------------------------------------- */
 /* item scan: one block */
 __global__ void __launch_bounds__(1024) k_items(PmcArgs a)
 {
-    __shared__ uint32_t s_part[1024];
+    __shared__ uint32_t s_part[32]; /* each warp's items */
     RoundDev* rd = a.round;
     const uint32_t M = rd->n_props;
     const uint32_t per = (M + blockDim.x - 1) / blockDim.x;
     const uint32_t b = threadIdx.x * per, e = min(b + per, M);
     uint32_t sum = 0;
     for (uint32_t q = b; q < e; ++q) sum += a.props[q].item_count;
-    s_part[threadIdx.x] = sum;
-    __syncthreads();
-    for (uint32_t d = 1; d < blockDim.x; d <<= 1) {
-        uint32_t t = (threadIdx.x >= d) ? s_part[threadIdx.x - d] : 0u;
-        __syncthreads();
-        s_part[threadIdx.x] += t;
-        __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t incl = sum, part = 0u;
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += t;
     }
-    uint32_t run = s_part[threadIdx.x] - sum;
+    if (lane == 31u) s_part[warp] = incl;
+    __syncthreads();
+    part = lane < nw ? s_part[lane] : 0u; /* every warp scans the warps' */
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, part, d);
+        if (lane >= d) part += t;
+    }
+    const uint32_t before = __shfl_sync(0xFFFFFFFFu, part, warp ? warp - 1u : 0u);
+    uint32_t run = (warp ? before : 0u) + incl - sum;
     for (uint32_t q = b; q < e; ++q) {
         a.props[q].item_begin = run;
         run += a.props[q].item_count;
     }
-    const uint32_t total = s_part[blockDim.x - 1];
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, part, 31);
     const uint32_t cap = rd->items_cap;
     __syncthreads(); /* every proposal's item_begin is written */
     if (threadIdx.x == 0) {
@@ -380,8 +431,7 @@ __global__ void __launch_bounds__(1024) k_items(PmcArgs a)
     }
     /* the item -> proposal map: a warp per proposal, its lanes on
      * consecutive items (coalesced stores) */
-    const uint32_t lane = threadIdx.x & 31u, nw = blockDim.x >> 5;
-    for (uint32_t q = threadIdx.x >> 5; q < M; q += nw) {
+    for (uint32_t q = warp; q < M; q += nw) {
         const uint32_t ib = a.props[q].item_begin, ic = a.props[q].item_count;
         for (uint32_t i = lane; i < ic; i += 32u)
             if (ib + i < cap) a.item_prop[ib + i] = q;
@@ -1174,7 +1224,7 @@ cudaError_t launch_round_plan(const PmcArgs& a, cudaStream_t st)
 
 cudaError_t launch_propose(const PmcArgs& a, uint32_t capacity, cudaStream_t st)
 {
-    k_propose<<<(capacity + kProposeWarps - 1) / kProposeWarps, 32 * kProposeWarps, 0, st>>>(a);
+    k_propose<<<(capacity + kProposePairs - 1) / kProposePairs, 64 * kProposePairs, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -38,19 +38,29 @@ PCS_HD Layout pcs_layout(const JobPmcDev& pm)
     return L;
 }
 
-/* standard normal pair from 4 words (Box-Muller in double) */
-PCS_HD void pcs_normal2(pcs_u4 r, double& n0, double& n1)
+/* standard normal pair from 4 words (Box-Muller in double): radius and angle */
+PCS_HD double pcs_normal_radius(pcs_u4 r)
 {
     const double u1 = 1.0 - pcs_u01_53(r.x, r.y); /* (0, 1] */
+    return sqrt(-2.0 * log(u1));
+}
+
+PCS_HD void pcs_normal_angle(pcs_u4 r, double& s, double& c)
+{
     const double u2 = pcs_u01_53(r.z, r.w);
-    const double rad = sqrt(-2.0 * log(u1));
-    double s, c;
 #if defined(__CUDA_ARCH__)
     sincospi(2.0 * u2, &s, &c);
 #else
     s = sin(2.0 * 3.14159265358979323846 * u2);
     c = cos(2.0 * 3.14159265358979323846 * u2);
 #endif
+}
+
+PCS_HD void pcs_normal2(pcs_u4 r, double& n0, double& n1)
+{
+    const double rad = pcs_normal_radius(r);
+    double s, c;
+    pcs_normal_angle(r, s, c);
     n0 = rad * s;
     n1 = rad * c;
 }
@@ -86,6 +96,17 @@ struct PoissonSetup {
     float lamf, af, bf, vrf, loglamf, linvf; /* the same constants rounded to float (pcs_ptrs_filtered) */
 };
 
+PCS_HD bool pcs_poisson_takes_log(double lam) { return lam >= 12.0; }
+
+/* loglam: log(lam) where pcs_poisson_takes_log, or any value to be set later
+ * (pcs_poisson_set_log) */
+PCS_HD void pcs_poisson_set_log(PoissonSetup& ps, double loglam)
+{
+    ps.loglam = loglam;
+    ps.loglamf = (float)loglam;
+}
+
+template <bool LOG = true>
 PCS_HD PoissonSetup pcs_poisson_setup(double lam)
 {
     PoissonSetup ps;
@@ -100,7 +121,6 @@ PCS_HD PoissonSetup pcs_poisson_setup(double lam)
         return ps;
     }
     const double slam = sqrt(lam);
-    ps.loglam = log(lam);
     ps.b = 0.931 + 2.53 * slam;
     ps.a = -0.059 + 0.02483 * ps.b;
     ps.invalpha = 1.1239 + 1.1328 / (ps.b - 3.4);
@@ -110,7 +130,7 @@ PCS_HD PoissonSetup pcs_poisson_setup(double lam)
     ps.af = (float)ps.a;
     ps.bf = (float)ps.b;
     ps.vrf = (float)ps.vr;
-    ps.loglamf = (float)ps.loglam;
+    if (LOG) pcs_poisson_set_log(ps, log(lam));
     ps.linvf = (float)ps.log_invalpha;
     return ps;
 }
@@ -345,11 +365,14 @@ struct CompArgs {
     float sd_scale, sd_shape;
 };
 
-PCS_HD CompArgs pcs_comp_args(const JobPmcDev& pm, const double* th, uint32_t i)
+PCS_HD double pcs_comp_power(const JobPmcDev& pm, const double* th, uint32_t i)
+{
+    return exp10(th[pcs_layout(pm).c + i]); /* 10^x: one exponential, where pow(10, x) adds a logarithm */
+}
+
+PCS_HD void pcs_comp_sd(const JobPmcDev& pm, const double* th, uint32_t i, CompArgs& ca)
 {
     const Layout L = pcs_layout(pm);
-    CompArgs ca;
-    ca.powc = exp10(th[L.c + i]); /* 10^x: one exponential, where pow(10, x) adds a logarithm */
     if (pm.model == PCS_DEV_MODEL_LOGNORMAL) {
         /* lognormal diameter (nm), mean mu and sd s: sigma_ln^2 = ln(1 + s^2 / mu^2) */
         const double mu = th[L.m + i], sdv = th[L.s + i];
@@ -361,7 +384,22 @@ PCS_HD CompArgs pcs_comp_args(const JobPmcDev& pm, const double* th, uint32_t i)
         ca.sd_scale = (float)sqrt(2.0 * th[L.m + i] * pm.delta_t);
         ca.sd_shape = 0.0f;
     }
+}
+
+PCS_HD CompArgs pcs_comp_args(const JobPmcDev& pm, const double* th, uint32_t i)
+{
+    CompArgs ca;
+    ca.powc = pcs_comp_power(pm, th, i);
+    pcs_comp_sd(pm, th, i, ca);
     return ca;
+}
+
+/* The Poisson mean per video (the components' powers are added in order). */
+PCS_HD double pcs_lambda(const JobPmcDev& pm, const CompArgs* ca)
+{
+    double csum = 0.0;
+    for (uint32_t i = 0; i < pm.C; ++i) csum += ca[i].powc;
+    return csum * pm.volume_factor;
 }
 
 /* Assembles a proposal's forward-model arguments from its components';
