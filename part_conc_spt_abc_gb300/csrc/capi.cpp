@@ -769,7 +769,7 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         d.max_bins = bins;
         d.max_count = d.min_count = count;
         d.tmaps = setup.map;
-        const uint32_t cl = (d_cum || d_d64 || d_ssd) ? 0u : distance_cluster_size(rows, bins);
+        const uint32_t cl = distance_cluster_size(rows, bins);
         PCS_CUDA(launch_distance(d, std::min<uint32_t>(count, (uint32_t)(distance_ctas_per_sm(rows) * c.sm_count)), st, cl));
         if (cum_out) PCS_CUDA(cudaMemcpyAsync(cum_out, d_cum, count * RB * 4, cudaMemcpyDeviceToHost, st));
         const Fetch f32(c, ws, dist_f32, d_d32, (size_t)count * 4);

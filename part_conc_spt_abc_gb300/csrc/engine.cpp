@@ -677,7 +677,7 @@ void Ctx::enqueue_round()
     d.max_count = rb.capacity;
     d.min_count = 1u; /* the round's number is the device's */
     d.tmaps = rb.tmaps.as<TmapDev>();
-    const uint32_t cl = d.dist_f64 ? 0u : distance_cluster_size(rb.max_rows, rb_max_b_);
+    const uint32_t cl = distance_cluster_size(rb.max_rows, rb_max_b_);
     PCS_CUDA(cudaEventRecordWithFlags(ev_dist0, stream, cudaEventRecordExternal));
     PCS_CUDA(launch_distance(d, std::min<uint32_t>(rb.capacity, (uint32_t)(distance_ctas_per_sm(rb.max_rows) * sm_count)),
                              stream, cl));

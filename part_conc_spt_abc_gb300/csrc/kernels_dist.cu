@@ -520,7 +520,11 @@ __device__ __forceinline__ uint64_t square_(uint32_t s, uint32_t o)
  * the current one is computed (two tiles), or, with one tile (tall
  * histograms), as soon as phase B has read it.  A copy wait that runs out ends
  * the loop on every CTA of the cluster together (each reads all CTAs' flags
- * after the barrier), so no CTA is left waiting at a cluster barrier. */
+ * after the barrier), so no CTA is left waiting at a cluster barrier.
+ * With F64 and SSD each CTA also publishes its strip's per-lane double sums
+ * and its warps' exact sums, as the strip kernel forms them, and CTA 0 adds
+ * them likewise; the prefix sums leave with the row carry added.  (16 of 1001
+ * x 256 with all of these: strip by strip 114 us, here 46.) */
 __device__ __forceinline__ void cluster_fill_(const DistArgs& a, uint32_t p, uint32_t k, uint32_t cl, uint32_t* T,
                                               uint32_t tid, uint64_t* mbar)
 {
@@ -529,9 +533,34 @@ __device__ __forceinline__ void cluster_fill_(const DistArgs& a, uint32_t p, uin
     else mbar_arrive_expect_tx_(mbar, 0u);
 }
 
+/* the double at `p` (this CTA's shared memory) in the cluster's CTA `rank` */
+__device__ __forceinline__ double ld_cluster_f64_(const void* p, uint32_t rank)
+{
+    uint32_t ra;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(smem_u32_(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];\n" : "=d"(v) : "r"(ra) : "memory");
+    return v;
+}
+
+/* what a CTA publishes of its strip: per-lane sums, and with SSD each warp's
+ * exact sum of squares */
+struct ClusterSums {
+    float* f;       /* [32][32] */
+    double* d;      /* [32][32] with F64 */
+    uint64_t* sq;   /* [16] (hi, lo) with SSD */
+    /* the one of two that histogram number `it` of the cluster uses */
+    __device__ __forceinline__ ClusterSums of(uint32_t it) const
+    {
+        const uint32_t b = it & 1u;
+        return {f + b * 1024u, d + b * 1024u, sq + b * (kStripThreads / 16u)};
+    }
+};
+
 /* CTA 0: histogram p's distance from every strip's per-lane sums */
-__device__ __forceinline__ void cluster_reduce_(const DistArgs& a, uint32_t p, uint32_t cl, const float* part,
-                                                float* s_tot)
+template <bool F64, bool SSD>
+__device__ __forceinline__ void cluster_reduce_(const DistArgs& a, uint32_t p, uint32_t cl, const ClusterSums& part,
+                                                float* s_tot, double* s_tot64)
 {
     const uint32_t tid = threadIdx.x, w = tid >> 5, l = tid & 31u;
     const uint32_t job = a.props[p].job;
@@ -548,21 +577,54 @@ __device__ __forceinline__ void cluster_reduce_(const DistArgs& a, uint32_t p, u
     for (uint32_t h = 0; h < 2u; ++h) {
         const uint32_t lw = 2u * w + h;
         float acc = 0.0f;
+        double acc64 = 0.0;
         for (uint32_t j = 0; j < ns; ++j)
-            if (32u * j + lw < B) acc = __fadd_rn(acc, __uint_as_float(ld_cluster_(part + lw * 32u + l, j)));
+            if (32u * j + lw < B) {
+                acc = __fadd_rn(acc, __uint_as_float(ld_cluster_(part.f + lw * 32u + l, j)));
+                if (F64) acc64 = __dadd_rn(acc64, ld_cluster_f64_(part.d + lw * 32u + l, j));
+            }
         const float ws = reduce0_(acc);
-        if (l == 0u) s_tot[lw] = ws;
+        const double wd = F64 ? reduce0_(acc64) : 0.0;
+        if (l == 0u) {
+            s_tot[lw] = ws;
+            if (F64) s_tot64[lw] = wd;
+        }
     }
     __syncthreads();
     if (w == 0u) {
         const float fin = reduce0_(s_tot[l]);
-        if (l == 0u) a.dist_f32[p] = fin;
+        const double fin64 = F64 ? reduce0_(s_tot64[l]) : 0.0;
+        uint64_t hi = 0u, lo = 0u;
+        if (SSD) {
+            if (l < kStripThreads / 32u)
+                for (uint32_t j = 0; j < ns; ++j) {
+                    uint64_t v[2];
+#pragma unroll
+                    for (uint32_t i = 0; i < 2u; ++i)
+                        v[i] = (uint64_t)ld_cluster_(part.sq + 2u * l + i, j) |
+                               (uint64_t)ld_cluster_(reinterpret_cast<const uint32_t*>(part.sq + 2u * l + i) + 1, j) << 32;
+                    add128_(hi, lo, v[0], v[1]);
+                }
+            for (uint32_t d = 16; d >= 1; d >>= 1) {
+                const uint64_t ohi = __shfl_down_sync(0xFFFFFFFFu, hi, d), olo = __shfl_down_sync(0xFFFFFFFFu, lo, d);
+                if (l + d < 32u) add128_(hi, lo, ohi, olo);
+            }
+        }
+        if (l == 0u) {
+            a.dist_f32[p] = fin;
+            if (F64 && a.dist_f64) a.dist_f64[p] = fin64;
+            if (SSD && a.ssd) {
+                a.ssd[2 * (uint64_t)p] = hi;
+                a.ssd[2 * (uint64_t)p + 1] = lo;
+            }
+        }
     }
 }
 
+template <bool F64, bool SSD>
 __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, uint32_t cl, uint32_t M,
                                                uint32_t* tiles, uint32_t tile_words, const uint32_t* zero,
-                                               uint32_t* carry, uint32_t* P2, float* part2, float* s_tot,
+                                               uint32_t* carry, uint32_t* P2, const ClusterSums& part2, float* s_tot, double* s_tot64,
                                                uint32_t (*s_col)[32], uint32_t (*s_K)[32], uint64_t* s_mbar,
                                                uint32_t* s_abort)
 {
@@ -586,7 +648,7 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
         const uint32_t pn = p + ncl;
         const bool has_next = pn < M;
         uint32_t* P = P2 + (it & 1u) * prow;
-        float* part = part2 + (it & 1u) * 1024u;
+        const ClusterSums part = part2.of(it);
         cp_async_wait_<0>();
         if (!mbar_wait_(&s_mbar[cur], (parity >> cur) & 1u)) {
             atomicOr(a.err, PCS_ERRBIT_TIMEOUT);
@@ -671,9 +733,14 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                 carry[r] = c;
             }
             __syncthreads();
+            uint32_t* cum = a.cum_out ? a.cum_out + a.props[p].hist_off : nullptr;
+            if (cum && c0 + l < B)
+                for (uint32_t r = w; r < R; r += kStripThreads / 32u) __stcs(cum + (uint64_t)r * B + c0 + l, T[sw_(r, l)] + carry[r]);
             /* phase B as in the strip walk, the row carry added to each cell */
             const uint32_t colA = c0 + 2u * w;
             float a2A = 0.0f, a2B = 0.0f;
+            double a2dA = 0.0, a2dB = 0.0;
+            uint64_t shi = 0u, slo = 0u;
             if (colA < B) {
                 const bool inB = colA + 1u < B;
                 const uint32_t* Tl = T + ((((w >> 1) ^ (l & 7u)) << 2) | ((2u * w) & 3u));
@@ -681,6 +748,7 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                 const uint32_t* refc = refT + (uint64_t)colA * R;
                 const bool exact = T[sw_(R - 1u, 31u)] + carry[R - 1u] < kExactBelow &&
                                    __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
+                uint64_t iA = 0u, iB = 0u;
                 if (exact && inB) {
                     const uint2* ref2 = reinterpret_cast<const uint2*>(refc);
 #pragma unroll 4
@@ -692,11 +760,17 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                         const float dB = exact_diff_(v.y + c, o.y);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
                         a2B = __fadd_rn(a2B, __fmul_rn(dB, dB));
+                        if (F64 || SSD) {
+                            iA += square_(v.x + c, o.x);
+                            iB += square_(v.y + c, o.y);
+                        }
                     }
                 } else if (exact) {
                     for (uint32_t r = l; r < R; r += 32u) {
-                        const float dA = exact_diff_(Tl[r << 5] + carry[r], __ldg(refc + r));
+                        const uint32_t v = Tl[r << 5] + carry[r], o = __ldg(refc + r);
+                        const float dA = exact_diff_(v, o);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
+                        if (F64 || SSD) iA += square_(v, o);
                     }
                 } else {
                     for (uint32_t r = l; r < R; r += 32u) {
@@ -704,19 +778,40 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                         if (inB) {
                             const uint2 v = *reinterpret_cast<const uint2*>(Tl + (r << 5));
                             const uint2 o = __ldg(reinterpret_cast<const uint2*>(refc) + r);
-                            const float dA = __fsub_rn(__uint2float_rn(v.x + c), __uint2float_rn(o.x));
-                            const float dB = __fsub_rn(__uint2float_rn(v.y + c), __uint2float_rn(o.y));
-                            a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
-                            a2B = __fadd_rn(a2B, __fmul_rn(dB, dB));
+                            term_<F64, SSD>(v.x + c, o.x, a2A, a2dA, shi, slo);
+                            term_<F64, SSD>(v.y + c, o.y, a2B, a2dB, shi, slo);
                         } else {
-                            const float dA = __fsub_rn(__uint2float_rn(Tl[r << 5] + c), __uint2float_rn(__ldg(refc + r)));
-                            a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
+                            term_<F64, SSD>(Tl[r << 5] + c, __ldg(refc + r), a2A, a2dA, shi, slo);
                         }
                     }
                 }
+                if (exact) {
+                    if (F64) {
+                        a2dA = (double)iA;
+                        a2dB = (double)iB;
+                    }
+                    if (SSD) {
+                        add128_(shi, slo, 0u, iA);
+                        add128_(shi, slo, 0u, iB);
+                    }
+                }
             }
-            part[(2u * w) * 32u + l] = a2A;
-            part[(2u * w + 1u) * 32u + l] = a2B;
+            part.f[(2u * w) * 32u + l] = a2A;
+            part.f[(2u * w + 1u) * 32u + l] = a2B;
+            if (F64) {
+                part.d[(2u * w) * 32u + l] = a2dA;
+                part.d[(2u * w + 1u) * 32u + l] = a2dB;
+            }
+            if (SSD) {
+                for (uint32_t d = 16; d >= 1; d >>= 1) {
+                    const uint64_t ohi = __shfl_down_sync(0xFFFFFFFFu, shi, d), olo = __shfl_down_sync(0xFFFFFFFFu, slo, d);
+                    if (l + d < 32u) add128_(shi, slo, ohi, olo);
+                }
+                if (l == 0u) {
+                    part.sq[2u * w] = shi;
+                    part.sq[2u * w + 1u] = slo;
+                }
+            }
         }
         /* this tile's generic accesses before its next box fill */
         fence_proxy_async_();
@@ -727,7 +822,7 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
             cp_async_commit_();
         }
         /* CTA 0: the previous histogram, whose sums every CTA published before the barrier */
-        if (k == 0u && it > 0u) cluster_reduce_(a, p_prev, cl, part2 + ((it - 1u) & 1u) * 1024u, s_tot);
+        if (k == 0u && it > 0u) cluster_reduce_<F64, SSD>(a, p_prev, cl, part2.of(it - 1u), s_tot, s_tot64);
         if (!has_next) break;
         if (db) cur ^= 1u;
         p_prev = p;
@@ -735,7 +830,7 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
         ++it;
     }
     cluster_sync_(); /* the last histogram's per-lane sums published */
-    if (!ab && k == 0u) cluster_reduce_(a, p, cl, part2 + (it & 1u) * 1024u, s_tot);
+    if (!ab && k == 0u) cluster_reduce_<F64, SSD>(a, p, cl, part2.of(it), s_tot, s_tot64);
     cluster_sync_(); /* no CTA leaves while CTA 0 reads its sums */
     cp_async_wait_<0>();
     for (uint32_t b = 0; b < 2u; ++b)
@@ -743,7 +838,8 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
     bulk_wait_all_();
 }
 
-/* Cluster mode (float distance only), clusters of cl CTAs. */
+/* Cluster mode, clusters of cl CTAs. */
+template <bool F64, bool SSD>
 __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_t db, uint32_t cl)
 {
     extern __shared__ __align__(16) uint32_t s_mem[];
@@ -751,13 +847,17 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
     if (cluster_id_() >= M) return; /* whole clusters return */
     const uint32_t prow = strip_cap_rows(a.max_rows), tile_words = prow * 32u;
     /* [1 + db][cap rows][32] tiles (1024-byte aligned), a zero box, the row
-     * carries, two last-column arrays, two 32 x 32 per-lane sum arrays */
+     * carries, two last-column arrays, two 32 x 32 per-lane sum arrays, with
+     * F64 two of doubles */
     uint32_t* tiles = s_mem + ((1024u - (smem_u32_(s_mem) & 1023u)) & 1023u) / 4u;
     uint32_t* zero = tiles + (1u + db) * tile_words;
     uint32_t* carry = zero + kBox * kBox;
     uint32_t* P2 = carry + prow;
-    float* part2 = reinterpret_cast<float*>(P2 + 2u * prow);
+    float* f2 = reinterpret_cast<float*>(P2 + 2u * prow);
+    double* d2 = reinterpret_cast<double*>(f2 + 2u * 1024u);
     __shared__ float s_tot[32];
+    __shared__ double s_tot64[32];
+    __shared__ uint64_t s_sq[2u * (kStripThreads / 16u)];
     __shared__ uint32_t s_col[16][32];
     __shared__ __align__(16) uint32_t s_K[16][32];
     __shared__ __align__(8) uint64_t s_mbar[2];
@@ -772,7 +872,9 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
     for (uint32_t i = tid; i < kBox * kBox; i += kStripThreads) zero[i] = 0u;
     fence_proxy_async_(); /* the zero box, before box stores read it */
     __syncthreads();
-    strip_cluster_(a, db, cl, M, tiles, tile_words, zero, carry, P2, part2, s_tot, s_col, s_K, s_mbar, &s_abort);
+    const ClusterSums part2 = {f2, d2, s_sq};
+    strip_cluster_<F64, SSD>(a, db, cl, M, tiles, tile_words, zero, carry, P2, part2, s_tot, s_tot64, s_col, s_K, s_mbar,
+                             &s_abort);
 }
 
 /* Row kernel: a CTA takes one histogram at a time, a warp 128 of its columns
@@ -1467,12 +1569,12 @@ static const size_t kStripSmemMax = 220u * 1024u;
 
 /* 1024 bytes to align the tiles, one or two tiles, the zero box, the row
  * carries; for cluster launches two of each strip's last column and of its
- * 32 x 32 per-lane sums */
-static size_t strip_smem_bytes(uint32_t max_rows, bool db, uint32_t cl)
+ * 32 x 32 per-lane sums (with F64 also double ones) */
+static size_t strip_smem_bytes(uint32_t max_rows, bool db, uint32_t cl, bool f64 = false)
 {
     const size_t rows = strip_cap_rows(max_rows);
     size_t n = 1024u + (db ? 2u : 1u) * rows * 32u * sizeof(uint32_t) + kBoxBytes + rows * sizeof(uint32_t);
-    if (cl > 1u) n += 2u * (rows * sizeof(uint32_t) + 32u * 32u * sizeof(float));
+    if (cl > 1u) n += 2u * (rows * sizeof(uint32_t) + 32u * 32u * (sizeof(float) + (f64 ? sizeof(double) : 0u)));
     return n;
 }
 
@@ -1499,10 +1601,10 @@ int distance_ctas_per_sm(uint32_t max_rows, uint32_t cl)
     const size_t smem = distance_smem_bytes(max_rows, cl);
     int n = 0;
     if (use_strip(max_rows, cl)) {
-        allow_smem(k_distance_strip<false, false>);
+        allow_smem(k_distance_strip<false, false>, kStripSmemMax);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance_strip<false, false>, (int)kStripThreads, smem);
     } else {
-        allow_smem(k_distance<false>);
+        allow_smem(k_distance<false>, kDynSmemMax + 256u);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance<false>, 1024, smem);
     }
     return n > 0 ? n : 1;
@@ -1510,15 +1612,16 @@ int distance_ctas_per_sm(uint32_t max_rows, uint32_t cl)
 
 /* Clusters of cl CTAs of k_distance_cluster that fit at once with `smem`
  * bytes of shared memory each, on the current device; queried once per
- * (device, cl, smem), since the plain form launches per proposal. */
-static cudaError_t cluster_fit_(cudaLaunchConfig_t& cfg, uint32_t cl, size_t smem, int& fit)
+ * (device, kernel, cl, smem), since the plain form launches per proposal. */
+static cudaError_t cluster_fit_(void (*k)(DistArgs, uint32_t, uint32_t), cudaLaunchConfig_t& cfg, uint32_t cl, size_t smem,
+                                int& fit)
 {
     static std::mutex mu;
-    static std::map<std::tuple<int, uint32_t, size_t>, int> cache;
+    static std::map<std::tuple<int, const void*, uint32_t, size_t>, int> cache;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    const auto key = std::make_tuple(dev, cl, smem);
+    const auto key = std::make_tuple(dev, (const void*)k, cl, smem);
     {
         std::lock_guard<std::mutex> g(mu);
         const auto it = cache.find(key);
@@ -1527,7 +1630,7 @@ static cudaError_t cluster_fit_(cudaLaunchConfig_t& cfg, uint32_t cl, size_t sme
             return cudaSuccess;
         }
     }
-    e = cudaOccupancyMaxActiveClusters(&fit, (void*)k_distance_cluster, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&fit, (const void*)k, &cfg);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> g(mu);
     cache[key] = fit;
@@ -1610,7 +1713,7 @@ static const size_t kSmemPerSm = 228u * 1024u; /* of which 1 KB per resident CTA
  * (x 120) 115 -> 104, at 21 (x 304) 281 -> 131; 16 turns (301 x 128 x 1024)
  * 89.6 -> 51.1.
  * With double sums the walk zeroes in a second pass and a launch for the
- * histograms left over follows: 8 turns (1001 x 256 x 152) 116 -> 138, 16
+ * histograms left over follows: 8 turns (1001 x 256 x 152) 114 -> 138, 16
  * (x 304) 228 -> 166, 32 (201 x 1000 x 20) 126 -> 63.
  * Where rows are not 16-byte aligned the lanes copy cell by cell: 8 turns
  * (201 x 255 x 100) 39.4 -> 43, 10 (51 x 31 x 3000) 44.6 -> 57, 12 (201 x 99
@@ -1632,7 +1735,7 @@ static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st
     void (*k)(DistArgs);
     if (a.dist_f64) k = a.ssd ? k_distance_rows<true, true> : k_distance_rows<true, false>;
     else k = a.ssd ? k_distance_rows<false, true> : k_distance_rows<false, false>;
-    const cudaError_t e = allow_smem(k);
+    const cudaError_t e = allow_smem(k, kRowsWarps * kRowsWarpBytes);
     if (e != cudaSuccess) return e;
     const uint32_t warps = (a.max_bins + 127u) / 128u;
     const size_t smem = (size_t)warps * kRowsWarpBytes;
@@ -1648,59 +1751,71 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
     if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (e0 != cudaSuccess) return e0;
     const uint32_t sms = (uint32_t)n_sm, strips = (a.max_bins + 31u) / 32u;
-    if (cl > 1u && (a.dist_f64 || a.ssd || a.cum_out || !use_strip(a.max_rows, cl) || cl > kMaxDistCluster)) cl = 0u;
+    const size_t smem = distance_smem_bytes(a.max_rows, 0u);
+    if (smem > 227u * 1024u) return cudaErrorInvalidValue;
+    const uint32_t count = std::max(1u, a.min_count);
+    const uint32_t slots = sms * (use_strip(a.max_rows, 0u) && 2u * (smem + 4096u) <= kSmemPerSm ? 2u : 1u);
+    uint32_t turns = strips * ((count + slots - 1u) / slots);
+
+    const bool f64 = a.dist_f64 != nullptr;
+    const size_t csmem1 = strip_smem_bytes(a.max_rows, false, cl, f64), csmem2 = strip_smem_bytes(a.max_rows, true, cl, f64);
+    if (cl > kMaxDistCluster || csmem1 > kStripSmemMax) cl = 0u;
+    const bool two = csmem2 <= kStripSmemMax;
+    void (*kcl)(DistArgs, uint32_t, uint32_t);
+    if (f64) kcl = a.ssd ? k_distance_cluster<true, true> : k_distance_cluster<true, false>;
+    else kcl = a.ssd ? k_distance_cluster<false, true> : k_distance_cluster<false, false>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    int fit = 0; /* clusters that fit at once */
     if (cl > 1u) {
-        /* clusters of cl CTAs where the histograms are tall, or where every
-         * histogram of the launch has a cluster to itself; as many clusters
-         * as fit at once, at most one per histogram slot */
-        const size_t smem = distance_smem_bytes(a.max_rows, cl);
-        cudaError_t e = allow_smem(k_distance_cluster);
+        const cudaError_t e = allow_smem(kcl, kStripSmemMax);
         if (e != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = cl;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.blockDim = dim3(kStripThreads);
-        cfg.dynamicSmemBytes = smem;
+        cfg.dynamicSmemBytes = two ? csmem2 : csmem1;
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cfg.gridDim = dim3(cl);
-        int fit = 0;
-        e = cluster_fit_(cfg, cl, smem, fit);
-        if (e != cudaSuccess) return e;
-        if (fit > 0 && (strip_cap_rows(a.max_rows) >= kClusterRowsMin || grid <= (uint32_t)fit)) {
-            if (use_rows_(a, (a.min_count + (uint32_t)fit - 1u) / (uint32_t)fit)) return launch_rows_(a, sms, st);
-            cfg.gridDim = dim3(std::min<uint32_t>(grid, (uint32_t)fit) * cl);
-            return cudaLaunchKernelEx(&cfg, k_distance_cluster, a, strip_db(a.max_rows, cl) ? 1u : 0u, cl);
-        }
-        cl = 0u;
+        const cudaError_t f = cluster_fit_(kcl, cfg, cl, cfg.dynamicSmemBytes, fit);
+        if (f != cudaSuccess) return f;
     }
-    const size_t smem = distance_smem_bytes(a.max_rows, 0u);
-    if (smem > 227u * 1024u) return cudaErrorInvalidValue;
-    const uint32_t slots = sms * (use_strip(a.max_rows, 0u) && 2u * (smem + 4096u) <= kSmemPerSm ? 2u : 1u);
-    const bool rows = use_rows_(a, strips * ((std::max(1u, a.min_count) + slots - 1u) / slots));
+    /* clusters of cl CTAs where the histograms are tall, or where every
+     * histogram of the launch has a cluster to itself, if that takes fewer
+     * turns than strips by single CTAs do (a turn is a strip's time either
+     * way: 152 of 1001 x 256 with double sums 178 us in 11 turns of clusters,
+     * 114 in 8 of strips; 152 of 601 x 128 34 in 4 of strips, 120 of them 41 in
+     * 4 of clusters); as many clusters as fit at once, at most one per
+     * histogram slot */
+    const uint32_t cturns = fit > 0 ? (count + (uint32_t)fit - 1u) / (uint32_t)fit : 0u;
+    const bool clusters = fit > 0 && (strip_cap_rows(a.max_rows) >= kClusterRowsMin || grid <= (uint32_t)fit) && cturns < turns;
+    if (clusters) turns = cturns;
+    const bool rows = use_rows_(a, turns);
     if (rows) {
         const cudaError_t e = launch_rows_(a, sms, st);
-        if (e != cudaSuccess || !a.dist_f64) return e;
+        if (e != cudaSuccess || !f64) return e;
+    } else if (clusters) {
+        cfg.gridDim = dim3(std::min<uint32_t>(grid, (uint32_t)fit) * cl);
+        return cudaLaunchKernelEx(&cfg, kcl, a, two ? 1u : 0u, cl);
     }
     if (use_strip(a.max_rows, 0u)) {
         void (*k)(DistArgs, uint32_t, uint32_t);
         if (a.dist_f64) k = a.ssd ? k_distance_strip<true, true> : k_distance_strip<true, false>;
         else k = a.ssd ? k_distance_strip<false, true> : k_distance_strip<false, false>;
-        cudaError_t e = allow_smem(k);
+        cudaError_t e = allow_smem(k, kStripSmemMax);
         if (e != cudaSuccess) return e;
         k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u, rows ? 1u : 0u);
         return cudaGetLastError();
     }
     if (a.dist_f64) {
-        cudaError_t e = allow_smem(k_distance<true>);
+        cudaError_t e = allow_smem(k_distance<true>, kDynSmemMax);
         if (e != cudaSuccess) return e;
         k_distance<true><<<grid, 1024, smem, st>>>(a, rows ? 1u : 0u);
     } else {
-        cudaError_t e = allow_smem(k_distance<false>);
+        cudaError_t e = allow_smem(k_distance<false>, kDynSmemMax + 256u);
         if (e != cudaSuccess) return e;
         k_distance<false><<<grid, 1024, smem, st>>>(a, 0u);
     }

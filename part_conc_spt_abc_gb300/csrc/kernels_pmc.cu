@@ -13,7 +13,7 @@
  *
  *   k_round_plan   shares the round's proposal capacity among the jobs
  *                  (trials per pending slot k = capacity / pending, clamped)
- *   k_propose      one warp per proposal: parent pick, perturbation,
+ *   k_propose      two warps per proposal: parent pick, perturbation,
  *                  label sort, per-proposal forward-model arguments, Poisson
  *                  counts per video (transformed rejection, Hoermann 1993)
  *   k_items        scan of work items and the item -> proposal map

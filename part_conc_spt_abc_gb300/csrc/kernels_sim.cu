@@ -1294,7 +1294,7 @@ template <int PPT, bool REPLAY, bool AGG>
 cudaError_t launch_sim_(const SimArgs& a, uint32_t grid, uint32_t block, size_t smem, cudaStream_t st)
 {
     auto fn = k_simulate<PPT, REPLAY, AGG>;
-    cudaError_t e = allow_smem(fn);
+    cudaError_t e = allow_smem(fn, kDynSmemMax);
     if (e != cudaSuccess) return e;
     fn<<<grid, block, smem, st>>>(a);
     return cudaGetLastError();
@@ -1305,7 +1305,7 @@ int occupancy_(uint32_t block, size_t smem)
 {
     int n = 0;
     auto fn = k_simulate<PPT, REPLAY, AGG>;
-    allow_smem(fn);
+    allow_smem(fn, kDynSmemMax);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)block, smem) != cudaSuccess) return 0;
     return n;
 }
@@ -1322,7 +1322,7 @@ template <bool AGG>
 cudaError_t launch_split_(const SimArgs& a, uint32_t grid, size_t smem, cudaStream_t st)
 {
     auto fn = k_simulate_split<AGG>;
-    cudaError_t e = allow_smem(fn);
+    cudaError_t e = allow_smem(fn, kDynSmemMax);
     if (e != cudaSuccess) return e;
     fn<<<grid, kSplitThreads, smem, st>>>(a);
     return cudaGetLastError();
@@ -1333,7 +1333,7 @@ int occupancy_split_(size_t smem)
 {
     int n = 0;
     auto fn = k_simulate_split<AGG>;
-    allow_smem(fn);
+    allow_smem(fn, kDynSmemMax);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)kSplitThreads, smem) != cudaSuccess) return 0;
     return n;
 }
@@ -1371,7 +1371,7 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
     if (walk_launch_(l, a.tile_words)) {
         const auto fn = walk_kernel_(l.block);
         const size_t tracks = walk_smem_(l.block);
-        const cudaError_t e = allow_smem(fn);
+        const cudaError_t e = allow_smem(fn, walk_smem_(1024u));
         if (e != cudaSuccess) return e;
         fn<<<l.grid, l.block, tracks, st>>>(a);
         return cudaGetLastError();
@@ -1410,7 +1410,7 @@ int simulate_occupancy(const SimLaunch& l, uint32_t tile_words)
         int n = 0;
         const auto fn = walk_kernel_(l.block);
         const size_t tracks = walk_smem_(l.block);
-        allow_smem(fn);
+        allow_smem(fn, walk_smem_(1024u));
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)l.block, tracks) == cudaSuccess ? n : 0;
     }
     const size_t smem = (size_t)tile_words * 4u;

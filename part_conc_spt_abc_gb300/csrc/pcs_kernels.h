@@ -46,7 +46,7 @@ struct SimLaunch {
     bool replay;
     bool aggregate;
     bool split; /* slab-split walk (k_simulate_split: 256 threads, 1 particle each, no replay) */
-    uint32_t few_items; /* the number of items of kFewChunk particles where simulate_few says so, else 0 */
+    uint32_t few_items = 0u; /* the number of items of kFewChunk particles where simulate_few says so, else 0 */
 };
 
 cudaError_t launch_simulate(const SimArgs& a, const SimLaunch& l, cudaStream_t st);
@@ -60,17 +60,16 @@ cudaError_t launch_debug_stream(uint64_t seed, uint32_t slot, uint32_t gen, uint
                                 uint32_t particle, uint32_t block, uint32_t* d_out,
                                 cudaStream_t st);
 
-/* Dynamic shared memory for a kernel, as much as a CTA may have.  The limit
- * belongs to the kernel and not to the launch: set to each launch's own size,
- * threads launching different sizes would lower it under one another. */
+/* Dynamic shared memory for a kernel: `most` is the most that any launch of it
+ * asks for.  The limit belongs to the kernel and not to the launch: set to each
+ * launch's own size, threads launching different sizes would lower it under
+ * one another. */
 template <typename F>
-inline cudaError_t allow_smem(F* fn)
+inline cudaError_t allow_smem(F* fn, size_t most)
 {
-    cudaFuncAttributes fa;
-    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227u * 1024u - fa.sharedSizeBytes));
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
+constexpr size_t kDynSmemMax = 227u * 1024u - 896u; /* of a CTA's 227 KB, for kernels with up to 896 bytes besides */
 
 /* ---------------- scan + distance (kernels_dist.cu) ---------------- */
 struct DistArgs {
