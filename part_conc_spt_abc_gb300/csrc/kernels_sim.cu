@@ -491,15 +491,18 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
  * interval is narrowed by it on both sides.
  *
  * Screened and full walks go to full warps through a queue per CTA (entries
- * (proposal, particle), guarded by a lock that is held for ~100 cycles once
- * per 32-particle walk): a warp takes 32 candidates to screen if there are
- * as many, else 32 full walks, else a new slice, whose particles it sorts
- * into the queue.  What is left in the queue at the end is walked in full.
+ * (proposal, particle), guarded by a lock that is held for ~100 cycles): a
+ * warp takes 32 candidates to screen if there are as many, else 32 full
+ * walks, else a new slice, whose particles it sorts into the queue -- or
+ * walks at once where none is a candidate.  What is left in the queue at the
+ * end is walked in full.  The lock is taken only to add or where there is
+ * something to take (short videos of 31 frames, which are never sorted, lost
+ * 5% to it; configuration 0's rounds 2%).
  *
  * Measured (forward model alone, before -> after): 1e10 particle-steps of
- * configuration 3 in one proposal 28.1 -> 22.4 ms; configuration 1, prior
- * pass and three generations (5.6e10 particle-steps) 158 -> 122 ms;
- * configuration 0, a whole job's 66 short rounds 24.7 -> 20.9 ms.  The bound
+ * configuration 3 in one proposal 28.1 -> 21.5 ms; configuration 1, prior
+ * pass and three generations (5.6e10 particle-steps) 158 -> 120 ms;
+ * configuration 0, a whole job's 66 short rounds 24.7 -> 20.3 ms.  The bound
  * is the FMA-heavy pipe, where a Philox round's 32 x 32 -> 64 bit product
  * takes four cycles: 52 products a group, 208 of the ~440 cycles per warp
  * and group of a full walk and of the ~290 of a screen walk. */
@@ -596,6 +599,16 @@ __device__ __forceinline__ Visit queue_visit_(ScreenQueue& s, uint2& e, uint32_t
     }
     __syncwarp();
     return v;
+}
+
+/* Whether a visit adds or may take something: a look without the lock.  (A
+ * count that another warp raises just after is that warp's to see: it visits
+ * after every push.) */
+__device__ __forceinline__ bool queue_worth_(const ScreenQueue& s, uint32_t push, bool sorting)
+{
+    const volatile ScreenQueue& q = s;
+    const uint32_t from = sorting ? 32u : 1u;
+    return __any_sync(0xFFFFFFFFu, push != 0u || q.nc >= from || q.nf >= from);
 }
 
 /* Tracks closed by a warp's walks, kept until 32 of them can be binned at
@@ -840,7 +853,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK <= 256u ? 3 : 1) k_simulate_walk(
     for (;;) {
         __syncwarp();
         Visit v = kVisitNone;
-        if (screening) v = queue_visit_(s_queue, e, push, sorting, a.err);
+        if (screening && queue_worth_(s_queue, push, sorting)) v = queue_visit_(s_queue, e, push, sorting, a.err);
         push = 0u;
         if (v == kVisitAbort) break;
         if (v == kVisitNone) {
@@ -881,10 +894,15 @@ __global__ void __launch_bounds__(BLOCK, BLOCK <= 256u ? 3 : 1) k_simulate_walk(
         }
         __syncwarp();
         if (v == kVisitSort) {
-            if (e.x != 0xFFFFFFFFu) push = screen_wanted_(q, c) ? 1u : 2u;
-        } else if (v == kVisitScreen) {
+            const bool screen = e.x != 0xFFFFFFFFu && screen_wanted_(q, c);
+            if (__any_sync(0xFFFFFFFFu, screen))
+                push = screen ? 1u : (e.x != 0xFFFFFFFFu ? 2u : 0u);
+            else
+                v = kVisitFull; /* a short video's, or all too near: at once, as they were started */
+        }
+        if (v == kVisitScreen) {
             if (!screen_walk_(q, c)) push = 2u;
-        } else {
+        } else if (v == kVisitFull) {
             walk_warp_(a, c, tracks, n_tracks, q, e.x);
         }
     }
