@@ -1266,16 +1266,17 @@ __global__ void __launch_bounds__(32 * kRowsWarps) k_distance_rows(DistArgs a)
 }
 
 /* the first histogram from p on in this CTA's sequence that is the strip
- * kernel's: all of them, or (redo) those that the row kernel left */
-__device__ __forceinline__ uint32_t strip_next_(const DistArgs& a, uint32_t p, uint32_t M, uint32_t redo)
+ * kernel's: all of them, or (REDO) those that the row kernel left */
+template <bool REDO>
+__device__ __forceinline__ uint32_t strip_next_(const DistArgs& a, uint32_t p, uint32_t M)
 {
-    if (redo)
+    if (REDO)
         while (p < M && __float_as_uint(a.dist_f32[p]) != kRedo) p += gridDim.x;
     return p;
 }
 
-template <bool F64, bool SSD>
-__global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t db, uint32_t redo)
+template <bool F64, bool SSD, bool REDO>
+__global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t db)
 {
     extern __shared__ __align__(16) uint32_t s_mem[];
     const uint32_t tile_words = strip_cap_rows(a.max_rows) * 32u;
@@ -1295,7 +1296,7 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
     const uint32_t tid = threadIdx.x;
     const uint32_t w = tid >> 5, l = tid & 31u;
     const uint32_t M = *a.n_props;
-    uint32_t p = strip_next_(a, blockIdx.x, M, redo);
+    uint32_t p = strip_next_<REDO>(a, blockIdx.x, M);
     if (p >= M) return;
     if (tid == 0) {
         mbar_init_(&s_mbar[0], kStripThreads);
@@ -1323,7 +1324,7 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
         /* the (proposal, strip) after this one */
         uint32_t pn = p, cn = c0 + 32u;
         if (!ok || cn >= B) {
-            pn = strip_next_(a, p + gridDim.x, M, redo);
+            pn = strip_next_<REDO>(a, p + gridDim.x, M);
             cn = 0u;
         }
         const bool has_next = pn < M;
@@ -1596,18 +1597,14 @@ size_t distance_smem_bytes(uint32_t max_rows, uint32_t cl)
 
 uint32_t distance_block_threads(uint32_t max_rows) { return use_strip(max_rows, 0u) ? kStripThreads : 1024u; }
 
+static const size_t kSmemPerSm = 228u * 1024u; /* of which 1 KB per resident CTA is not the CTA's */
+
+/* From the launch bounds and shared memory: two strip CTAs where both fit
+ * (5.25 KB each besides the dynamic part), one of the others.  (Asking the
+ * driver took 3 us of a 50 us call, between its two launches.) */
 int distance_ctas_per_sm(uint32_t max_rows, uint32_t cl)
 {
-    const size_t smem = distance_smem_bytes(max_rows, cl);
-    int n = 0;
-    if (use_strip(max_rows, cl)) {
-        allow_smem(k_distance_strip<false, false>, kStripSmemMax);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance_strip<false, false>, (int)kStripThreads, smem);
-    } else {
-        allow_smem(k_distance<false>, kDynSmemMax + 256u);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_distance<false>, 1024, smem);
-    }
-    return n > 0 ? n : 1;
+    return use_strip(max_rows, cl) && 2u * (distance_smem_bytes(max_rows, cl) + 5376u) <= kSmemPerSm ? 2 : 1;
 }
 
 /* Clusters of cl CTAs of k_distance_cluster that fit at once with `smem`
@@ -1640,33 +1637,40 @@ static cudaError_t cluster_fit_(void (*k)(DistArgs, uint32_t, uint32_t), cudaLau
 /* Device-side set-up of a standalone distance launch: the descriptors of
  * `count` consecutive histograms sharing one job, and the observed
  * histogram's column-major copy (pairs of columns interleaved,
- * pcs_sat_t_index) through tiles of 32 rows x 64 columns in shared memory,
- * read in 256-byte rows and written in 256-byte runs of a pair (done cell by
- * cell on the host it took 0.4 ms for 1001 x 256). */
+ * pcs_sat_t_index) through tiles of 16 rows x 32 columns in shared memory,
+ * read in 128-byte rows and written in 128-byte runs of a pair (done cell by
+ * cell on the host it took 0.4 ms for 1001 x 256).  Two cells per thread, and
+ * the job and its map by a block of their own: a launch of few cells is a
+ * chain of latencies (tiles of 32 x 64 took 5.5 us, a cell per thread written
+ * one by one 3.8). */
 constexpr uint32_t kPropWords = sizeof(PropDev) / 4u;
 
 __global__ void __launch_bounds__(256) k_distance_setup(DistSetup d, const __grid_constant__ TmapDev map)
 {
-    __shared__ uint32_t s_t[32][65];
-    const uint32_t tid = threadIdx.x;
+    __shared__ uint32_t s_t[16][33];
+    const uint32_t tid = threadIdx.x, blocks = gridDim.x - 1u;
     const uint32_t R = d.rows, B = d.bins;
-    if (blockIdx.x == 0u && tid == 0u) {
-        JobDev j;
-        memset(&j, 0, sizeof j);
-        j.R = R;
-        j.B = B;
-        j.ref_sat = d.ref;
-        j.ref_sat_t = d.ref_t;
-        j.tmap_depth = d.map_depth;
-        *d.job = j;
-        *d.map = map;
-        /* the map, for the tensor copies of the kernel that follows (which acquires it) */
-        asm volatile("fence.proxy.tensormap::generic.release.gpu;\n" ::: "memory");
-        *d.n_props = d.count;
-        if (d.err) *d.err = 0u;
+    if (blockIdx.x == blocks) { /* the last block */
+        if (tid == 0u) {
+            JobDev j;
+            memset(&j, 0, sizeof j);
+            j.R = R;
+            j.B = B;
+            j.ref_sat = d.ref;
+            j.ref_sat_t = d.ref_t;
+            j.tmap_depth = d.map_depth;
+            *d.job = j;
+            *d.n_props = d.count;
+            if (d.err) *d.err = 0u;
+        } else if (tid == 32u && d.map_depth) {
+            *d.map = map;
+            /* the map, for the tensor copies of the kernel that follows (which acquires it) */
+            asm volatile("fence.proxy.tensormap::generic.release.gpu;\n" ::: "memory");
+        }
+        return;
     }
     /* the histograms' descriptors, word by word across the threads */
-    for (uint64_t i = (uint64_t)blockIdx.x * 256u + tid; i < (uint64_t)d.count * kPropWords; i += (uint64_t)gridDim.x * 256u) {
+    for (uint64_t i = (uint64_t)blockIdx.x * 256u + tid; i < (uint64_t)d.count * kPropWords; i += (uint64_t)blocks * 256u) {
         const uint32_t q = (uint32_t)(i / kPropWords), k = (uint32_t)(i % kPropWords);
         const uint64_t off = (uint64_t)q * R * B;
         uint32_t v = 0u;
@@ -1675,16 +1679,18 @@ __global__ void __launch_bounds__(256) k_distance_setup(DistSetup d, const __gri
         if (k == offsetof(PropDev, hist_off) / 4u + 1u) v = (uint32_t)(off >> 32);
         reinterpret_cast<uint32_t*>(d.props)[i] = v;
     }
-    const uint32_t tc = (B + 63u) / 64u, tr = (R + 31u) / 32u;
-    for (uint64_t t = blockIdx.x; t < (uint64_t)tc * tr; t += gridDim.x) {
-        const uint32_t r0 = (uint32_t)(t / tc) * 32u, c0 = (uint32_t)(t % tc) * 64u;
-        for (uint32_t i = tid; i < 2048u; i += 256u) {
-            const uint32_t r = r0 + i / 64u, c = c0 + i % 64u;
-            if (r < R && c < B) s_t[i / 64u][i % 64u] = d.ref[(uint64_t)r * B + c];
+    const uint32_t tc = (B + 31u) / 32u, tr = (R + 15u) / 16u;
+    for (uint64_t t = blockIdx.x; t < (uint64_t)tc * tr; t += blocks) {
+        const uint32_t r0 = (uint32_t)(t / tc) * 16u, c0 = (uint32_t)(t % tc) * 32u;
+#pragma unroll
+        for (uint32_t i = tid; i < 512u; i += 256u) {
+            const uint32_t r = r0 + i / 32u, c = c0 + i % 32u;
+            if (r < R && c < B) s_t[i / 32u][i % 32u] = d.ref[(uint64_t)r * B + c];
         }
         __syncthreads();
-        for (uint32_t i = tid; i < 2048u; i += 256u) {
-            const uint32_t k = i % 64u, x = 2u * (i / 64u) + (k & 1u);
+#pragma unroll
+        for (uint32_t i = tid; i < 512u; i += 256u) {
+            const uint32_t k = i % 32u, x = 2u * (i / 32u) + (k & 1u);
             const uint32_t r = r0 + k / 2u, c = c0 + x;
             if (r < R && c < B) d.ref_t[pcs_sat_t_index(r, c, R, B)] = s_t[k / 2u][x];
         }
@@ -1694,13 +1700,11 @@ __global__ void __launch_bounds__(256) k_distance_setup(DistSetup d, const __gri
 
 cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaStream_t st)
 {
-    const uint64_t tiles = (uint64_t)((d.bins + 63u) / 64u) * ((d.rows + 31u) / 32u);
+    const uint64_t tiles = (uint64_t)((d.bins + 31u) / 32u) * ((d.rows + 15u) / 16u);
     const uint64_t blocks = std::max<uint64_t>(tiles, ((uint64_t)d.count * kPropWords + 1023u) / 1024u);
-    k_distance_setup<<<(unsigned)std::min<uint64_t>(blocks, 4096u), 256, 0, st>>>(d, map);
+    k_distance_setup<<<(unsigned)std::min<uint64_t>(blocks, 4096u) + 1u, 256, 0, st>>>(d, map);
     return cudaGetLastError();
 }
-
-static const size_t kSmemPerSm = 228u * 1024u; /* of which 1 KB per resident CTA is not the CTA's */
 
 /* Rows or strips.  The row kernel takes one walk down the rows (10 us + 90 ns
  * per row) for any number of columns and histograms until its warps fill the
@@ -1716,8 +1720,9 @@ static const size_t kSmemPerSm = 228u * 1024u; /* of which 1 KB per resident CTA
  * histograms left over follows: 8 turns (1001 x 256 x 152) 114 -> 138, 16
  * (x 304) 228 -> 166, 32 (201 x 1000 x 20) 126 -> 63.
  * Where rows are not 16-byte aligned the lanes copy cell by cell: 8 turns
- * (201 x 255 x 100) 39.4 -> 43, 10 (51 x 31 x 3000) 44.6 -> 57, 12 (201 x 99
- * x 912) 75.9 -> 57.8, 32 (201 x 999 x 38) 145 -> 90.
+ * (201 x 255 x 100) 39.4 -> 43, 12 (201 x 99 x 912) 75.9 -> 57.8, 32 (201 x
+ * 999 x 38) 145 -> 90; and a warp has to replace three strips: with one (51 x
+ * 31 x 3000) 44.6 -> 57, with two (329 x 49 x 2036, whole calls) 203 -> 235.
  * Histograms too tall for a strip in shared memory (above 1664 rows), whose
  * kernel works through blocks of rows: 2 turns (1800 x 40 x 2) 154 -> 157,
  * 4 (x 200) 836 -> 146, 16 (1800 x 256 x 200) 5409 -> 195. */
@@ -1726,7 +1731,9 @@ static bool use_rows_(const DistArgs& a, uint32_t turns)
     uint32_t from = 8u;
     if (a.dist_f64) from += 4u;
     if (a.max_bins & 3u) from += 4u;
-    if (!use_strip(a.max_rows, 0u)) from = 3u;
+    const bool strips = use_strip(a.max_rows, 0u);
+    if (!strips) from = 3u;
+    if (strips && (a.max_bins & 3u) != 0u && (a.max_bins + 31u) / 32u < 3u * ((a.max_bins + 127u) / 128u)) return false;
     return a.max_bins <= 128u * kRowsWarps && turns >= from;
 }
 
@@ -1754,12 +1761,14 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
     const size_t smem = distance_smem_bytes(a.max_rows, 0u);
     if (smem > 227u * 1024u) return cudaErrorInvalidValue;
     const uint32_t count = std::max(1u, a.min_count);
-    const uint32_t slots = sms * (use_strip(a.max_rows, 0u) && 2u * (smem + 4096u) <= kSmemPerSm ? 2u : 1u);
+    const uint32_t slots = sms * (uint32_t)distance_ctas_per_sm(a.max_rows, 0u);
     uint32_t turns = strips * ((count + slots - 1u) / slots);
 
     const bool f64 = a.dist_f64 != nullptr;
     const size_t csmem1 = strip_smem_bytes(a.max_rows, false, cl, f64), csmem2 = strip_smem_bytes(a.max_rows, true, cl, f64);
     if (cl > kMaxDistCluster || csmem1 > kStripSmemMax) cl = 0u;
+    const bool tall = strip_cap_rows(a.max_rows) >= kClusterRowsMin;
+    if (cl > 1u && !tall && grid > 2u * sms / cl) cl = 0u; /* more histograms than clusters ever fit */
     const bool two = csmem2 <= kStripSmemMax;
     void (*kcl)(DistArgs, uint32_t, uint32_t);
     if (f64) kcl = a.ssd ? k_distance_cluster<true, true> : k_distance_cluster<true, false>;
@@ -1784,14 +1793,18 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
         if (f != cudaSuccess) return f;
     }
     /* clusters of cl CTAs where the histograms are tall, or where every
-     * histogram of the launch has a cluster to itself, if that takes fewer
-     * turns than strips by single CTAs do (a turn is a strip's time either
-     * way: 152 of 1001 x 256 with double sums 178 us in 11 turns of clusters,
-     * 114 in 8 of strips; 152 of 601 x 128 34 in 4 of strips, 120 of them 41 in
-     * 4 of clusters); as many clusters as fit at once, at most one per
-     * histogram slot */
+     * histogram of the launch has a cluster to itself, if that takes clearly
+     * fewer turns than strips by single CTAs do (a turn is a strip's time and
+     * with clusters a fifth more: 152 of 1001 x 256 with double sums 178 us in
+     * 11 turns of clusters, 114 in 8 of strips; 152 of 601 x 128 34 in 4 of
+     * strips, 120 of them 41 in 4 of clusters; 476 of 645 x 63, whole calls, 150
+     * in 7 of clusters, 142 in 8 of strips) and those are more than a cluster
+     * launch's own 3.5 us (kernel alone, strips and clusters: 108 of 107 x 61
+     * 11.5 and 12.9 us, 71 of 153 x 34 11.3 and 11.7, 5 of 261 x 48 14.5 and
+     * 12.1); as many clusters as fit at once, at most one per histogram slot */
     const uint32_t cturns = fit > 0 ? (count + (uint32_t)fit - 1u) / (uint32_t)fit : 0u;
-    const bool clusters = fit > 0 && (strip_cap_rows(a.max_rows) >= kClusterRowsMin || grid <= (uint32_t)fit) && cturns < turns;
+    const bool clusters = fit > 0 && (tall || grid <= (uint32_t)fit) && 6u * cturns < 5u * turns &&
+                          (turns - cturns) * (230u + a.max_rows) > 400u;
     if (clusters) turns = cturns;
     const bool rows = use_rows_(a, turns);
     if (rows) {
@@ -1802,12 +1815,13 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
         return cudaLaunchKernelEx(&cfg, kcl, a, two ? 1u : 0u, cl);
     }
     if (use_strip(a.max_rows, 0u)) {
-        void (*k)(DistArgs, uint32_t, uint32_t);
-        if (a.dist_f64) k = a.ssd ? k_distance_strip<true, true> : k_distance_strip<true, false>;
-        else k = a.ssd ? k_distance_strip<false, true> : k_distance_strip<false, false>;
+        void (*k)(DistArgs, uint32_t);
+        if (rows) k = a.ssd ? k_distance_strip<true, true, true> : k_distance_strip<true, false, true>;
+        else if (f64) k = a.ssd ? k_distance_strip<true, true, false> : k_distance_strip<true, false, false>;
+        else k = a.ssd ? k_distance_strip<false, true, false> : k_distance_strip<false, false, false>;
         cudaError_t e = allow_smem(k, kStripSmemMax);
         if (e != cudaSuccess) return e;
-        k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u, rows ? 1u : 0u);
+        k<<<grid, kStripThreads, smem, st>>>(a, strip_db(a.max_rows, 0u) ? 1u : 0u);
         return cudaGetLastError();
     }
     if (a.dist_f64) {
