@@ -409,13 +409,13 @@ class JobSequence:
 
 
 def simulate_traffic(launch_ms: float):
-    """DRAM bytes (read + write) of one k_simulate launch, from the ncu
+    """DRAM bytes (read + write) of one forward-model launch, from the ncu
     capture of a configuration-1 launch summarised in profiles/ (line
     'dram bytes per ms of launch: X'), scaled to this run's mean launch
     time; None when the summary is absent."""
     import re
     try:
-        with open(os.path.join(ROOT, "profiles", "k_simulate_config1_ncu_full.md")) as f:
+        with open(os.path.join(ROOT, "profiles", "k_simulate_walk_config1_ncu_full.md")) as f:
             m = re.search(r"dram bytes per ms of launch:\s*([0-9.eE+]+)", f.read())
     except OSError:
         return None
@@ -624,7 +624,8 @@ def measure_config(args, P, cfg, steps, warmup, rank, world, local, e2e=True):
                      "achieved_def": (f"({OPS_SPLIT_STEP} x particle-steps + {OPS_SPLIT_TASK} x x,y tasks) algorithmic "
                                       "thread-ops per launch / launch time" if split else
                                       f"{OPS_PER_STEP} algorithmic thread-ops per particle-step x steps per launch / "
-                                      "launch time"),
+                                      "launch time (a walk of every particle; those that provably are never detected "
+                                      "are walked along one coordinate, in fewer operations, so this can pass 1)"),
                      "ops_per_particle_step": ops_per_launch / max(1.0, steps_per_launch),
                      "peak_def": f"{sm_count} SMs x 128 lanes x {peaks.get('sm_max_mhz', 2070.0)} MHz ({peak_src} clock)"},
         "roofline_distance": {"bound": "hbm", "achieved": dist_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
