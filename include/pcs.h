@@ -416,6 +416,11 @@ pcs_status pcs_debug_particle_stream(pcs_ctx* ctx, uint64_t seed, uint32_t slot,
                                      uint32_t generation, uint32_t particle, uint32_t block,
                                      uint32_t out[4]);
 
+/* Which kernel the calling thread's last launch chose ("" before the first):
+ * family 0 the forward model, 1 the distance.  For tests of the rules that
+ * choose; rounds replayed from a graph do not count, their capture does. */
+const char* pcs_debug_last_kernel(int family);
+
 /* The proposals of the context's last batched round that belong to `job`
  * (checks of the proposal construction, src/gpu/detail/simulation_impl.inl
  * :256-347, which the reference builds on the host per proposal): for each,

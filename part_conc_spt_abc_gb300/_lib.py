@@ -181,6 +181,7 @@ SIGNATURES = {
                                          _u32p]),
     "pcs_debug_particle_stream": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32,
                                             C.c_uint32, C.c_uint32, _u32p]),
+    "pcs_debug_last_kernel": (C.c_char_p, [C.c_int]),
     "pcs_debug_round_proposals": (C.c_int, [C.c_void_p, C.c_uint32, _u32p, C.c_void_p, _f64p, _u32p]),
 }
 

@@ -830,6 +830,11 @@ pcs_status pcs_observed_sat_julia(pcs_ctx* ctx, const uint32_t* K, const double*
     });
 }
 
+const char* pcs_debug_last_kernel(int family)
+{
+    return family == 0 || family == 1 ? last_kernel((KernelFamily)family) : "";
+}
+
 pcs_status pcs_debug_particle_stream(pcs_ctx* ctx, uint64_t seed, uint32_t slot, uint32_t trial,
                                      uint32_t generation, uint32_t particle, uint32_t block, uint32_t out[4])
 {

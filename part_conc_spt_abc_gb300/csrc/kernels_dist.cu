@@ -1753,6 +1753,8 @@ static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st
 
 cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl)
 {
+    /* a caller that leaves these unset would get some kernel, but not the one that suits it */
+    if (!a.max_rows || !a.max_bins || !a.max_count) return cudaErrorInvalidValue;
     int dev = 0, n_sm = 0;
     cudaError_t e0 = cudaGetDevice(&dev);
     if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -1766,7 +1768,7 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
 
     const bool f64 = a.dist_f64 != nullptr;
     const size_t csmem1 = strip_smem_bytes(a.max_rows, false, cl, f64), csmem2 = strip_smem_bytes(a.max_rows, true, cl, f64);
-    if (cl > kMaxDistCluster || csmem1 > kStripSmemMax) cl = 0u;
+    if (a.strips_only || cl > kMaxDistCluster || csmem1 > kStripSmemMax) cl = 0u;
     const bool tall = strip_cap_rows(a.max_rows) >= kClusterRowsMin;
     if (cl > 1u && !tall && grid > 2u * sms / cl) cl = 0u; /* more histograms than clusters ever fit */
     const bool two = csmem2 <= kStripSmemMax;
@@ -1806,7 +1808,11 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
     const bool clusters = fit > 0 && (tall || grid <= (uint32_t)fit) && 6u * cturns < 5u * turns &&
                           (turns - cturns) * (230u + a.max_rows) > 400u;
     if (clusters) turns = cturns;
-    const bool rows = use_rows_(a, turns);
+    const bool rows = !a.strips_only && use_rows_(a, turns);
+    last_kernel(kFamilyDistance) = rows                        ? "k_distance_rows"
+                                   : clusters                  ? "k_distance_cluster"
+                                   : use_strip(a.max_rows, 0u) ? "k_distance_strip"
+                                                               : "k_distance";
     if (rows) {
         const cudaError_t e = launch_rows_(a, sms, st);
         if (e != cudaSuccess || !f64) return e;

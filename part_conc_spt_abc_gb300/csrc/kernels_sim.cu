@@ -1374,12 +1374,14 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
         SimArgs a = a_in;
         a.tile_words = split_tile_words_(a.tile_words);
         const size_t smem = (size_t)a.tile_words * 4u + sizeof(SplitShared);
+        last_kernel(kFamilyForward) = "k_simulate_split";
         return l.aggregate ? launch_split_<true>(a, l.grid, smem, st) : launch_split_<false>(a, l.grid, smem, st);
     }
     const SimArgs& a = a_in;
     if (l.few_items) {
         if (a.chunk != kFewChunk) return cudaErrorInvalidValue;
         const uint32_t per = kFewThreads / 32u;
+        last_kernel(kFamilyForward) = "k_simulate_few";
         if (l.few_items <= kFewItems8)
             k_simulate_few<8><<<(l.few_items * (kFewChunk / 4u) + per - 1u) / per, kFewThreads, 0, st>>>(a);
         else
@@ -1391,10 +1393,12 @@ cudaError_t launch_simulate(const SimArgs& a_in, const SimLaunch& l, cudaStream_
         const size_t tracks = walk_smem_(l.block);
         const cudaError_t e = allow_smem(fn, walk_smem_(1024u));
         if (e != cudaSuccess) return e;
+        last_kernel(kFamilyForward) = "k_simulate_walk";
         fn<<<l.grid, l.block, tracks, st>>>(a);
         return cudaGetLastError();
     }
     const size_t smem = (size_t)a.tile_words * 4u;
+    last_kernel(kFamilyForward) = "k_simulate";
 #define PCS_SIM_CASE(P, R, G)                                                               \
     if (l.ppt == P && l.replay == R && l.aggregate == G) return launch_sim_<P, R, G>(a, l.grid, l.block, smem, st);
     PCS_SIM_CASE(1, false, false)

@@ -71,6 +71,15 @@ inline cudaError_t allow_smem(F* fn, size_t most)
 }
 constexpr size_t kDynSmemMax = 227u * 1024u - 896u; /* of a CTA's 227 KB, for kernels with up to 896 bytes besides */
 
+/* The kernel that the calling thread's last launch of a family chose
+ * (pcs_debug_last_kernel); a captured round counts when it is captured. */
+enum KernelFamily { kFamilyForward = 0, kFamilyDistance = 1 };
+inline const char*& last_kernel(KernelFamily f)
+{
+    static thread_local const char* name[2] = {"", ""};
+    return name[f];
+}
+
 /* ---------------- scan + distance (kernels_dist.cu) ---------------- */
 struct DistArgs {
     const JobDev* jobs;
@@ -82,10 +91,12 @@ struct DistArgs {
     double* dist_f64;           /* [M] nullable: double-accumulator distance */
     uint64_t* ssd;              /* [M][2] nullable: exact integer sum (hi, lo) */
     uint32_t* err;
-    uint32_t max_rows;          /* rows of the carry array in shared memory */
+    /* what launch_distance chooses by; it refuses zeros in the first three */
+    uint32_t max_rows;          /* rows of the tallest histogram */
     uint32_t max_bins;          /* bins of the widest histogram */
     uint32_t max_count;         /* histograms at most */
     uint32_t min_count;         /* histograms at least, as far as the host knows */
+    uint32_t strips_only;       /* 1: a CTA's strips for each histogram, as the reference launches K_distance */
     const TmapDev* tmaps;       /* nullable: per job (index of jobs), tensor maps over hist */
 };
 /* A standalone launch's tables, filled on the device (launch_distance_setup):
@@ -105,10 +116,9 @@ struct DistSetup {
 cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaStream_t st);
 /* grid: CTAs at most (one histogram each).  cl > 1 (at least every job's
  * strips of 32 bins; 0 or 1: none) allows clusters of cl CTAs, one strip of
- * a histogram per CTA, which the launch takes where the histograms have at
- * least kClusterRowsMin rows or `grid` clusters fit at once; otherwise one
- * CTA walks each histogram's strips.  Variants with the double or integer
- * sums or the prefix-sum output take no clusters. */
+ * a histogram per CTA, for histograms of at least kClusterRowsMin rows or
+ * where `grid` clusters fit at once.  Which of clusters, rows and strips runs
+ * follows from the turns each takes (kernels_dist.cu). */
 cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl = 0u);
 /* the cluster size for histograms of up to max_rows x max_bins, or 0 */
 uint32_t distance_cluster_size(uint32_t max_rows, uint32_t max_bins);

@@ -174,9 +174,13 @@ void run_plain(Job& j, uint32_t max_steps, uint32_t queues)
         d.dist_f32 = q.d_dist.as<float>();
         d.err = c.err.as<uint32_t>();
         d.max_rows = j.R;
-        /* the reference's geometry: one CTA per histogram; the persistent
-         * form spreads the histogram's strips over a cluster */
-        PCS_CUDA(launch_distance(d, 1, q.st, ref_geometry ? 0u : distance_cluster_size(j.R, j.B)));
+        d.max_bins = j.B;
+        d.max_count = d.min_count = 1u;
+        /* the reference's geometry: one CTA walks the histogram strip by strip.
+         * The persistent form takes what a standalone call of one histogram
+         * takes: a cluster over its strips, the row kernel past 8 of them */
+        d.strips_only = ref_geometry;
+        PCS_CUDA(launch_distance(d, 1, q.st, distance_cluster_size(j.R, j.B)));
         PCS_CUDA(cudaMemcpyAsync(q.h_dist, q.d_dist.p, sizeof(float), cudaMemcpyDeviceToHost, q.st));
         PCS_CUDA(cudaEventRecord(q.done, q.st));
         q.slot = (int)slot;
