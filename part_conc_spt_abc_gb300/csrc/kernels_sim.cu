@@ -716,7 +716,8 @@ __device__ __forceinline__ void walk_warp_(const SimArgs& a, const ItemCtx& c, T
      * lies farther than this from the box's edge, one vote per group spares
      * the x and y wraps (-2% on configuration 3, -0.7% on configuration 1; a
      * vote that always says no costs 1%). */
-    const float in_x = c.hlx * (1.0f - 1.0e-6f) - 23.2f * q.sd, in_y = c.hly * (1.0f - 1.0e-6f) - 23.2f * q.sd;
+    const float far = 23.2f * fabsf(q.sd); /* a negative sd mirrors the steps */
+    const float in_x = c.hlx * (1.0f - 1.0e-6f) - far, in_y = c.hly * (1.0f - 1.0e-6f) - far;
     const bool vote = __all_sync(0xFFFFFFFFu, q.F == 0u || (c.hax < in_x && c.hay < in_y));
     uint32_t s0 = 1;
     for (; s0 + 3u < f_min; s0 += 4u) {
