@@ -270,7 +270,11 @@ __global__ void __launch_bounds__(1024, 1) k_distance(DistArgs a, uint32_t redo)
  * conversion per strip give the same double.  GB300's FP64 rate is a small
  * fraction of its FP32 rate: three FP64 operations and two conversions per
  * cell set the pace before (a short round of 201 x 1000: 398 -> 136 us;
- * 16 of 1001 x 256 with both sums and the prefix sums: 433 -> 114 us). */
+ * 16 of 1001 x 256 with both sums and the prefix sums: 433 -> 114 us).
+ * The standalone calls that ask for these take any counts, also an observed
+ * array that falls somewhere or prefix sums that wrap: the lane looks at all
+ * it has read and takes the conversions after all where some count is 2^22 or
+ * more.  (Calls for the float alone trust the last cells.) */
 const uint32_t kStripThreads = 512;
 const uint32_t kBox = 32;                     /* rows and columns of a tensor-map box */
 const uint32_t kBoxBytes = kBox * kBox * 4u;  /* 4096 */
@@ -746,9 +750,10 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                 const uint32_t* Tl = T + ((((w >> 1) ^ (l & 7u)) << 2) | ((2u * w) & 3u));
                 const uint32_t* __restrict__ refT = a.jobs[job].ref_sat_t;
                 const uint32_t* refc = refT + (uint64_t)colA * R;
-                const bool exact = T[sw_(R - 1u, 31u)] + carry[R - 1u] < kExactBelow &&
-                                   __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
+                bool exact = (F64 || SSD || !cum) && T[sw_(R - 1u, 31u)] + carry[R - 1u] < kExactBelow &&
+                             __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
                 uint64_t iA = 0u, iB = 0u;
+                uint32_t seen = 0u;
                 if (exact && inB) {
                     const uint2* ref2 = reinterpret_cast<const uint2*>(refc);
 #pragma unroll 4
@@ -763,6 +768,7 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                         if (F64 || SSD) {
                             iA += square_(v.x + c, o.x);
                             iB += square_(v.y + c, o.y);
+                            seen |= (v.x + c) | (v.y + c) | o.x | o.y;
                         }
                     }
                 } else if (exact) {
@@ -770,9 +776,15 @@ __device__ __forceinline__ void strip_cluster_(const DistArgs& a, uint32_t db, u
                         const uint32_t v = Tl[r << 5] + carry[r], o = __ldg(refc + r);
                         const float dA = exact_diff_(v, o);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
-                        if (F64 || SSD) iA += square_(v, o);
+                        if (F64 || SSD) {
+                            iA += square_(v, o);
+                            seen |= v | o;
+                        }
                     }
-                } else {
+                }
+                if (F64 || SSD) exact = exact && seen < kExactBelow;
+                if (!exact) {
+                    a2A = a2B = 0.0f;
                     for (uint32_t r = l; r < R; r += 32u) {
                         const uint32_t c = carry[r];
                         if (inB) {
@@ -901,7 +913,8 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
  *
  * Where every value of a block of rows is below 2^22 the differences are
  * exact integers (see k_distance_strip); other blocks take the reference's
- * conversions.  F64 needs exact differences and an exact sum of squares
+ * conversions.  All of the block's counts are looked at, not its last row's:
+ * an observed array passed to a standalone call need not grow down the rows.  F64 needs exact differences and an exact sum of squares
  * below 2^53, where the reference's chain of double additions is exact in any
  * order.  Whether that holds is known when the last row has passed: a
  * histogram for which it does not is left as it was (with F64 the zeroing
@@ -1089,9 +1102,14 @@ struct RowsWalk {
         float4 v[kRowsBlock];
 #pragma unroll
         for (uint32_t i = 0; i < kRowsBlock; ++i) v[i] = at[i * 32u];
-        /* counts grow down the rows: the block's largest are its last row's */
-        const uint4 sl = s[kRowsBlock - 1u], ol = o[kRowsBlock - 1u];
-        const bool exact = !__any_sync(0xFFFFFFFFu, (sl.w | ol.x | ol.y | ol.z | ol.w) >= kExactBelow);
+        /* every bit that a count of the block has (rows past the last repeat it) */
+        uint32_t seen = 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < kRowsBlock; ++i) {
+            seen |= s[i].x | s[i].y | s[i].z | s[i].w;
+            seen |= o[i].x | o[i].y | o[i].z | o[i].w;
+        }
+        const bool exact = !__any_sync(0xFFFFFFFFu, seen >= kExactBelow);
         if (!exact) high = true;
         if (F64 || exact) {
             terms<FULL>(b, s, v, [](uint32_t t, uint32_t q) { return exact_diff_(t, q); });
@@ -1101,14 +1119,15 @@ struct RowsWalk {
 #pragma unroll
         for (uint32_t i = 0; i < kRowsBlock; ++i) at[i * 32u] = v[i];
         if (F64 || SSD) {
+            uint64_t sq = 0u; /* of the block: below 2^49 */
 #pragma unroll
             for (uint32_t i = 0; i < kRowsBlock; ++i) {
                 if (!FULL && b * kRowsBlock + i >= R) break;
                 if (F64 || exact) {
-                    if (VEC || nc > 0u) lo += square_(s[i].x, o[i].x);
-                    if (VEC || nc > 1u) lo += square_(s[i].y, o[i].y);
-                    if (VEC || nc > 2u) lo += square_(s[i].z, o[i].z);
-                    if (VEC || nc > 3u) lo += square_(s[i].w, o[i].w);
+                    if (VEC || nc > 0u) sq += square_(s[i].x, o[i].x);
+                    if (VEC || nc > 1u) sq += square_(s[i].y, o[i].y);
+                    if (VEC || nc > 2u) sq += square_(s[i].z, o[i].z);
+                    if (VEC || nc > 3u) sq += square_(s[i].w, o[i].w);
                 } else {
                     if (VEC || nc > 0u) wide_square_(s[i].x, o[i].x);
                     if (VEC || nc > 1u) wide_square_(s[i].y, o[i].y);
@@ -1116,6 +1135,7 @@ struct RowsWalk {
                     if (VEC || nc > 3u) wide_square_(s[i].w, o[i].w);
                 }
             }
+            add128_(hi, lo, 0u, sq);
         }
         observe(b + 1u);
         if (cum) {
@@ -1433,9 +1453,10 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                 float a2A = 0.0f, a2B = 0.0f;
                 double a2dA = 0.0, a2dB = 0.0;
                 /* the largest cumulative counts: the strip's and the observed histogram's last cells */
-                const bool exact = T[sw_(R - 1u, 31u)] < kExactBelow &&
-                                   __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
+                bool exact = (F64 || SSD || !cum) && T[sw_(R - 1u, 31u)] < kExactBelow &&
+                             __ldg(refT + pcs_sat_t_index(R - 1u, B - 1u, R, B)) < kExactBelow;
                 uint64_t iA = 0u, iB = 0u; /* exact sums of squares of the lane's rows */
+                uint32_t seen = 0u;        /* every bit that a count of them has */
                 if (exact && inB) {
                     const uint2* ref2 = reinterpret_cast<const uint2*>(refc);
 #pragma unroll 4
@@ -1449,6 +1470,7 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                         if (F64 || SSD) {
                             iA += square_(s.x, o.x);
                             iB += square_(s.y, o.y);
+                            seen |= s.x | s.y | o.x | o.y;
                         }
                     }
                 } else if (exact) {
@@ -1457,9 +1479,15 @@ __global__ void __launch_bounds__(512, 2) k_distance_strip(DistArgs a, uint32_t 
                         const uint32_t s = Tl[r << 5], o = __ldg(refc + r);
                         const float dA = exact_diff_(s, o);
                         a2A = __fadd_rn(a2A, __fmul_rn(dA, dA));
-                        if (F64 || SSD) iA += square_(s, o);
+                        if (F64 || SSD) {
+                            iA += square_(s, o);
+                            seen |= s | o;
+                        }
                     }
-                } else {
+                }
+                if (F64 || SSD) exact = exact && seen < kExactBelow;
+                if (!exact) {
+                    a2A = a2B = 0.0f;
                     for (uint32_t r = l; r < R; r += 32u) {
                         if (inB) {
                             const uint2 s = *reinterpret_cast<const uint2*>(Tl + (r << 5));
