@@ -499,7 +499,7 @@ pcs_status pcs_serve_step(pcs_ctx* ctx, uint32_t* active)
             const uint64_t need_total = c.mem_used + j->arena_bytes() + hist_b;
             const uint64_t need_b = j->arena_bytes() + (uint64_t)c.tune.capacity * j->R * j->B * 4ull;
             const bool over_cap = c.mem_cap && need_total > c.mem_cap;
-            if (!over_cap && need_b + (64ull << 20) > (uint64_t)free_b && c.release_workspace())
+            if (!over_cap && need_b + (64ull << 20) > (uint64_t)free_b && c.ws.give_back())
                 PCS_CUDA(cudaMemGetInfo(&free_b, &total_b));
             if (over_cap || need_b + (64ull << 20) > (uint64_t)free_b) {
                 if (used == 0) throw Error(PCS_ERR_OUT_OF_MEMORY, "job does not fit in device memory");
@@ -611,7 +611,7 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
                      o_items = o_counts + Lease::need<uint32_t>(count * cstride),
                      in_bytes = o_items + Lease::need<uint32_t>(n_items);
         const uint64_t rp_n = replay ? totals[0] : 0u, rp_steps = replay ? replay->normal_stride : 0u;
-        Lease ws(c, in_bytes + Lease::need<uint32_t>(count * RB) + Lease::need<float>(4 * rp_n) +
+        Lease ws(c.ws, c.stream, in_bytes + Lease::need<uint32_t>(count * RB) + Lease::need<float>(4 * rp_n) +
                         Lease::need<float>(3 * rp_n * rp_steps) + Lease::need<float>(rp_n));
         char* d_in = ws.get<char>(in_bytes);
         uint32_t* d_hist = ws.get<uint32_t>(count * RB);
@@ -729,7 +729,7 @@ pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t*
         const size_t smem = distance_smem_bytes(rows);
         if (smem > 227u * 1024u) throw Error(PCS_ERR_UNSUPPORTED, "too many histogram rows for one CTA");
         cudaStream_t st = c.stream;
-        Lease ws(c, Lease::need<uint32_t>(count * RB) * (cum_out ? 2u : 1u) + 2u * Lease::need<uint32_t>(RB) +
+        Lease ws(c.ws, c.stream, Lease::need<uint32_t>(count * RB) * (cum_out ? 2u : 1u) + 2u * Lease::need<uint32_t>(RB) +
                         Lease::need<float>(count) + Lease::need<double>(count) + Lease::need<uint64_t>(2ull * count) +
                         Lease::need<JobDev>(1) + Lease::need<TmapDev>(1) + Lease::need<PropDev>(count) +
                         Lease::need<uint32_t>(1));
@@ -792,7 +792,7 @@ pcs_status pcs_observed_sat(pcs_ctx* ctx, const uint32_t* K, const double* DE, s
         if (rows == 0 || bins == 0) throw Error(PCS_ERR_INVALID_ARGUMENT, "rows and bins must be positive");
         cudaStream_t st = c.stream;
         const uint64_t RB = (uint64_t)rows * bins;
-        Lease ws(c, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
+        Lease ws(c.ws, c.stream, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
         uint32_t* dK = ws.get<uint32_t>(n);
         double* dDE = ws.get<double>(n);
         uint32_t* dS = ws.get<uint32_t>(RB);
@@ -816,7 +816,7 @@ pcs_status pcs_observed_sat_julia(pcs_ctx* ctx, const uint32_t* K, const double*
         if (kmax == 0 || bins == 0) throw Error(PCS_ERR_INVALID_ARGUMENT, "kmax and bins must be positive");
         cudaStream_t st = c.stream;
         const uint64_t RB = (uint64_t)kmax * bins;
-        Lease ws(c, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
+        Lease ws(c.ws, c.stream, Lease::need<uint32_t>(n) + Lease::need<double>(n) + Lease::need<uint32_t>(RB));
         uint32_t* dK = ws.get<uint32_t>(n);
         double* dDE = ws.get<double>(n);
         uint32_t* dS = ws.get<uint32_t>(RB);

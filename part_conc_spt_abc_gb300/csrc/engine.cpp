@@ -29,94 +29,6 @@ void cuda_check(cudaError_t e, const char* what)
     }
 }
 
-void DevBuf::alloc(size_t n)
-{
-    release();
-    if (n == 0) n = 16;
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e != cudaSuccess) {
-        p = nullptr;
-        (void)cudaGetLastError();
-        throw Error(PCS_ERR_OUT_OF_MEMORY, "device allocation of " + std::to_string(n) + " bytes failed");
-    }
-    bytes = n;
-}
-
-void DevBuf::release()
-{
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
-}
-
-/* ======================================================================= */
-/* workspace of the standalone entry points                                */
-/* ======================================================================= */
-
-Lease::Lease(Ctx& c, size_t bytes) : c_(c), held_(c.ws.mu, std::try_to_lock)
-{
-    size_ = std::max<size_t>(bytes, 256u);
-    if (held_.owns_lock() && size_ <= Workspace::kKeep) {
-        if (c.ws.dev.bytes < size_) {
-            size_t n = 1u << 20;
-            while (n < size_) n <<= 1;
-            c.ws.dev.release();
-            if (cudaMalloc(&c.ws.dev.p, n) == cudaSuccess) {
-                c.ws.dev.bytes = n;
-            } else { /* no room to keep that much: this call's own, below */
-                (void)cudaGetLastError();
-                c.ws.dev.p = nullptr;
-            }
-        }
-        base_ = c.ws.dev.as<char>();
-    }
-    if (!base_) {
-        own_.alloc(size_);
-        base_ = own_.as<char>();
-    }
-}
-
-Lease::~Lease()
-{
-    /* a call that failed on its way may have left work that uses this memory */
-    if (!done_) cudaStreamSynchronize(c_.stream);
-}
-
-void* Lease::take(size_t bytes)
-{
-    if (used_ + bytes > size_) throw Error(PCS_ERR_INVALID_ARGUMENT, "workspace overflow");
-    void* p = base_ + used_;
-    used_ += bytes;
-    return p;
-}
-
-char* Lease::stage(size_t n)
-{
-    n = (n + 63u) / 64u * 64u;
-    if (!held_.owns_lock() || !c_.ws.pinned || staged_ + n > Workspace::kPinned) return nullptr;
-    char* p = c_.ws.pinned + staged_;
-    staged_ += n;
-    return p;
-}
-
-bool Ctx::release_workspace()
-{
-    std::unique_lock<std::mutex> held(ws.mu, std::try_to_lock);
-    if (!held.owns_lock() || !ws.dev.p) return false;
-    ws.dev.release();
-    return true;
-}
-
-void Ctx::alloc(DevBuf& b, size_t n)
-{
-    try {
-        b.alloc(n);
-    } catch (const Error& e) {
-        if (e.status != PCS_ERR_OUT_OF_MEMORY || !release_workspace()) throw;
-        b.alloc(n);
-    }
-}
-
 /* ======================================================================= */
 /* validation                                                              */
 /* ======================================================================= */
@@ -226,7 +138,7 @@ T* carve(char*& cur, uint64_t n)
 void Job::build_device_state()
 {
     if (initialised) return;
-    ctx->alloc(arena, arena_bytes() + 4096);
+    ctx->ws.alloc(arena, arena_bytes() + 4096);
     char* cur = arena.as<char>();
     const uint64_t nP = (uint64_t)N * P;
     double* d_theta = carve<double>(cur, nP);
@@ -250,8 +162,8 @@ void Job::build_device_state()
     /* observed data -> cumulative histogram on the device */
     {
         DevBuf dK, dDE;
-        ctx->alloc(dK, std::max<size_t>(K.size(), 1) * 4);
-        ctx->alloc(dDE, std::max<size_t>(DE.size(), 1) * 8);
+        ctx->ws.alloc(dK, std::max<size_t>(K.size(), 1) * 4);
+        ctx->ws.alloc(dDE, std::max<size_t>(DE.size(), 1) * 8);
         if (!K.empty()) {
             PCS_CUDA(cudaMemcpyAsync(dK.p, K.data(), K.size() * 4, cudaMemcpyHostToDevice, st));
             PCS_CUDA(cudaMemcpyAsync(dDE.p, DE.data(), DE.size() * 8, cudaMemcpyHostToDevice, st));
@@ -565,20 +477,20 @@ void Ctx::ensure_round_buffers(uint32_t v_max, uint32_t max_rows, uint32_t max_n
     rb.items_cap = (uint32_t)std::max<uint64_t>(items_need, rb.items_cap);
     rb.counts_cap = (uint64_t)cap * (2ull * rb.v_max + 1ull);
     rb.hist_cap = std::max<uint64_t>(hist_need, rb.hist_cap);
-    alloc(rb.round, sizeof(RoundDev));
-    alloc(rb.props, sizeof(PropDev) * (size_t)cap);
-    alloc(rb.theta_prop, sizeof(double) * (size_t)cap * PCS_MAX_P);
-    alloc(rb.counts, sizeof(uint32_t) * rb.counts_cap);
-    alloc(rb.item_prop, sizeof(uint32_t) * (size_t)rb.items_cap);
-    alloc(rb.hist, sizeof(uint32_t) * rb.hist_cap);
+    ws.alloc(rb.round, sizeof(RoundDev));
+    ws.alloc(rb.props, sizeof(PropDev) * (size_t)cap);
+    ws.alloc(rb.theta_prop, sizeof(double) * (size_t)cap * PCS_MAX_P);
+    ws.alloc(rb.counts, sizeof(uint32_t) * rb.counts_cap);
+    ws.alloc(rb.item_prop, sizeof(uint32_t) * (size_t)rb.items_cap);
+    ws.alloc(rb.hist, sizeof(uint32_t) * rb.hist_cap);
     PCS_CUDA(cudaMemsetAsync(rb.hist.p, 0, sizeof(uint32_t) * rb.hist_cap, stream));
-    alloc(rb.dist32, sizeof(float) * (size_t)cap);
-    alloc(rb.dist64, sizeof(double) * (size_t)cap);
+    ws.alloc(rb.dist32, sizeof(float) * (size_t)cap);
+    ws.alloc(rb.dist64, sizeof(double) * (size_t)cap);
     if (!rb.jobs.p) {
-        alloc(rb.tmaps, sizeof(TmapDev) * kMaxRoundJobs);
+        ws.alloc(rb.tmaps, sizeof(TmapDev) * kMaxRoundJobs);
         PCS_CUDA(cudaMemsetAsync(rb.tmaps.p, 0, sizeof(TmapDev) * kMaxRoundJobs, stream));
-        alloc(rb.jobs, sizeof(JobDev) * kMaxRoundJobs);
-        alloc(rb.pmc, sizeof(JobPmcDev) * kMaxRoundJobs);
+        ws.alloc(rb.jobs, sizeof(JobDev) * kMaxRoundJobs);
+        ws.alloc(rb.pmc, sizeof(JobPmcDev) * kMaxRoundJobs);
         PCS_CUDA(cudaMemsetAsync(rb.jobs.p, 0, sizeof(JobDev) * kMaxRoundJobs, stream));
         /* empty table slots read as finished jobs */
         std::vector<JobPmcDev> empty(kMaxRoundJobs);

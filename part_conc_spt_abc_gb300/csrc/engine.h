@@ -49,25 +49,29 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
-struct Ctx;
-
 /* Memory that the standalone entry points keep between calls: device memory
  * up to kKeep bytes (allocating and freeing nine buffers took 30-40 us of a
  * 90 us call) and a pinned page for small transfers.  One call at a time
  * holds it (Lease); a call that finds it taken by another thread, or needs
  * more, allocates its own for the call.  Given back at pcs_close, and when
- * an allocation of the context's jobs fails (Ctx::alloc). */
+ * another allocation of the context fails: its jobs', the plain form's
+ * (alloc) or that of a call which needs more. */
 struct Workspace {
     static const size_t kKeep = 64ull << 20, kPinned = 64ull << 10;
     std::mutex mu;
     DevBuf dev;
     char* pinned = nullptr;
+
+    /* frees the device memory; false if there is none or a call holds it */
+    bool give_back();
+    /* b.alloc(n); if that fails, once more after give_back() */
+    void alloc(DevBuf& b, size_t n);
 };
 
 class Lease {
 public:
     /* bytes: the sum of need<T>(n) over the get<T>(n) that follow */
-    Lease(Ctx& c, size_t bytes);
+    Lease(Workspace& ws, cudaStream_t stream, size_t bytes);
     ~Lease();
     Lease(const Lease&) = delete;
     Lease& operator=(const Lease&) = delete;
@@ -80,7 +84,9 @@ public:
 
 private:
     void* take(size_t bytes);
-    Ctx& c_;
+    void own_alloc_();
+    Workspace& ws_;
+    cudaStream_t stream_;
     std::unique_lock<std::mutex> held_;
     DevBuf own_;
     char* base_ = nullptr;
@@ -146,11 +152,6 @@ struct Ctx {
 
     explicit Ctx(int dev, int inflight);
     ~Ctx();
-
-    /* b.alloc(n); if that fails, once more with the workspace given back */
-    void alloc(DevBuf& b, size_t n);
-    /* frees the workspace's device memory; false if there is none or a call holds it */
-    bool release_workspace();
 
     /* round machinery */
     void ensure_round_buffers(uint32_t v_max, uint32_t max_rows, uint32_t max_n, uint64_t rb_max);

@@ -68,7 +68,7 @@ void run_plain(Job& j, uint32_t max_steps, uint32_t queues)
     PCS_CUDA(cudaMemcpy(factor.data(), pm.factor, factor.size() * 8, cudaMemcpyDeviceToHost));
 
     DevBuf d_job;
-    d_job.alloc(sizeof(JobDev));
+    c.ws.alloc(d_job, sizeof(JobDev));
     PCS_CUDA(cudaMemcpy(d_job.p, &j.jd, sizeof(JobDev), cudaMemcpyHostToDevice));
 
     /* particles per proposal are bounded by the prior's largest Poisson mean */
@@ -84,13 +84,13 @@ void run_plain(Job& j, uint32_t max_steps, uint32_t queues)
     for (auto& q : qs) {
         PCS_CUDA(cudaStreamCreateWithFlags(&q.st, cudaStreamNonBlocking));
         PCS_CUDA(cudaEventCreateWithFlags(&q.done, cudaEventDisableTiming));
-        q.d_prop.alloc(sizeof(PropDev));
-        q.d_counts.alloc(sizeof(uint32_t) * (2 * V + 1));
-        q.d_items.alloc(sizeof(uint32_t) * items_cap);
-        q.d_ctl.alloc(16);
-        q.d_hist.alloc(sizeof(uint32_t) * RB);
-        q.d_dist.alloc(sizeof(float));
-        q.d_nprops.alloc(4);
+        c.ws.alloc(q.d_prop, sizeof(PropDev));
+        c.ws.alloc(q.d_counts, sizeof(uint32_t) * (2 * V + 1));
+        c.ws.alloc(q.d_items, sizeof(uint32_t) * items_cap);
+        c.ws.alloc(q.d_ctl, 16);
+        c.ws.alloc(q.d_hist, sizeof(uint32_t) * RB);
+        c.ws.alloc(q.d_dist, sizeof(float));
+        c.ws.alloc(q.d_nprops, 4);
         PCS_CUDA(cudaMemset(q.d_items.p, 0, sizeof(uint32_t) * items_cap));
         PCS_CUDA(cudaMemset(q.d_hist.p, 0, sizeof(uint32_t) * RB));
         const uint32_t one = 1u;
