@@ -273,7 +273,9 @@ pcs_status pcs_serve_poll(pcs_ctx* ctx, pcs_job* job, int* finished);
 /* Caps the device memory the serve loop may use (bytes, 0 = free memory):
  * a queued job is admitted while the admitted jobs' arenas, its own and the
  * round histograms (round capacity x the widest admitted job's R x B words)
- * fit; a job that does not fit even alone fails with PCS_ERR_OUT_OF_MEMORY. */
+ * fit; a job that does not fit even alone fails with PCS_ERR_OUT_OF_MEMORY.
+ * While a cap is set the standalone entry points below keep no device memory
+ * between calls (without one up to 64 MiB). */
 pcs_status pcs_serve_set_memory_cap(pcs_ctx* ctx, uint64_t bytes);
 
 /* ------------------------------------------------------------------ */

@@ -474,7 +474,11 @@ pcs_status pcs_serve_submit(pcs_ctx* ctx, pcs_job* job)
 
 pcs_status pcs_serve_set_memory_cap(pcs_ctx* ctx, uint64_t bytes)
 {
-    return guard([&] { C_(ctx).mem_cap = bytes; });
+    return guard([&] {
+        Ctx& c = C_(ctx);
+        c.mem_cap = bytes;
+        c.ws.set_keep(bytes == 0);
+    });
 }
 
 pcs_status pcs_serve_step(pcs_ctx* ctx, uint32_t* active)

@@ -12,6 +12,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <chrono>
 #include <cstdint>
 #include <deque>
@@ -55,13 +56,18 @@ struct DevBuf {
  * holds it (Lease); a call that finds it taken by another thread, or needs
  * more, allocates its own for the call.  Given back at pcs_close, and when
  * another allocation of the context fails: its jobs', the plain form's
- * (alloc) or that of a call which needs more. */
+ * (alloc) or that of a call which needs more.  Under a cap on the serve
+ * loop's memory, which does not count it, nothing is kept. */
 struct Workspace {
     static const size_t kKeep = 64ull << 20, kPinned = 64ull << 10;
     std::mutex mu;
     DevBuf dev;
     char* pinned = nullptr;
+    std::atomic<bool> keep{true};
 
+    /* false: what is kept is given back, at once or at the end of the call
+     * that holds it, and calls allocate their own from then on */
+    void set_keep(bool k);
     /* frees the device memory; false if there is none or a call holds it */
     bool give_back();
     /* b.alloc(n); if that fails, once more after give_back() */

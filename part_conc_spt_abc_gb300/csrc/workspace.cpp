@@ -36,6 +36,12 @@ bool Workspace::give_back()
     return true;
 }
 
+void Workspace::set_keep(bool k)
+{
+    keep = k;
+    if (!k) give_back();
+}
+
 void Workspace::alloc(DevBuf& b, size_t n)
 {
     try {
@@ -49,7 +55,8 @@ void Workspace::alloc(DevBuf& b, size_t n)
 Lease::Lease(Workspace& ws, cudaStream_t stream, size_t bytes) : ws_(ws), stream_(stream), held_(ws.mu, std::try_to_lock)
 {
     size_ = std::max<size_t>(bytes, 256u);
-    if (held_.owns_lock() && size_ <= Workspace::kKeep) {
+    if (held_.owns_lock() && !ws_.keep) ws_.dev.release();
+    if (held_.owns_lock() && ws_.keep && size_ <= Workspace::kKeep) {
         if (ws_.dev.bytes < size_) {
             size_t n = 1u << 20;
             while (n < size_) n <<= 1;
@@ -87,6 +94,7 @@ Lease::~Lease()
 {
     /* a call that failed on its way may have left work that uses this memory */
     if (!done_) cudaStreamSynchronize(stream_);
+    if (held_.owns_lock() && !ws_.keep) ws_.dev.release();
 }
 
 void* Lease::take(size_t bytes)

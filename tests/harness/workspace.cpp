@@ -68,6 +68,21 @@ int ws_call(void* w, size_t bytes, size_t inner)
     }
 }
 
+/* a cap set (1) or lifted (0) */
+void ws_cap(void* w, int on) { static_cast<pcs::Workspace*>(w)->set_keep(!on); }
+
+/* a cap set during a call of `bytes`: what is allocated after it */
+size_t ws_cap_during_call(void* w, size_t bytes)
+{
+    pcs::Workspace& ws = *static_cast<pcs::Workspace*>(w);
+    {
+        pcs::Lease lease(ws, nullptr, bytes);
+        std::thread([&] { ws_cap(w, 1); }).join();
+        lease.done();
+    }
+    return g_used;
+}
+
 /* a job's buffer, freed at once */
 int ws_job(void* w, size_t bytes)
 {
