@@ -192,6 +192,7 @@ void Job::build_device_state()
     jd.Z = Z;
     jd.P = P;
     pcs_seed_masks(seed, &jd.seed_lo, &jd.seed_hi);
+    jd.distance_double = p.distance_double ? 1u : 0u;
     jd.frames_max = R - 1;
     jd.frames = d_frames;
     jd.ref_sat = d_sat;
@@ -542,9 +543,7 @@ void Ctx::enqueue_round()
     a.h_pmc = h_status;
     a.h_round = h_round_out;
     a.h_err = h_err;
-    a.use_f64_distance = 0u;
-    for (Job* j : table)
-        if (j && j->p.distance_double) a.use_f64_distance = 1u;
+    a.use_f64_distance = rb_f64_;
 
     PCS_CUDA(launch_round_plan(a, stream));
     PCS_CUDA(launch_propose(a, rb.capacity, stream));
@@ -693,16 +692,19 @@ void Ctx::admit(Job* j)
     j->slot = slot;
     uint32_t v_max = 0, max_rows = 0, max_n = 0, max_b = 0;
     uint64_t rb_max = 0;
+    bool f64 = false;
     for (Job* t : table)
         if (t) {
+            f64 |= t->p.distance_double != 0;
             v_max = std::max(v_max, t->V);
             max_rows = std::max(max_rows, t->R);
             max_n = std::max(max_n, t->N);
             max_b = std::max(max_b, t->B);
             rb_max = std::max<uint64_t>(rb_max, (uint64_t)t->R * t->B);
         }
-    if (max_b != rb_max_b_) {
+    if (max_b != rb_max_b_ || f64 != rb_f64_) {
         rb_max_b_ = max_b;
+        rb_f64_ = f64;
         graph_dirty = true;
     }
     ensure_round_buffers(v_max, max_rows, max_n, rb_max);

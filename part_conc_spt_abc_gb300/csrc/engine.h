@@ -145,6 +145,7 @@ struct Ctx {
     std::vector<Job*> table;       /* jobs in the round table (index = table slot) */
     std::deque<Job*> queue;        /* serve: submitted, not yet admitted */
     uint32_t rb_max_b_ = 0;        /* widest histogram row among admitted jobs */
+    bool rb_f64_ = false;          /* some admitted job's distances are double */
     uint64_t mem_cap = 0;
     uint64_t mem_used = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -478,7 +478,9 @@ __global__ void __launch_bounds__(1024) k_accept(PmcArgs a)
     while (g < 32u && g < k) g <<= 1;
     const uint32_t lane = threadIdx.x & 31u, gl = lane & (g - 1u), g0 = lane & ~(g - 1u);
     const unsigned gmask = g == 32u ? 0xFFFFFFFFu : (1u << g) - 1u;
-    const bool prior = pm.generation == 0u, f64 = a.use_f64_distance && a.dist_f64;
+    const bool prior = pm.generation == 0u;
+    /* the job's own choice: another job's in the round may have the doubles formed */
+    const bool f64 = a.jobs[j].distance_double && a.use_f64_distance && a.dist_f64;
     const double gamma = pm.gamma, sure = s_sure, never = s_never;
     unsigned long long trials = 0ull, accepted = 0ull;
     for (uint32_t i0 = 0; i0 < npend; i0 += blockDim.x / g) {

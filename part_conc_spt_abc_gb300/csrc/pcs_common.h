@@ -227,6 +227,7 @@ struct JobDev {
     uint32_t seed_lo, seed_hi;
     uint32_t frames_max;
     uint32_t tmap_depth;   /* histograms the job's tensor map spans (0: no tensor map) */
+    uint32_t distance_double; /* 1: trials are accepted by the double distance */
     const uint32_t* frames;     /* [V] */
     const uint32_t* ref_sat;    /* [R*B] observed cumulative histogram */
     const uint32_t* ref_sat_t;  /* [B*R] column-major copy, pairs interleaved (pcs_sat_t_index) */
