@@ -1747,7 +1747,8 @@ cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaSt
  * With double sums the walk zeroes in a second pass and a launch for the
  * histograms left over follows: 8 turns (1001 x 256 x 152) 114 -> 138, 16
  * (x 304) 228 -> 166, 32 (201 x 1000 x 20) 126 -> 63.
- * Where rows are not 16-byte aligned the lanes copy cell by cell: 8 turns
+ * Where rows are not 16-byte aligned (in a round of several jobs: the widest
+ * one's, which has the most of the work) the lanes copy cell by cell: 8 turns
  * (201 x 255 x 100) 39.4 -> 43, 12 (201 x 99 x 912) 75.9 -> 57.8, 32 (201 x
  * 999 x 38) 145 -> 90; and a warp has to replace three strips: with one (51 x
  * 31 x 3000) 44.6 -> 57, with two (329 x 49 x 2036, whole calls) 203 -> 235.
@@ -1822,16 +1823,17 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
         const cudaError_t f = cluster_fit_(kcl, cfg, cl, cfg.dynamicSmemBytes, fit);
         if (f != cudaSuccess) return f;
     }
-    /* clusters of cl CTAs where the histograms are tall, or where every
-     * histogram of the launch has a cluster to itself, if that takes clearly
-     * fewer turns than strips by single CTAs do (a turn is a strip's time and
-     * with clusters a fifth more: 152 of 1001 x 256 with double sums 178 us in
-     * 11 turns of clusters, 114 in 8 of strips; 152 of 601 x 128 34 in 4 of
-     * strips, 120 of them 41 in 4 of clusters; 476 of 645 x 63, whole calls, 150
-     * in 7 of clusters, 142 in 8 of strips) and those are more than a cluster
-     * launch's own 3.5 us (kernel alone, strips and clusters: 108 of 107 x 61
-     * 11.5 and 12.9 us, 71 of 153 x 34 11.3 and 11.7, 5 of 261 x 48 14.5 and
-     * 12.1); as many clusters as fit at once, at most one per histogram slot */
+    /* clusters of cl CTAs where the histograms are tall, or where every histogram of
+     * the launch has a cluster to itself, if that takes clearly fewer turns than
+     * strips by single CTAs do.  A turn is a strip's time, 2.2 us + 9.5 ns per row
+     * (see use_rows_), that is (230 + rows) x 9.5 ns, and with clusters a fifth more,
+     * hence the 6 to 5 (152 of 1001 x 256 with double sums 178 us in 11 turns of
+     * clusters, 114 in 8 of strips; 152 of 601 x 128 34 in 4 of strips, 120 of them 41
+     * in 4 of clusters; 476 of 645 x 63, whole calls, 150 in 7 of clusters, 142 in 8
+     * of strips); and the turns saved have to be more than a cluster launch's own 3.5
+     * us, with a margin 400 x 9.5 ns (kernel alone, strips and clusters: 108 of 107 x
+     * 61 11.5 and 12.9 us, 71 of 153 x 34 11.3 and 11.7, 5 of 261 x 48 14.5 and 12.1);
+     * as many clusters as fit at once, at most one per histogram slot */
     const uint32_t cturns = fit > 0 ? (count + (uint32_t)fit - 1u) / (uint32_t)fit : 0u;
     const bool clusters = fit > 0 && (tall || grid <= (uint32_t)fit) && 6u * cturns < 5u * turns &&
                           (turns - cturns) * (230u + a.max_rows) > 400u;

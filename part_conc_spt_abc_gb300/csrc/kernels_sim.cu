@@ -831,8 +831,10 @@ __device__ __forceinline__ bool screen_walk_(const Walker& q, const ItemCtx& c)
 
 } // namespace
 
-/* Registers: 80 a thread in CTAs of up to 256 threads (24 warps per SM; 64
- * and 32 warps, or 128 and 16, were slower by 1-4%), 64 in CTAs of 1024. */
+/* Registers: at most 80 a thread in CTAs of up to 256 threads (it uses 71; 24
+ * warps per SM; 64 and 32 warps, or 128 and 16, were slower by 1-4%).  CTAs of
+ * 512 threads also use 71, so one fits on an SM (16 warps), and CTAs of 1024
+ * have 64 (32 warps, some spills); the autotuner times all three. */
 template <uint32_t BLOCK>
 __global__ void __launch_bounds__(BLOCK, BLOCK <= 256u ? 3 : 1) k_simulate_walk(const __grid_constant__ SimArgs a)
 {
@@ -1329,7 +1331,7 @@ int occupancy_(uint32_t block, size_t smem)
     return n;
 }
 
-/* the tile-less walk's build for `block` threads (64 registers each way) */
+/* the tile-less walk's build for `block` threads */
 auto walk_kernel_(uint32_t block) -> void (*)(SimArgs)
 {
     return block <= 256u ? k_simulate_walk<256> : (block <= 512u ? k_simulate_walk<512> : k_simulate_walk<1024>);
