@@ -53,10 +53,16 @@ sys.path.insert(0, ROOT)
 #   slab-split walk, per task (a group walked in x, y): 8 uniforms (176) + 4
 #     pairs (48) + bridge means (12) + four x, y steps with detection and DE
 #     (72) + track bookkeeping (12) = 320.
-# The compiled per-step walk executes fewer thread instructions than its 105
-# (~73 on a configuration-1 round, ncu): wide multiplies and fused
-# multiply-adds do more than one of these operations each.
+# What the per-step walk cannot do without are its draws: every frame of every
+# particle, screened or not, takes three quarters of a Philox4x32-10 call, of
+# whose 20 32 x 32 -> 64 bit products 16 depend on the frame (pcs_draw_pre): 12
+# per particle-step.  A warp's product holds a scheduler's FMA-heavy pipe for
+# four cycles, so an SM does 32 a cycle.  The 105 are the work of walking every
+# particle; a screened one's step takes fewer, so a rate by them is no share of
+# a bound.
 OPS_PER_STEP = 105
+PRODUCTS_PER_STEP = 12
+PRODUCTS_PER_CYCLE = 32  # per SM
 OPS_SPLIT_STEP = 49.5
 OPS_SPLIT_TASK = 320
 # bytes the distance kernel moves per histogram cell: read count, write zero,
@@ -582,16 +588,18 @@ def measure_config(args, P, cfg, steps, warmup, rank, world, local, e2e=True):
     if e2e:
         e2e_value, h2d, d2h = e2e_run(P, ctx, inp, sequence, steps, rank, world)
 
-    # ---- roofline of the dominant kernel (forward model: issue bound) -----
+    # ---- roofline of the dominant kernel (forward model: arithmetic pipes) -----
     sim_ms = ks.simulate_ms / max(1, ks.simulate_launches)
     steps_per_launch = ks.particle_steps / max(1, ks.simulate_launches)
     split = t.walk == 1
     tasks_per_launch = ks.split_tasks / max(1, ks.simulate_launches)
     ops_per_launch = (steps_per_launch * OPS_SPLIT_STEP + tasks_per_launch * OPS_SPLIT_TASK if split
-                      else steps_per_launch * OPS_PER_STEP)
+                      else steps_per_launch * PRODUCTS_PER_STEP)
     achieved = ops_per_launch / (sim_ms / 1e3) / 1e12
     sm_count = device_sm_count(P, local)
-    peak = sm_count * 128 * float(peaks.get("sm_max_mhz", 2070.0)) * 1e6 / 1e12
+    sm_mhz = float(peaks.get("sm_max_mhz", 2070.0))
+    per_cycle = 128 if split else PRODUCTS_PER_CYCLE
+    peak = sm_count * per_cycle * sm_mhz * 1e6 / 1e12
     traffic = simulate_traffic(sim_ms) if cfg == 1 else None
     dist_ms = ks.distance_ms / max(1, ks.distance_launches)
     dist_gbs = (ks.histogram_cells / max(1, ks.distance_launches)) * DIST_BYTES_PER_CELL / (dist_ms / 1e3) / 1e9
@@ -618,16 +626,20 @@ def measure_config(args, P, cfg, steps, warmup, rank, world, local, e2e=True):
         "e2e": ({"value": e2e_value, "unit": "particle-steps/s", "h2d_bytes_per_step": int(h2d),
                  "d2h_bytes_per_step": int(d2h)} if e2e else None),
         "gpu_launches": int(ks.kernel_launches),
-        "roofline": {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "Tops/s",
+        "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
+                     "unit": "Tops/s" if split else "T products/s (32 x 32 -> 64 bits)",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": "k_simulate (fused forward model + histogram)",
+                     "kernel": ("k_simulate_split" if split else "k_simulate" if t.hist_tile_rows or t.particles_per_thread > 1
+                                else "k_simulate_walk")
+                               + " (fused forward model + histogram)",
                      "achieved_def": (f"({OPS_SPLIT_STEP} x particle-steps + {OPS_SPLIT_TASK} x x,y tasks) algorithmic "
                                       "thread-ops per launch / launch time" if split else
-                                      f"{OPS_PER_STEP} algorithmic thread-ops per particle-step x steps per launch / "
-                                      "launch time (a walk of every particle; those that provably are never detected "
-                                      "are walked along one coordinate, in fewer operations, so this can pass 1)"),
+                                      f"{PRODUCTS_PER_STEP} Philox products per particle-step x steps per launch / launch "
+                                      "time: the draws, which no walk of these streams can do without"),
                      "ops_per_particle_step": ops_per_launch / max(1.0, steps_per_launch),
-                     "peak_def": f"{sm_count} SMs x 128 lanes x {peaks.get('sm_max_mhz', 2070.0)} MHz ({peak_src} clock)"},
+                     "peak_def": f"{sm_count} SMs x {per_cycle} " + ("lanes" if split else "products a cycle (FMA-heavy pipe)")
+                                 + f" x {sm_mhz} MHz ({peak_src} clock)",
+                     "walk_of_every_particle_tops": steps_per_launch * OPS_PER_STEP / (sim_ms / 1e3) / 1e12},
         "roofline_distance": {"bound": "hbm", "achieved": dist_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                               "frac": dist_gbs / float(peaks.get("hbm_gbs", 6800.0)),
                               "kernel": "k_distance", "peak_src": peak_src},

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(sim_max_block(PPT)) k_simulate(SimArgs a)
  * pass and three generations (5.6e10 particle-steps) 158 -> 120 ms;
  * configuration 0, a whole job's 66 short rounds 24.7 -> 20.3 ms.  The bound
  * is the FMA-heavy pipe, where a Philox round's 32 x 32 -> 64 bit product
- * takes four cycles: 52 products a group, 208 of the ~440 cycles per warp
+ * takes four cycles: 48 products a group, 192 of the ~440 cycles per warp
  * and group of a full walk and of the ~290 of a screen walk. */
 
 constexpr uint32_t kScreenQueue = 96;     /* entries of each queue: at most 62 stay between visits, 32 more during one */
