@@ -911,20 +911,19 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
  * A walk down few rows at a time costs a fixed 90 ns per row, so few
  * histograms of few columns stay with the strips (use_rows_).
  *
- * Where every value of a block of rows is below 2^22 the differences are
- * exact integers (see k_distance_strip); other blocks take the reference's
+ * Where every value of a block of rows is below 2^22 the differences are exact
+ * integers (see k_distance_strip); other blocks take the reference's
  * conversions.  All of the block's counts are looked at, not its last row's:
  * an observed array passed to a standalone call need not grow down the rows.
  * The vote comes after the integer form's terms, which are dropped where it
  * fails, so nothing waits for it (device time of whole device calls: 304 of
- * 1001 x 256 144 us, 143 without
- * the look at every count, 146 with the vote before the terms; 152 of 1700 x
- * 256 202, 201, 214).  F64 needs exact differences and an exact sum of squares
- * below 2^53, where the reference's chain of double additions is exact in any
- * order.  Whether that holds is known when the last row has passed: a
- * histogram for which it does not is left as it was (with F64 the zeroing
- * waits for the verdict) with kRedo as its distance, and the strip kernel
- * launched after it takes it. */
+ * 1001 x 256 144 us, 143 without the look at every count, 146 with the vote
+ * before the terms; 152 of 1700 x 256 202, 201, 214).  F64 needs exact
+ * differences and an exact sum of squares below 2^53, where the reference's
+ * chain of double additions is exact in any order.  Whether that holds is
+ * known when the last row has passed: a histogram for which it does not is
+ * left as it was (with F64 the zeroing waits for the verdict) with kRedo as
+ * its distance, and the strip kernel launched after it takes it. */
 const uint32_t kRowsBlock = 8u, kRowsRing = 3u, kRowsWarps = 8u;
 const uint32_t kRowsAccBytes = 32u * 128u * 4u, kRowsRingBytes = kRowsRing * kRowsBlock * 512u;
 const uint32_t kRowsWarpBytes = kRowsAccBytes + kRowsRingBytes;
