@@ -505,6 +505,24 @@ void Ctx::ensure_round_buffers(uint32_t v_max, uint32_t max_rows, uint32_t max_n
     graph_dirty = true;
 }
 
+/* The rounds' mean width, jobs weighted by their populations; the graph is
+ * captured anew where that changes the distance kernel's choice. */
+void Ctx::look_at_widths()
+{
+    uint64_t strips = 0, slots = 0;
+    for (Job* t : table)
+        if (t) {
+            strips += (uint64_t)t->N * ((t->B + 31u) / 32u);
+            slots += t->N;
+        }
+    if (!slots) return;
+    const bool narrow = distance_mostly_narrow(rb.max_rows, rb_max_b_, (uint32_t)(16u * strips / slots));
+    if (narrow != rb_narrow_) {
+        rb_narrow_ = narrow;
+        graph_dirty = true;
+    }
+}
+
 void Ctx::upload_table()
 {
     RoundDev& r = *h_round;
@@ -587,6 +605,7 @@ void Ctx::enqueue_round()
     d.max_bins = rb_max_b_;
     d.max_count = rb.capacity;
     d.min_count = 1u; /* the round's number is the device's */
+    d.mostly_narrow = rb_narrow_;
     d.tmaps = rb.tmaps.as<TmapDev>();
     const uint32_t cl = distance_cluster_size(rb.max_rows, rb_max_b_);
     PCS_CUDA(cudaEventRecordWithFlags(ev_dist0, stream, cudaEventRecordExternal));
@@ -708,6 +727,7 @@ void Ctx::admit(Job* j)
         graph_dirty = true;
     }
     ensure_round_buffers(v_max, max_rows, max_n, rb_max);
+    look_at_widths();
     /* every job's tensor map: the histogram area may have moved */
     std::vector<TmapDev> maps(table.size());
     for (size_t i = 0; i < table.size(); ++i) {
@@ -738,6 +758,7 @@ void Ctx::retire(Job* j)
     table[j->slot] = nullptr;
     j->slot = -1;
     while (!table.empty() && !table.back()) table.pop_back();
+    look_at_widths();
     upload_table();
     PCS_CUDA(cudaStreamSynchronize(stream));
 }

@@ -146,6 +146,7 @@ struct Ctx {
     std::deque<Job*> queue;        /* serve: submitted, not yet admitted */
     uint32_t rb_max_b_ = 0;        /* widest histogram row among admitted jobs */
     bool rb_f64_ = false;          /* some admitted job's distances are double */
+    bool rb_narrow_ = false;       /* distance_mostly_narrow of the admitted jobs */
     uint64_t mem_cap = 0;
     uint64_t mem_used = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -163,6 +164,7 @@ struct Ctx {
     /* round machinery */
     void ensure_round_buffers(uint32_t v_max, uint32_t max_rows, uint32_t max_n, uint64_t rb_max);
     void upload_table();
+    void look_at_widths();
     void enqueue_round();
     void run_round(double* ms_out);
     void admit(Job* j);

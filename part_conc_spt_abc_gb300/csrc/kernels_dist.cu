@@ -1775,7 +1775,33 @@ static bool use_rows_(const DistArgs& a, uint32_t turns)
     const bool strips = use_strip(a.max_rows, 0u);
     if (!strips) from = 3u;
     if (strips && (a.max_bins & 3u) != 0u && (a.max_bins + 31u) / 32u < 3u * ((a.max_bins + 127u) / 128u)) return false;
+    if (strips && a.mostly_narrow) return false;
     return a.max_bins <= 128u * kRowsWarps && turns >= from;
+}
+
+/* CTAs of the row kernel that fit on an SM */
+static uint32_t rows_per_sm_(uint32_t max_bins)
+{
+    const size_t smem = (size_t)((max_bins + 127u) / 128u) * kRowsWarpBytes;
+    return std::max<uint32_t>(1u, (uint32_t)(kSmemPerSm / (smem + 2048u)));
+}
+
+/* A round of several jobs: every CTA of the row kernel has the warps that the
+ * widest job needs, and a narrow histogram takes one of them for as long as a
+ * wide one, where strips take turns by each histogram's own width.  The lines
+ * cross at 12 strips on average and CTA that fits on an SM (7 for 61 rows).
+ * Served jobs of 256 bins (three CTAs fit), 400 (two) and 1024 (one) beside
+ * narrow ones, distance time of all rounds, strips -> rows in ms, 201 rows: 256,
+ * 64, 64, 64 (3.5 strips) 2.85 -> 3.29, 256, 64, 64 (4) 2.35 -> 2.31, 256, 256,
+ * 64, 64 (5) 3.41 -> 2.87; 320, 128, 128, 64 (5) 3.48 -> 3.86, 320, 320, 64, 64
+ * (6) 4.26 -> 4.08; 1024, 64, 64, 64 (9.5) 8.50 -> 10.3, 1024, 256, 128, 64
+ * (11.5) 8.72 -> 8.73, 1024, 512, 256, 128 (15) 10.4 -> 8.8; 61 rows: 1024 and
+ * seven of 33 (5.75) 4.50 -> 5.46, 320, 32, 32 (4) 1.93 -> 1.52; 451 rows: 320,
+ * 128, 128, 64 (5) 4.05 -> 4.13, 1024, 256, 128, 64 9.9 -> 9.6. */
+bool distance_mostly_narrow(uint32_t max_rows, uint32_t max_bins, uint32_t strips16)
+{
+    const uint32_t line = std::min(12u, 4u + max_rows / 25u);
+    return strips16 * rows_per_sm_(max_bins) < 16u * line;
 }
 
 static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st)
@@ -1787,8 +1813,7 @@ static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st
     if (e != cudaSuccess) return e;
     const uint32_t warps = (a.max_bins + 127u) / 128u;
     const size_t smem = (size_t)warps * kRowsWarpBytes;
-    const uint32_t per_sm = std::max<uint32_t>(1u, (uint32_t)(kSmemPerSm / (smem + 2048u)));
-    k<<<std::min(a.max_count, per_sm * sms), 32u * warps, smem, st>>>(a);
+    k<<<std::min(a.max_count, rows_per_sm_(a.max_bins) * sms), 32u * warps, smem, st>>>(a);
     return cudaGetLastError();
 }
 

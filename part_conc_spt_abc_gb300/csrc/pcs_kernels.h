@@ -96,6 +96,7 @@ struct DistArgs {
     uint32_t max_bins;          /* bins of the widest histogram */
     uint32_t max_count;         /* histograms at most */
     uint32_t min_count;         /* histograms at least, as far as the host knows */
+    uint32_t mostly_narrow;     /* 1: a round of jobs most of which are too narrow for rows (distance_mostly_narrow) */
     uint32_t strips_only;       /* 1: a CTA's strips for each histogram, as the reference launches K_distance */
     const TmapDev* tmaps;       /* nullable: per job (index of jobs), tensor maps over hist */
 };
@@ -120,6 +121,9 @@ cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaSt
  * where `grid` clusters fit at once.  Which of clusters, rows and strips runs
  * follows from the turns each takes (kernels_dist.cu). */
 cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl = 0u);
+/* Whether the row kernel would lose on histograms that have `strips16` / 16
+ * strips of 32 bins on average, max_bins at most. */
+bool distance_mostly_narrow(uint32_t max_rows, uint32_t max_bins, uint32_t strips16);
 /* the cluster size for histograms of up to max_rows x max_bins, or 0 */
 uint32_t distance_cluster_size(uint32_t max_rows, uint32_t max_bins);
 const uint32_t kMaxDistCluster = 8u;
