@@ -1131,15 +1131,18 @@ struct RowsWalk {
 #pragma unroll
         for (uint32_t i = 0; i < kRowsBlock; ++i) at[i * 32u] = v[i];
         if (F64 || SSD) {
-            uint64_t sq = 0u; /* of the block: below 2^49 */
+            /* With F64 the sum counts only where every block is exact: below
+             * 2^44 a cell, no carry.  Else a block's is below 2^49. */
+            uint64_t sq = 0u;
+            uint64_t& sum = F64 ? lo : sq;
 #pragma unroll
             for (uint32_t i = 0; i < kRowsBlock; ++i) {
                 if (!FULL && b * kRowsBlock + i >= R) break;
                 if (F64 || exact) {
-                    if (VEC || nc > 0u) sq += square_(s[i].x, o[i].x);
-                    if (VEC || nc > 1u) sq += square_(s[i].y, o[i].y);
-                    if (VEC || nc > 2u) sq += square_(s[i].z, o[i].z);
-                    if (VEC || nc > 3u) sq += square_(s[i].w, o[i].w);
+                    if (VEC || nc > 0u) sum += square_(s[i].x, o[i].x);
+                    if (VEC || nc > 1u) sum += square_(s[i].y, o[i].y);
+                    if (VEC || nc > 2u) sum += square_(s[i].z, o[i].z);
+                    if (VEC || nc > 3u) sum += square_(s[i].w, o[i].w);
                 } else {
                     if (VEC || nc > 0u) wide_square_(s[i].x, o[i].x);
                     if (VEC || nc > 1u) wide_square_(s[i].y, o[i].y);
@@ -1147,7 +1150,7 @@ struct RowsWalk {
                     if (VEC || nc > 3u) wide_square_(s[i].w, o[i].w);
                 }
             }
-            add128_(hi, lo, 0u, sq);
+            if (!F64) add128_(hi, lo, 0u, sq);
         }
         observe(b + 1u);
         if (cum) {
