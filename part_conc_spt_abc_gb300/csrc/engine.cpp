@@ -3,7 +3,7 @@
  *
  * A round is a fixed sequence of kernels over every job in the context's
  * round table (plan -> propose -> items -> simulate -> distance -> accept ->
- * whiten -> kernel sum -> finalize) followed by a copy of the job status
+ * whiten -> kernel sum -> finalize), whose last kernel writes the job status
  * table to pinned host memory.  The sequence is captured once into a CUDA
  * graph and replayed; all per-round variation (which jobs, how many
  * proposals, how many work items) is read by the kernels from device memory,
@@ -610,7 +610,7 @@ void Ctx::enqueue_round()
     const uint32_t cl = distance_cluster_size(rb.max_rows, rb_max_b_);
     PCS_CUDA(cudaEventRecordWithFlags(ev_dist0, stream, cudaEventRecordExternal));
     PCS_CUDA(launch_distance(d, std::min<uint32_t>(rb.capacity, (uint32_t)(distance_ctas_per_sm(rb.max_rows) * sm_count)),
-                             stream, cl));
+                             stream, cl, &distance_kernels_));
     PCS_CUDA(cudaEventRecordWithFlags(ev_dist1, stream, cudaEventRecordExternal));
 
     PCS_CUDA(cudaEventRecordWithFlags(ev_pmc0, stream, cudaEventRecordExternal));
@@ -656,7 +656,7 @@ void Ctx::run_round(double* ms_out)
     PCS_CUDA(cudaEventElapsedTime(&pmc_ms, ev_pmc0, ev_pmc1));
     if (ms_out) *ms_out = ms;
     stats.rounds += 1;
-    stats.kernel_launches += kKernelsPerRound;
+    stats.kernel_launches += kKernelsPerRound + distance_kernels_;
     stats.simulate_launches += 1;
     stats.simulate_ms += sim_ms;
     stats.distance_launches += 1;

@@ -155,7 +155,8 @@ struct Ctx {
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
     RoundDev* h_round_out = nullptr; /* pinned copy of the round counters */
     pcs_kernel_stats stats{};
-    static const uint32_t kKernelsPerRound = 9;
+    static const uint32_t kKernelsPerRound = 8; /* besides the distance's */
+    uint32_t distance_kernels_ = 1;
     std::mutex mu;
 
     explicit Ctx(int dev, int inflight);

@@ -1820,7 +1820,7 @@ static cudaError_t launch_rows_(const DistArgs& a, uint32_t sms, cudaStream_t st
     return cudaGetLastError();
 }
 
-cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl)
+cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl, uint32_t* launched)
 {
     /* a caller that leaves these unset would get some kernel, but not the one that suits it */
     if (!a.max_rows || !a.max_bins || !a.max_count) return cudaErrorInvalidValue;
@@ -1879,6 +1879,7 @@ cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, u
                           (turns - cturns) * (230u + a.max_rows) > 400u;
     if (clusters) turns = cturns;
     const bool rows = !a.strips_only && use_rows_(a, turns);
+    if (launched) *launched = rows && f64 ? 2u : 1u;
     last_kernel(kFamilyDistance) = rows                        ? "k_distance_rows"
                                    : clusters                  ? "k_distance_cluster"
                                    : use_strip(a.max_rows, 0u) ? "k_distance_strip"

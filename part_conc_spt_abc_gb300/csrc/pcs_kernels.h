@@ -119,8 +119,9 @@ cudaError_t launch_distance_setup(const DistSetup& d, const TmapDev& map, cudaSt
  * strips of 32 bins; 0 or 1: none) allows clusters of cl CTAs, one strip of
  * a histogram per CTA, for histograms of at least kClusterRowsMin rows or
  * where `grid` clusters fit at once.  Which of clusters, rows and strips runs
- * follows from the turns each takes (kernels_dist.cu). */
-cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl = 0u);
+ * follows from the turns each takes (kernels_dist.cu).  *launched: the kernels
+ * launched, two for rows with double sums. */
+cudaError_t launch_distance(const DistArgs& a, uint32_t grid, cudaStream_t st, uint32_t cl = 0u, uint32_t* launched = nullptr);
 /* Whether the row kernel would lose on histograms that have `strips16` / 16
  * strips of 32 bins on average, max_bins at most. */
 bool distance_mostly_narrow(uint32_t max_rows, uint32_t max_bins, uint32_t strips16);
