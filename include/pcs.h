@@ -372,7 +372,10 @@ pcs_status pcs_simulate_hist(pcs_ctx* ctx, const pcs_setup* setup, const pcs_run
  * histogram (host buffers).  cum_out (nullable) receives the 2-D inclusive
  * prefix sums; dist_f32 the float sum of squared differences in the
  * reference kernel's reduction order; dist_f64 (nullable) the same in
- * double; ssd (nullable) the exact integer sum as [count][2] (hi, lo). */
+ * double; ssd (nullable) the exact integer sum as [count][2] (hi, lo).
+ * ref_sat is a cumulative histogram.  (Any counts give the same results as the
+ * reference's arithmetic where dist_f64, ssd or cum_out is asked for; the
+ * float alone may go by the last cells' size.) */
 pcs_status pcs_scan_distance(pcs_ctx* ctx, const uint32_t* hist, const uint32_t* ref_sat,
                              uint32_t rows, uint32_t bins, uint32_t count, uint32_t* cum_out,
                              float* dist_f32, double* dist_f64, uint64_t* ssd);

@@ -138,7 +138,7 @@ struct Ctx {
     Workspace ws;
     uint32_t* h_err = nullptr;
     RoundBufs rb;
-    JobPmcDev* h_status = nullptr; /* pinned mirror of the pmc table */
+    JobPmcDev* h_status = nullptr; /* pinned: the jobs' states, written by k_finalize */
     RoundDev* h_round = nullptr;   /* pinned */
     cudaGraphExec_t graph = nullptr;
     bool graph_dirty = true;
@@ -153,7 +153,7 @@ struct Ctx {
     cudaEvent_t ev_sim0 = nullptr, ev_sim1 = nullptr, ev_dist0 = nullptr, ev_dist1 = nullptr;
     cudaEvent_t ev_pmc0 = nullptr, ev_pmc1 = nullptr;
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
-    RoundDev* h_round_out = nullptr; /* pinned copy of the round counters */
+    RoundDev* h_round_out = nullptr; /* pinned: the round counters, written by k_finalize */
     pcs_kernel_stats stats{};
     static const uint32_t kKernelsPerRound = 8; /* besides the distance's */
     uint32_t distance_kernels_ = 1;

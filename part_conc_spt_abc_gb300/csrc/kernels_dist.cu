@@ -18,6 +18,8 @@
  *            or each has a cluster): a thread-block cluster per histogram,
  *            one strip per CTA, the row carries and per-lane sums
  *            exchanged through distributed shared memory;
+ *   k_distance_rows (up to 1024 bins, many or wide histograms): a warp per
+ *            128 columns, the rows stream past it;
  *   k_distance (taller histograms, 1024 threads): the same in blocks of
  *            256 rows (tile row pitch 33 words), with the column carry in a
  *            register.
@@ -902,11 +904,11 @@ __global__ void __launch_bounds__(512, 2) k_distance_cluster(DistArgs a, uint32_
  * [32][128] floats per warp, one 16-byte read and write per row and lane; at
  * the end the strips' are added in order and the reference's trees follow.
  *
- * 62 warp instructions per 128 cells, where the strip kernel, passing over
+ * 65 warp instructions per 128 cells, where the strip kernel, passing over
  * its tile three times, has about 150; of 8 warps per SM (shared memory: 28 KB
- * each, 64 KB of loads in flight) the two per scheduler issue in 31 % of the
+ * each, 64 KB of loads in flight) the two per scheduler issue in 32 % of the
  * cycles, between waits for shared memory, scans and the observed cells.
- * 1024 of 301 x 128: 88 us (strips) -> 51 us.  One lane per column instead
+ * 1024 of 301 x 128: 88 us (strips) -> 52 us.  One lane per column instead
  * (7 KB per warp, 32 warps per SM) has 48 instructions per 32 cells: 86 us.
  * A walk down few rows at a time costs a fixed 90 ns per row, so few
  * histograms of few columns stay with the strips (use_rows_).
@@ -1792,7 +1794,8 @@ static uint32_t rows_per_sm_(uint32_t max_bins)
 /* A round of several jobs: every CTA of the row kernel has the warps that the
  * widest job needs, and a narrow histogram takes one of them for as long as a
  * wide one, where strips take turns by each histogram's own width.  The lines
- * cross at 12 strips on average and CTA that fits on an SM (7 for 61 rows).
+ * cross at 12 strips on average where one CTA fits on an SM, 6 where two do, 4
+ * where three do (for 61 rows at 6.4, 3.2 and 2.1).
  * Served jobs of 256 bins (three CTAs fit), 400 (two) and 1024 (one) beside
  * narrow ones, distance time of all rounds, strips -> rows in ms, 201 rows: 256,
  * 64, 64, 64 (3.5 strips) 2.85 -> 3.29, 256, 64, 64 (4) 2.35 -> 2.31, 256, 256,
