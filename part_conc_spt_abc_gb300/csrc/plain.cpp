@@ -177,10 +177,15 @@ void run_plain(Job& j, uint32_t max_steps, uint32_t queues)
         d.max_bins = j.B;
         d.max_count = d.min_count = 1u;
         /* the reference's geometry: one CTA walks the histogram strip by strip.
-         * The persistent form takes what a standalone call of one histogram
-         * takes: a cluster over its strips, the row kernel past 8 of them */
+         * So it does in the persistent form up to 7 strips, and rows stream past
+         * one CTA from 8 on: with `queues` histograms in flight beside as many
+         * walks the CTA's time does not show, and a cluster over the strips,
+         * which one histogram alone is fastest with, has to wait for room for
+         * all its CTAs at once (configuration 1 1.38e11 particle-steps/s, with
+         * clusters 1.34e11; configuration 2 1.81e11, 1.75e11; the serving
+         * stream's first four jobs within 1 %) */
         d.strips_only = ref_geometry;
-        PCS_CUDA(launch_distance(d, 1, q.st, distance_cluster_size(j.R, j.B)));
+        PCS_CUDA(launch_distance(d, 1, q.st, 0u));
         PCS_CUDA(cudaMemcpyAsync(q.h_dist, q.d_dist.p, sizeof(float), cudaMemcpyDeviceToHost, q.st));
         PCS_CUDA(cudaEventRecord(q.done, q.st));
         q.slot = (int)slot;

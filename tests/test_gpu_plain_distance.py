@@ -1,14 +1,13 @@
 """The distance kernel that each plain form launches: strips of one CTA in the
-reference's geometry; in the persistent one a cluster over the histogram's
-strips, or the row kernel where there are more strips than a cluster has CTAs.
-Both give the same estimation, bit for bit."""
+reference's geometry; in the persistent one, too, but the row kernel where
+there are eight strips or more.  Both give the same estimation, bit for bit."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("frames,bins,persistent", [(60, 100, b"k_distance_cluster"), (200, 64, b"k_distance_cluster"),
+@pytest.mark.parametrize("frames,bins,persistent", [(60, 100, b"k_distance_strip"), (700, 64, b"k_distance_strip"),
                                                     (60, 30, b"k_distance_strip"), (60, 300, b"k_distance_rows")])
 def test_plain_forms(pcs, ctx, frames, bins, persistent):
     import part_conc_spt_abc_gb300.workloads as W
